@@ -154,7 +154,7 @@ __global__ void moments_reduce_kernel(int C, int Pf, const int* __restrict__ ite
 __global__ void permute_kernel(int n, const int* __restrict__ perm, const double* __restrict__ q3,
                                double* __restrict__ qx, double* __restrict__ qy,
                                double* __restrict__ qz, float* __restrict__ fqx,
-                               float* __restrict__ fqy, float* __restrict__ fqz) {
+                               float* __restrict__ fqy, float* __restrict__ fqz, PackSrc ps) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   int o = perm[p];
@@ -165,6 +165,24 @@ __global__ void permute_kernel(int n, const int* __restrict__ perm, const double
   fqx[p] = (float)a;
   fqy[p] = (float)b;
   fqz[p] = (float)c;
+  const double w = ps.a[p], wq = ps.pack == PACK_SL ? w : 1.0;
+  if (ps.pack == PACK_E2G) {
+    double2* r = reinterpret_cast<double2*>(ps.pk) + 6 * (size_t)p;
+    const double u = ps.nx[p], v = ps.ny[p], z = ps.nz[p];
+    r[0] = make_double2(ps.x[p], ps.y[p]);
+    r[1] = make_double2(ps.z[p], w);
+    r[2] = make_double2(a, b);
+    r[3] = make_double2(c, u * u + v * v + z * z);
+    r[4] = make_double2(u, v);
+    r[5] = make_double2(z, 0.0);
+    return;
+  }
+  double2* r = reinterpret_cast<double2*>(ps.pk) + 5 * (size_t)p;
+  r[0] = make_double2(ps.x[p], ps.y[p]);
+  r[1] = make_double2(ps.z[p], w);
+  r[2] = make_double2(w * ps.nx[p], w * ps.ny[p]);
+  r[3] = make_double2(w * ps.nz[p], wq * a);
+  r[4] = make_double2(wq * b, wq * c);
 }
 
 __global__ void permute_soa_kernel(int n, const int* __restrict__ perm,
@@ -359,9 +377,9 @@ void launch_moments_reduce(int C, int Pf, int nnodes_out, const int* d_item_star
 }
 
 void launch_permute(int n, const int* perm, const double* q3, double* qx, double* qy, double* qz,
-                    float* fqx, float* fqy, float* fqz, cudaStream_t st) {
+                    float* fqx, float* fqy, float* fqz, const PackSrc& ps, cudaStream_t st) {
   if (n <= 0) return;
-  permute_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, perm, q3, qx, qy, qz, fqx, fqy, fqz);
+  permute_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, perm, q3, qx, qy, qz, fqx, fqy, fqz, ps);
 }
 
 void launch_permute_soa(int n, const int* perm, const double* src, double* dst, cudaStream_t st) {

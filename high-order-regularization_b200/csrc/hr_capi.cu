@@ -177,7 +177,8 @@ void single_eval(Ctx& C, int kind, const hr_eval_opts* opt, double delta, const 
   tree.build(*S, P, N0, theta, direct, st);
   DBuf<double> q3;
   q3.upload(dens, 3 * (size_t)S->n, st);
-  tree.set_density(C, q3.p, dl, !direct, opt && opt->precision != HR_FP64);
+  tree.set_density(C, q3.p, kind > K_DL_OFF ? PACK_E2G : (dl ? PACK_DL : PACK_SL), !direct,
+                   opt && opt->precision != HR_FP64);
   std::vector<uint8_t> near =
       (kind == K_SL_OFF || kind == K_DL_OFF) ? near_flags(nt, b, delta) : std::vector<uint8_t>(nt, 1);
   DevTargets tg;
@@ -678,7 +679,7 @@ void plan_matvec(hr_plan2s& P, const double* x_dev, double* y_dev, int prec) {
   hr_plan2s::Inner* in = (prec != HR_FP64 && P.inner) ? P.inner.get() : nullptr;
   DevTree* trees = in ? in->tree : P.tree;
   plan_ready(P);  // the stencils and the FP64 stresslet batch
-  for (int s = 0; s < 2; s++) trees[s].set_density(C, P.xin.p + P.off[s], true, tree, prec != HR_FP64);
+  for (int s = 0; s < 2; s++) trees[s].set_density(C, P.xin.p + P.off[s], PACK_DL, tree, prec != HR_FP64);
   for (int t = 0; t < 2; t++) {
     P.tg[t].g0.zero(st);
     launch_interp(P.sten[t].ne, P.sten[t].tgt.p, P.sten[t].idx.p, P.sten[t].pq.p,
@@ -706,7 +707,7 @@ void plan_rhs(hr_plan2s& P, const double* f1_dev, const double* f2_dev, double* 
   if (f2_dev != P.fin.p + P.off[1])
     HR_CHECK_CUDA(cudaMemcpyAsync(P.fin.p + P.off[1], f2_dev, sizeof(double) * 3 * P.nq[1],
                                   cudaMemcpyDeviceToDevice, st));
-  for (int s = 0; s < 2; s++) P.tree[s].set_density(C, P.fin.p + P.off[s], false, tree);
+  for (int s = 0; s < 2; s++) P.tree[s].set_density(C, P.fin.p + P.off[s], PACK_SL, tree);
   P.sl.launch(C);
   // SL_1 = on1 + comp2 ; SL_2 = comp1 + on2 ; b = -SL * 2/3
   launch_rhs_combine(3 * P.nq[0], 2.0 / 3.0, P.out_on[0].p, P.out_off[0].p, b_dev + P.off[0], st);
@@ -1260,10 +1261,10 @@ extern "C" int hr_plan2s_check_upward_pass(hr_plan2s* plan, const double* x, dou
       DevTree& T = P.tree[s];
       const size_t m = (size_t)T.nn * 12 * T.Pf;
       std::vector<double> a(m), b(m);
-      T.set_density(C, P.xin.p + P.off[s], true, true, false);
+      T.set_density(C, P.xin.p + P.off[s], PACK_DL, true, false);
       HR_CHECK_CUDA(cudaMemcpyAsync(a.data(), T.mom.p, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
       HR_CHECK_CUDA(cudaStreamSynchronize(st));
-      T.set_density(C, P.xin.p + P.off[s], true, true, true);
+      T.set_density(C, P.xin.p + P.off[s], PACK_DL, true, true);
       HR_CHECK_CUDA(cudaMemcpyAsync(b.data(), T.mom.p, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
       HR_CHECK_CUDA(cudaStreamSynchronize(st));
       C.check_tc();

@@ -25,6 +25,7 @@ struct EvalTask {
   double scale;   // final factor of the sum (1/8pi, -6/8pi, ...)
   const double *sx, *sy, *sz, *snx, *sny, *snz, *sa;  // sources, tree order
   const double *qx, *qy, *qz;                         // density, tree order
+  const double* pk;                                   // packed sources, tree order (Pack), for the FP64 sums
   double ctr[3];                                      // source surface centre (FP32 frame origin)
   // FP32 copies for the mixed-precision far field: positions relative to ctr
   const float *fx, *fy, *fz, *fnx, *fny, *fnz, *fa, *fqx, *fqy, *fqz;
@@ -68,15 +69,29 @@ struct BlockRef {
 
 enum Family : int { F_SL = 0, F_DL = 1, F_E2G = 2 };
 
-// Evaluates every work item of a combined list — the first n_on items (lean:
-// on-surface tasks, or the extend-to-grid box-face sums) in one launch on st,
-// the rest in another on `side` (forked from and joined back to st with the
-// two events; on st as well when side is null) — then reduces the partial sums
-// per target (deterministic order) and applies the epilogue. With count, the
-// FP64 launches also add their per-branch pair counts to the tasks' counters.
-void launch_eval(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs,
-                 int nitems, int n_on, int ntask_blocks, const int2* d_task_blocks, cudaStream_t st,
-                 cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, bool mixed, bool count);
+// A source's packed record; the area weight a is multiplied into what a
+// family's pairs only use times it.
+enum Pack : int {
+  PACK_SL = 0,   // 10 doubles: x, y, z, a, a normal, a density
+  PACK_DL = 1,   // 10 doubles: x, y, z, a, a normal, density
+  PACK_E2G = 2,  // 12 doubles: x, y, z, a, density, normal.normal, normal, 0
+};
+
+// The reduced-precision sums of a batch: every work item of a combined list,
+// the first n_on items (lean: on-surface tasks, or the extend-to-grid box-face
+// sums) in one launch on st, the rest in another on side.
+void launch_eval(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems, int n_on,
+                 cudaStream_t st, cudaStream_t side);
+
+// The FP64 sums of a batch likewise (hr_eval64.cu). next: two zeroed work
+// counters (one per launch); launch_reduce zeroes them again. With count, the
+// per-branch pair counts are added to the tasks' counters.
+void launch_eval64(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems,
+                   int n_on, unsigned* next, int num_sms, cudaStream_t st, cudaStream_t side, bool count);
+// The batch's reduction (the items' partial sums per target, in slot order) and
+// epilogue; zeroes the two counters at next.
+void launch_reduce(const EvalTask* d_tasks, int ntask_blocks, const int2* d_task_blocks, unsigned* next,
+                   cudaStream_t st);
 
 // Upward pass: proxy moments of every non-root node of a tree.
 struct MomItem {
@@ -109,8 +124,15 @@ void launch_moments_reduce(int C, int Pf, int nnodes_out, const int* d_item_star
                            const double* partial, double* mom, float* momf, cudaStream_t st);
 
 // Gathers interleaved reference-order density into tree-order SoA.
+// and fills the density of the packed records pk (xyz, normals and areas of
+// the tree) as `pack` says.
+struct PackSrc {
+  const double *x, *y, *z, *nx, *ny, *nz, *a;
+  double* pk;
+  int pack;
+};
 void launch_permute(int n, const int* perm, const double* q3, double* qx, double* qy, double* qz,
-                    float* fqx, float* fqy, float* fqz, cudaStream_t st);
+                    float* fqx, float* fqy, float* fqz, const PackSrc& ps, cudaStream_t st);
 void launch_permute_soa(int n, const int* perm, const double* src, double* dst, cudaStream_t st);
 
 // Six-point density interpolation at nearest points.

@@ -308,7 +308,7 @@ extern "C" int hr_e2g_create(hr_ctx* ctx, int N, hr_e2g** out) {
     surf.center[0] = surf.center[1] = surf.center[2] = 1.5;
     E->tree.build(surf, 6, 1000, 0.6, true, st);
     E->q3.upload(S.f, st);
-    E->tree.set_density(C, E->q3.p, false, false);
+    E->tree.set_density(C, E->q3.p, PACK_E2G, false);
     // face targets in the reference loop order (E2G/main.cpp:1058-1075)
     std::vector<double> fx;
     std::vector<long> fg;

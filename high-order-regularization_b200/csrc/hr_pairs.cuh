@@ -3,10 +3,8 @@
 // The formulas are the reference's:
 //   reg_coeff         get_reg_coeff_7ord + evaluate_In_024   2S/utilities.cpp:163-175, 327-337
 //   sl_7ord           Stokes_SL_7ord                         2S/utilities.cpp:179-207
-//   sl_7ord_onsurf    Stokes_SL_7ord_onSurf                  2S/utilities.cpp:211-254
 //   dl_7ord           Stokes_DL_7ord                         2S/utilities.cpp:258-288
-//   dl_7ord_onsurf    Stokes_DL_7ord_onSurf                  2S/utilities.cpp:292-323
-//   lapl_dl_7ord      Lapl_DL_7ord                           E2G/utilities.cpp:190-211
+//   sl_lapl_7ord      Stokes_SL_7ord and Lapl_DL_7ord        E2G/utilities.cpp:190-211
 // evaluated from r^2 and one reciprocal square root per pair: every 1/r^k
 // of the reference becomes a product of rinv = rsqrt(r^2), r/delta becomes
 // r * (1/delta), and the switch r/delta > 8 becomes r^2 > 64 delta^2. Each
@@ -37,7 +35,6 @@ constexpr float kPlainOnSurf32 = 28.5f;
 struct Reg {
   double d, inv_d, d64, r0sq;  // delta, 1/delta, 64 delta^2, (1e-14)^2
   double inv_d2, inv_d3, inv_d5;
-  double dplain;               // kPlainOnSurf64 delta^2
 };
 
 __device__ __forceinline__ Reg make_reg(double d) {
@@ -49,7 +46,6 @@ __device__ __forceinline__ Reg make_reg(double d) {
   g.inv_d2 = g.inv_d * g.inv_d;
   g.inv_d3 = g.inv_d2 * g.inv_d;
   g.inv_d5 = g.inv_d3 * g.inv_d2;
-  g.dplain = kPlainOnSurf64 * d * d;
   return g;
 }
 
@@ -100,34 +96,6 @@ __device__ __forceinline__ bool sl_7ord(double r2, double rinv, const Reg& g, co
   return true;
 }
 
-// Regularized Stokeslet factors, on-surface target (lambda = 0).
-__device__ __forceinline__ bool sl_7ord_onsurf(double r2, double rinv, const Reg& g, double& s1,
-                                               double& s2) {
-  const double rp = d_rootpi();
-  if (r2 < g.r0sq) {
-    s1 = 32.0 / 5.0 / rp / g.d;
-    s2 = 256.0 / 15.0 / rp / (g.d * g.d * g.d);
-    return false;
-  }
-  double rinv3 = rinv * rinv * rinv;
-  if (r2 > g.d64) {
-    s1 = rinv;
-    s2 = rinv3;
-    return false;
-  }
-  double rd = r2 * rinv * g.inv_d;
-  double rd2 = rd * rd;
-  double rd4 = rd2 * rd2;
-  double rd6 = rd4 * rd2;
-  double errfn = erf(rd);
-  double r_expfn = 2.0 / rp * rd * exp(-rd2);
-  double poly1 = 11.0 / 5.0 - 26.0 / 15.0 * rd2 + 4.0 / 15.0 * rd4;
-  double poly2 = -1.0 + (118.0 * rd2 - 68.0 * rd4 + 8.0 * rd6) * (1.0 / 15.0);
-  s1 = (errfn + poly1 * r_expfn) * rinv;
-  s2 = (errfn + poly2 * r_expfn) * rinv3;
-  return true;
-}
-
 // Regularized stresslet factors (s2 ~ 1/r^3, s3 ~ 1/r^5), off-surface target.
 __device__ __forceinline__ bool dl_7ord(double r2, double rinv, const Reg& g, const Coef& c,
                                         double& s2, double& s3) {
@@ -161,56 +129,8 @@ __device__ __forceinline__ bool dl_7ord(double r2, double rinv, const Reg& g, co
   return true;
 }
 
-// Regularized stresslet factor s3 ~ 1/r^5, on-surface target.
-__device__ __forceinline__ bool dl_7ord_onsurf(double r2, double rinv, const Reg& g, double& s3) {
-  const double rp = d_rootpi();
-  if (r2 < g.r0sq) {
-    s3 = 128.0 / 45.0 / rp / (g.d * g.d * g.d * g.d * g.d);
-    return false;
-  }
-  double rinv2 = rinv * rinv;
-  double rinv5 = rinv2 * rinv2 * rinv;
-  if (r2 > g.d64) {
-    s3 = rinv5;
-    return false;
-  }
-  double rd = r2 * rinv * g.inv_d;
-  double rd2 = rd * rd;
-  double rd4 = rd2 * rd2;
-  double rd6 = rd4 * rd2;
-  double errfn = erf(rd);
-  double r_expfn = 2.0 / rp * rd * exp(-rd2);
-  double poly3 = -1.0 - 2.0 / 3.0 * rd2 + 52.0 / 45.0 * rd4 - 8.0 / 45.0 * rd6;
-  s3 = (errfn + poly3 * r_expfn) * rinv5;
-  return true;
-}
-
-// Regularized 1/r^3 kernel of the pressure (Laplace double layer type).
-__device__ __forceinline__ bool lapl_dl_7ord(double r2, double rinv, const Reg& g, const Coef& c,
-                                             double& s2) {
-  const double rp = d_rootpi();
-  if (r2 < g.r0sq) {
-    s2 = 256.0 / 15.0 / rp / (g.d * g.d * g.d);
-    return false;
-  }
-  double rinv3 = rinv * rinv * rinv;
-  if (r2 > g.d64) {
-    s2 = rinv3;
-    return false;
-  }
-  double rd = r2 * rinv * g.inv_d;
-  double rd2 = rd * rd;
-  double rd4 = rd2 * rd2;
-  double errfn = erf(rd);
-  double r_expfn = rd * exp(-rd2);
-  double poly2 = -2.0 / rp + 2.0 * (c.c1 + 2.0 * (c.c2 + c.c3)) * rd2 -
-                 4.0 * (c.c2 + 5.0 * c.c3) * rd4 + 8.0 * c.c3 * rd4 * rd2;
-  s2 = (errfn + poly2 * r_expfn) * rinv3;
-  return true;
-}
-
-// sl_7ord and lapl_dl_7ord of one pair together: s1, s2 as sl_7ord, s2p as
-// lapl_dl_7ord (its own association of the last polynomial term), sharing
+// Stokes_SL_7ord and Lapl_DL_7ord of one pair together: s1, s2 as sl_7ord, s2p
+// the pressure's (its own association of the last polynomial term), sharing
 // the powers of r/delta, erf and exp.
 __device__ __forceinline__ bool sl_lapl_7ord(double r2, double rinv, const Reg& g, const Coef& c, double& s1,
                                              double& s2, double& s2p) {
@@ -287,21 +207,6 @@ __device__ __forceinline__ void sl_7ord_f(float r2, float rinv, const RegF& g, c
   s2 = (errfn + poly2 * r_expfn) * rinv3;
 }
 
-__device__ __forceinline__ void sl_7ord_onsurf_f(float r2, float rinv, const RegF& g, float& s1, float& s2) {
-  const float rinv3 = rinv * rinv * rinv;
-  if (r2 > g.d64) {
-    s1 = rinv;
-    s2 = rinv3;
-    return;
-  }
-  const float rd = r2 * rinv * g.inv_d, rd2 = rd * rd, rd4 = rd2 * rd2, rd6 = rd4 * rd2;
-  const float errfn = erff(rd), r_expfn = 2.0f / kRootPiF * rd * expf(-rd2);
-  const float poly1 = 11.0f / 5.0f - 26.0f / 15.0f * rd2 + 4.0f / 15.0f * rd4;
-  const float poly2 = -1.0f + (118.0f * rd2 - 68.0f * rd4 + 8.0f * rd6) * (1.0f / 15.0f);
-  s1 = (errfn + poly1 * r_expfn) * rinv;
-  s2 = (errfn + poly2 * r_expfn) * rinv3;
-}
-
 __device__ __forceinline__ void dl_7ord_f(float r2, float rinv, const RegF& g, const CoefF& c, float& s2,
                                           float& s3) {
   const float rinv2 = rinv * rinv, rinv3 = rinv2 * rinv;
@@ -322,19 +227,7 @@ __device__ __forceinline__ void dl_7ord_f(float r2, float rinv, const RegF& g, c
   s3 = (errfn + poly3 * r_expfn) * (rinv3 * rinv2);
 }
 
-__device__ __forceinline__ void dl_7ord_onsurf_f(float r2, float rinv, const RegF& g, float& s3) {
-  const float rinv2 = rinv * rinv, rinv5 = rinv2 * rinv2 * rinv;
-  if (r2 > g.d64) {
-    s3 = rinv5;
-    return;
-  }
-  const float rd = r2 * rinv * g.inv_d, rd2 = rd * rd, rd4 = rd2 * rd2, rd6 = rd4 * rd2;
-  const float errfn = erff(rd), r_expfn = 2.0f / kRootPiF * rd * expf(-rd2);
-  const float poly3 = -1.0f - 2.0f / 3.0f * rd2 + 52.0f / 45.0f * rd4 - 8.0f / 45.0f * rd6;
-  s3 = (errfn + poly3 * r_expfn) * rinv5;
-}
-
-// sl_7ord_f and lapl_dl_7ord_f of one pair together (as sl_lapl_7ord).
+// sl_lapl_7ord in FP32.
 __device__ __forceinline__ void sl_lapl_7ord_f(float r2, float rinv, const RegF& g, const CoefF& c, float& s1,
                                                float& s2, float& s2p) {
   const float rinv3 = rinv * rinv * rinv;
@@ -354,19 +247,6 @@ __device__ __forceinline__ void sl_lapl_7ord_f(float r2, float rinv, const RegF&
   s1 = (errfn + poly1 * r_expfn) * rinv;
   s2 = (errfn + poly2 * r_expfn) * rinv3;
   s2p = (errfn + poly2p * r_expfn) * rinv3;
-}
-
-__device__ __forceinline__ void lapl_dl_7ord_f(float r2, float rinv, const RegF& g, const CoefF& c, float& s2) {
-  const float rinv3 = rinv * rinv * rinv;
-  if (r2 > g.d64) {
-    s2 = rinv3;
-    return;
-  }
-  const float rd = r2 * rinv * g.inv_d, rd2 = rd * rd, rd4 = rd2 * rd2;
-  const float errfn = erff(rd), r_expfn = rd * expf(-rd2);
-  const float poly2 = -2.0f / kRootPiF + 2.0f * (c.c1 + 2.0f * (c.c2 + c.c3)) * rd2 -
-                      4.0f * (c.c2 + 5.0f * c.c3) * rd4 + 8.0f * c.c3 * rd4 * rd2;
-  s2 = (errfn + poly2 * r_expfn) * rinv3;
 }
 
 }  // namespace hr

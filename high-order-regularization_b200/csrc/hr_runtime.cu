@@ -142,6 +142,7 @@ void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direc
   qx.alloc(n);
   qy.alloc(n);
   qz.alloc(n);
+  pk.alloc(12 * (size_t)n);
   for (int k = 0; k < 3; k++) ctr[k] = S.center[k];
   {
     std::vector<float> a0(n), a1(n), a2(n), b0(n), b1(n), b2(n), c0(n);
@@ -213,8 +214,10 @@ void Ctx::check_tc() {
   }
 }
 
-void DevTree::set_density(Ctx& C, const double* q3_dev, bool dl, bool moments, bool tc) {
-  launch_permute(n, perm.p, q3_dev, qx.p, qy.p, qz.p, fqx.p, fqy.p, fqz.p, C.stream);
+void DevTree::set_density(Ctx& C, const double* q3_dev, int pack, bool moments, bool tc) {
+  const bool dl = pack == PACK_DL;
+  launch_permute(n, perm.p, q3_dev, qx.p, qy.p, qz.p, fqx.p, fqy.p, fqz.p,
+                 {x.p, y.p, z.p, nx.p, ny.p, nz.p, a.p, pk.p, pack}, C.stream);
   C.launches++;
   if (moments && nitems > 0 && tc && moments_tc_supported(P1)) {
     if (!C.tc_err.p) {
@@ -271,6 +274,7 @@ EvalTask make_task(int kind, double DEL, double scale, const DevTree& T, const D
   k.qx = T.qx.p;
   k.qy = T.qy.p;
   k.qz = T.qz.p;
+  k.pk = T.pk.p;
   for (int c = 0; c < 3; c++) k.ctr[c] = T.ctr[c];
   k.fx = T.fx.p;
   k.fy = T.fy.p;
@@ -304,49 +308,101 @@ EvalTask make_task(int kind, double DEL, double scale, const DevTree& T, const D
   return k;
 }
 
+namespace {
+
+// Lean kinds (their own launch): on-surface sums, the extend-to-grid box-face sums.
+bool lean_kind(int k) {
+  return k == K_SL_ON || k == K_DL_ON || k == K_E2G_SL_AWAY || k == K_E2G_P_AWAY || k == K_E2G_UP_AWAY;
+}
+
+// Cost of one target-source pair and of one target-proxy pair for a warp, in
+// FP64 instructions of the kernels of hr_eval64.cu.
+struct PairCost {
+  double direct, proxy;
+};
+PairCost pair_cost(int kind) {
+  switch (kind) {
+    case K_DL_ON: return {36, 25};
+    case K_DL_OFF: return {75, 25};
+    case K_SL_ON: return {40, 22};
+    case K_SL_OFF: return {50, 22};
+    case K_E2G_SL_AWAY:
+    case K_E2G_P_AWAY:
+    case K_E2G_UP_AWAY: return {28, 0};
+    default: return {60, 0};  // the extend-to-grid band
+  }
+}
+
+}  // namespace
+
 void Batch::finalize(cudaStream_t st, int num_sms) {
-  // 1. segments: a far entry whole, a near entry cut into source ranges of
-  //    at most kSegSrc; cost ~ active warps x pair evaluations.
-  constexpr int kSegSrc = 512;
   struct HSeg {
     Seg s;
     double cost;
   };
-  std::vector<std::vector<std::vector<HSeg>>> per(tasks.size());
-  double total = 0.0;
+  // The FP64 kernels take work by the warp (hr_eval64.cu); the others by the CTA.
+  const bool by_warp = !tasks.empty() && !tasks[0].mixed;
+  auto entry_warps = [](const Entry& E) {
+    int warps = 0;
+    for (int w = 0; w < 4; w++) warps += E.mask[w] != 0u;
+    return warps;
+  };
+  // 1. the cost of each launch (lean items, the others)
+  double total[2] = {0.0, 0.0};
   for (size_t t = 0; t < tasks.size(); t++) {
     const Lists& L = *lists[t];
     const Tree& T = *trees[t];
-    const int P1 = T.P + 1;
-    const double Pf = (double)P1 * P1 * P1;
+    const double Pf = (double)(T.P + 1) * (T.P + 1) * (T.P + 1);
+    const PairCost pc = by_warp ? pair_cost(tasks[t].kind) : PairCost{2.0, 1.5};
+    double sum = 0.0;
+    // every cost is a multiple of 1/2 far below 2^52: exact in any order
+#pragma omp parallel for schedule(dynamic, 16) reduction(+ : sum)
+    for (int b = 0; b < L.nblocks(); b++)
+      for (int e = L.blk_start[b]; e < L.blk_start[b + 1]; e++) {
+        const Entry& E = L.entries[e];
+        sum += entry_warps(E) * (E.type == 0 ? Pf * pc.proxy : (T.m1[E.node] + 1 - T.m0[E.node]) * pc.direct);
+      }
+    total[lean_kind(tasks[t].kind) ? 0 : 1] += sum;
+  }
+  // 2. the cost of an item (a run of consecutive segments of one block).
+  //    Small items keep the tail short. By the CTA: total / (SMs x 4 resident
+  //    CTAs x 16 waves), never below two tiles. By the warp: each launch on its
+  //    own and with its kinds' costs, in segments no longer than an item and
+  //    never below kMinSrc sources (stresslet batch at h = 1/64, P = 6, with
+  //    kWaves = 8 / 16 / 24 / 48: 4.06 / 3.87 / 3.89 / 3.92 ms; one partition
+  //    for both launches 4.14 ms).
+  constexpr double kWaves = 16, kMinSrc = 128;
+  double target[2];
+  for (int c = 0; c < 2; c++) target[c] = std::max((total[0] + total[1]) / (num_sms * 4.0 * 16.0), 2.0 * 256.0 * 2.0);
+  if (by_warp)
+    for (int c = 0; c < 2; c++) target[c] = std::max(4.0 * total[c] / (num_sms * 16.0 * kWaves), 4.0 * kMinSrc * 36.0);
+  // 3. segments: a far entry whole, a near entry cut into source ranges of at
+  //    most 512; cost ~ active warps x pair evaluations.
+  std::vector<std::vector<std::vector<HSeg>>> per(tasks.size());
+  for (size_t t = 0; t < tasks.size(); t++) {
+    const Lists& L = *lists[t];
+    const Tree& T = *trees[t];
+    const double Pf = (double)(T.P + 1) * (T.P + 1) * (T.P + 1);
+    const PairCost pc = by_warp ? pair_cost(tasks[t].kind) : PairCost{2.0, 1.5};
+    const double want = target[lean_kind(tasks[t].kind) ? 0 : 1];
+    const int seg = by_warp ? std::min(512, std::max((int)kMinSrc, (int)(want / (4.0 * pc.direct)) / 32 * 32)) : 512;
     per[t].resize(L.nblocks());
-    // blocks are independent; every cost is a multiple of 1/2 far below 2^52,
-    // so the sum is exact (and the item size the same) in any order
-#pragma omp parallel for schedule(dynamic, 16) reduction(+ : total)
+#pragma omp parallel for schedule(dynamic, 16)
     for (int b = 0; b < L.nblocks(); b++) {
       for (int e = L.blk_start[b]; e < L.blk_start[b + 1]; e++) {
         const Entry& E = L.entries[e];
-        int warps = 0;
-        for (int w = 0; w < 4; w++) warps += E.mask[w] != 0u;
+        const int warps = entry_warps(E);
         if (E.type == 0) {
-          double c = warps * Pf * 1.5;
-          per[t][b].push_back({Seg{e, 0, 0}, c});
-          total += c;
+          per[t][b].push_back({Seg{e, 0, 0}, warps * Pf * pc.proxy});
         } else {
-          for (int s0 = T.m0[E.node]; s0 <= T.m1[E.node]; s0 += kSegSrc) {
-            int s1 = std::min(T.m1[E.node] + 1, s0 + kSegSrc);
-            double c = warps * (double)(s1 - s0) * 2.0;
-            per[t][b].push_back({Seg{e, s0, s1}, c});
-            total += c;
+          for (int s0 = T.m0[E.node]; s0 <= T.m1[E.node]; s0 += seg) {
+            const int s1 = std::min(T.m1[E.node] + 1, s0 + seg);
+            per[t][b].push_back({Seg{e, s0, s1}, warps * (double)(s1 - s0) * pc.direct});
           }
         }
       }
     }
   }
-  // 2. items: runs of consecutive segments of one block, each about
-  //    total / (SMs x 4 resident CTAs x 16 waves), never below two tiles;
-  //    small items keep the tail short where the cost estimate is off.
-  const double target = std::max(total / (num_sms * 4.0 * 16.0), 2.0 * 256.0 * 2.0);
   // Blocks in task order; each block's runs are formed on its own (in
   // parallel), then offsets give every segment and item (slot) the position
   // a serial pass over the blocks would give it.
@@ -358,6 +414,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
 #pragma omp parallel for schedule(dynamic, 64)
   for (long q = 0; q < nbt; q++) {
     const auto& v = per[tblocks[q].x][tblocks[q].y];
+    const double want = target[lean_kind(tasks[tblocks[q].x].kind) ? 0 : 1];
     size_t i = 0;
     while (i < v.size()) {
       double c = 0.0;
@@ -366,7 +423,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
         c += v[i].cost;
         i++;
         n++;
-      } while (i < v.size() && c + v[i].cost <= target);
+      } while (i < v.size() && c + v[i].cost <= want);
       runs[q].push_back({n, c});
     }
     // a block without work still gets one (empty) item so that its partial
@@ -407,11 +464,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   }
   // lean items first (their own launch: on-surface kinds, or the extend-to-grid
   // box-face sums), each part by decreasing cost
-  auto on_kind = [&](const BlockRef& r) {
-    const int k = tasks[r.task].kind;
-    return family == F_E2G ? (k == K_E2G_SL_AWAY || k == K_E2G_P_AWAY || k == K_E2G_UP_AWAY)
-                           : (k == K_SL_ON || k == K_DL_ON);
-  };
+  auto on_kind = [&](const BlockRef& r) { return lean_kind(tasks[r.task].kind); };
   std::stable_sort(items.begin(), items.end(),
                    [&](const std::pair<double, BlockRef>& a, const std::pair<double, BlockRef>& b) {
                      const bool oa = on_kind(a.second), ob = on_kind(b.second);
@@ -431,6 +484,10 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   d_item_start.upload(starts, st);
   d_task_blocks.upload(tblocks, st);
   d_partial.alloc((size_t)std::max(1, slot) * kTB * kPartComps);
+  d_next.alloc(2);
+  d_next.zero(st);
+  // the FP64 kernels stage one smoothing table per launch
+  for (const EvalTask& t : tasks) HR_REQUIRE(t.DEL == tasks[0].DEL, "the tasks of a batch share one delta");
   for (size_t t = 0; t < tasks.size(); t++) {
     tasks[t].item_start = d_item_start.p + start_off[t];
     tasks[t].partial = d_partial.p;
@@ -440,8 +497,21 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
 }
 
 void Batch::launch(Ctx& C) {
-  launch_eval(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, ntask_blocks, d_task_blocks.p,
-              C.stream, C.side, C.ev_fork, C.ev_join, !tasks.empty() && tasks[0].mixed, C.count_work);
+  const bool two = n_on > 0 && nitems > n_on;
+  cudaStream_t side = two ? C.side : C.stream;
+  if (two) {
+    HR_CHECK_CUDA(cudaEventRecord(C.ev_fork, C.stream));
+    HR_CHECK_CUDA(cudaStreamWaitEvent(C.side, C.ev_fork, 0));
+  }
+  if (!tasks.empty() && tasks[0].mixed) launch_eval(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, C.stream, side);
+  else
+    launch_eval64(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, d_next.p, C.num_sms, C.stream, side,
+                  C.count_work);
+  if (two) {
+    HR_CHECK_CUDA(cudaEventRecord(C.ev_join, C.side));
+    HR_CHECK_CUDA(cudaStreamWaitEvent(C.stream, C.ev_join, 0));
+  }
+  launch_reduce(d_tasks.p, ntask_blocks, d_task_blocks.p, d_next.p, C.stream);
   C.launches += 1 + (n_on > 0 ? 1 : 0) + (nitems > n_on ? 1 : 0);
 }
 

@@ -123,6 +123,7 @@ struct DevTree {
   DBuf<int> perm, m0, m1;
   DBuf<double> tcheb;
   DBuf<double> qx, qy, qz;
+  DBuf<double> pk;  // packed records (Pack), up to 12 doubles per source
   DBuf<float> fx, fy, fz, fnx, fny, fnz, fa, fqx, fqy, fqz;  // FP32 copies, centre-relative
   double ctr[3] = {0, 0, 0};
   DBuf<double> mom;  // nn * Pf * C, proxy-major (C = 10 DL symmetric form, 6 SL)
@@ -134,8 +135,9 @@ struct DevTree {
   long long moment_terms = 0;  // sum over non-root nodes of Pf * members
   void build(const hr_surface& S, int P, int N0, double theta, bool direct, cudaStream_t st);
   // density (reference order, interleaved, device) -> tree-order SoA (+ moments)
+  // and packed records as `pack` (PACK_DL: stresslet moments, otherwise Stokeslet);
   // tc: the upward pass on the tensor cores (reduced-precision operator)
-  void set_density(Ctx& C, const double* q3_dev, bool dl, bool moments, bool tc = false);
+  void set_density(Ctx& C, const double* q3_dev, int pack, bool moments, bool tc = false);
 };
 
 // Target data on the device, reference order.
@@ -174,6 +176,7 @@ struct Batch {
   DBuf<int> d_item_start;
   DBuf<int2> d_task_blocks;
   DBuf<double> d_partial;
+  DBuf<unsigned> d_next;  // work counters of the FP64 launches, zero between launches
   int nitems = 0, ntask_blocks = 0;
   int n_on = 0;  // leading lean items (on-surface / box-face tasks, launched on their own)
   bool ready = false;  // finalize has run
