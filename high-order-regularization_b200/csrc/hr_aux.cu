@@ -1,5 +1,7 @@
 // hr_aux.cu — upward pass, density interpolation, permutations, combines and
 // the deterministic vector kernels used by GMRES.
+#include <algorithm>
+
 #include "hr_device.h"
 #include "hr_pairs.cuh"
 
@@ -7,147 +9,251 @@ namespace hr {
 
 namespace {
 
-constexpr int kMomThreads = 384;
-constexpr int kMomTile = 64;  // sources staged per sub-tile
-static_assert(kMomThreads >= 4 * kMomTile, "a thread per (axis, source) and per source for the channels");
 constexpr int kMaxP1 = 16;
 
-// Upward pass of one (node, source range) item: the barycentric Lagrange
-// proxy moments of Panel_Moments_SL / Panel_Moments_DL (2S/KITC.cpp:351-668):
+// Upward pass: the barycentric Lagrange proxy moments of Panel_Moments_SL /
+// Panel_Moments_DL (2S/KITC.cpp:351-668) of one (node, source range) item,
 //   M[c][ijk] = sum_s L_i(x_s) L_j(y_s) L_k(z_s) A_s q_c(s),
 //   L_i(x) = (w_i / (x - t_i)) / sum_m (w_m / (x - t_m)),  w_j = (-1)^j d_j,
 // with the removable singularity |x - t_j| < 1e-7 handled as in the reference.
-// SL channels: f (3), n (3). DL channels: g (x) n (9, g-major), n (3).
-template <bool DL>
-__global__ void __launch_bounds__(kMomThreads) moments_kernel(
-    const MomItem* __restrict__ items, int P1, const double* __restrict__ tcheb,
-    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-    const double* __restrict__ nx, const double* __restrict__ ny, const double* __restrict__ nz,
-    const double* __restrict__ a, const double* __restrict__ qx, const double* __restrict__ qy,
-    const double* __restrict__ qz, double* __restrict__ partial) {
-  constexpr int C = DL ? 12 : 6;
-  __shared__ double sL[3][kMaxP1][kMomTile];  // normalized Lagrange values per axis
-  __shared__ double sA[kMomTile];
-  __shared__ double sQ[C][kMomTile];
-  __shared__ double sT[3 * kMaxP1];
-  const MomItem it = items[blockIdx.x];
-  const int Pf = P1 * P1 * P1;
-  const int tid = threadIdx.x;
-  if (tid < 3 * P1) sT[tid] = tcheb[(size_t)it.node * 3 * P1 + tid];
-  // barycentric weights w_j = (-1)^j d_j, d_0 = d_P = 1/2 (2S/KITC.cpp:365-375)
-  __syncthreads();
-  for (int kk0 = 0; kk0 < Pf; kk0 += kMomThreads) {
-    const int kk = kk0 + tid;
-    const int i = kk / (P1 * P1), j = (kk / P1) % P1, k = kk % P1;
-    double acc[C];
+// SL channels: f (3), n (3). DL channels: the combinations that the far field
+// reads (moments_reduce_kernel): the six of the symmetric part of g (x) n, n (3).
+//
+// It is a contraction, D[(j,k), (c,i)] = sum_s (L_j L_k)(s) (L_i A q_c)(s), and
+// runs on the FP64 matrix instruction (mma m8n8k4): the same 16 multiply-adds
+// per cycle and SM quarter as the FP64 pipe's peak, but with one operand
+// fetch per 8 of them, where the scalar form (one thread per proxy, 5 operands
+// from shared memory per source and channel) was bound by shared-memory reads.
+// A warp owns 4 x 4 tiles of 8 x 8 (8 fragment loads per 16 MMAs, no test per
+// tile: rows and columns are padded with zero fragments to whole groups); a
+// CTA, up to 8 warps, shares the operands of 32 sources at a time, written
+// fragment by fragment (32 consecutive doubles, no bank conflicts). More tiles
+// than 8 warps hold (P > 7) go to further CTAs of the item, so that several
+// CTAs per SM overlap one another's operand and MMA phases.
+// Both surfaces at h = 1/64, P = 6: 220 -> 78 us (stresslet; two launches of 110 us
+// before), the operator application 4.07 -> 3.93 ms; P = 10: the work around the
+// boundary sums 0.96 -> 0.41 ms. 8 x 2 tiles per warp and one CTA of 14 warps per
+// item measured the same (77 / 306 us): the operand phase between the MMAs bounds
+// it now.
+constexpr int kMomSrc = 32, kMomRT = 4, kMomCT = 4, kMomWarps = 8;
+
+struct MomShape {
+  int P1, nrt, nct;  // row and column tiles, in whole groups
+  int jobs;          // warp jobs: row groups x column groups
+  int warps;         // per CTA
+  int ctas;          // per item
+  int smem;          // bytes
+};
+
+MomShape mom_shape(int C, int P1) {
+  MomShape m;
+  m.P1 = P1;
+  m.nrt = ((P1 * P1 + 7) / 8 + kMomRT - 1) / kMomRT * kMomRT;
+  m.nct = ((C * P1 + 7) / 8 + kMomCT - 1) / kMomCT * kMomCT;
+  m.jobs = (m.nrt / kMomRT) * (m.nct / kMomCT);
+  m.ctas = (m.jobs + kMomWarps - 1) / kMomWarps;
+  m.warps = (m.jobs + m.ctas - 1) / m.ctas;
+  m.smem = (int)sizeof(double) * (kMomSrc * 8 * (m.nrt + m.nct) + 3 * P1 * (kMomSrc + 1) + C * kMomSrc + 3 * P1);
+  return m;
+}
+
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+template <int C>
+__global__ void __launch_bounds__(kMomWarps * 32) moments_kernel(MomTree t0, MomTree t1, MomShape sh) {
+  constexpr bool DL = C == 9;
+  extern __shared__ __align__(16) double msm[];
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int P1 = sh.P1, M2 = P1 * P1, Pf = M2 * P1;
+  double* sA = msm;                                   // [source quad][row tile][32]
+  double* sB = sA + kMomSrc * 8 * sh.nrt;             // [source quad][column tile][32]
+  double* sL = sB + kMomSrc * 8 * sh.nct;             // [axis][P1][kMomSrc + 1]
+  double* sQ = sL + 3 * P1 * (kMomSrc + 1);           // [C][kMomSrc]
+  double* sT = sQ + C * kMomSrc;                      // Chebyshev points
+  const bool first = (int)blockIdx.x < t0.nitems;
+  const MomTree& t = first ? t0 : t1;
+  const MomItem it = t.items[first ? blockIdx.x : blockIdx.x - t0.nitems];
+  for (int i = tid; i < 3 * P1; i += nthr) sT[i] = t.tcheb[(size_t)it.node * 3 * P1 + i];
+  const int nrg = sh.nrt / kMomRT;
+  const int job = blockIdx.y * sh.warps + warp;
+  const bool has_job = job < sh.jobs;
+  const int rt0 = (job % nrg) * kMomRT, ct0 = (job / nrg) * kMomCT;
+  double acc[kMomRT][kMomCT][2];
 #pragma unroll
-    for (int c = 0; c < C; c++) acc[c] = 0.0;
-    for (int s0 = it.s0; s0 < it.s1; s0 += kMomTile) {
-      const int cnt = min(kMomTile, it.s1 - s0);
-      __syncthreads();
-      // threads 0..191: the Lagrange values of one (axis, source) each,
-      // normalized by their own axis sum; threads 192..255: area and channel
-      // values of one source each
-      if (tid < 3 * kMomTile) {
-        const int ax = tid / kMomTile, src = tid - ax * kMomTile;
+  for (int r = 0; r < kMomRT; r++)
+#pragma unroll
+    for (int c = 0; c < kMomCT; c++) acc[r][c][0] = acc[r][c][1] = 0.0;
+  __syncthreads();
+  for (int s0 = it.s0; s0 < it.s1; s0 += kMomSrc) {
+    const int cnt = min(kMomSrc, it.s1 - s0);
+    // the Lagrange values of one (axis, source) per thread, normalized by
+    // their own axis sum; then the channels of a source per thread. Beyond the
+    // last source both are zero.
+    for (int e = tid; e < 4 * kMomSrc; e += nthr) {
+      const int ax = e / kMomSrc, src = e - ax * kMomSrc, s = s0 + src;
+      if (ax < 3) {
+        double* L = sL + (ax * P1) * (kMomSrc + 1) + src;
         if (src < cnt) {
-          const int s = s0 + src;
-          const double pc = ax == 0 ? x[s] : (ax == 1 ? y[s] : z[s]);
-          double L[kMaxP1];
+          const double pc = ax == 0 ? t.x[s] : (ax == 1 ? t.y[s] : t.z[s]);
           int flag = -1;
           double S = 0.0;
           for (int jj = 0; jj < P1; jj++) {
+            // barycentric weights w_j = (-1)^j d_j, d_0 = d_P = 1/2 (2S/KITC.cpp:365-375)
             const double w = ((jj % 2 == 0) ? 1.0 : -1.0) * ((jj == 0 || jj == P1 - 1) ? 0.5 : 1.0);
             const double d = pc - sT[ax * P1 + jj];
+            double v = 0.0;
             if (fabs(d) < 1.e-07) {
               flag = jj;
-              L[jj] = 0.0;
             } else {
-              L[jj] = w / d;
-              S += L[jj];
+              v = w / d;
+              S += v;
             }
+            L[jj * (kMomSrc + 1)] = v;
           }
           const double inv = 1.0 / S;
           for (int jj = 0; jj < P1; jj++)
-            sL[ax][jj][src] = (flag > -1) ? (jj == flag ? 1.0 : 0.0) : L[jj] * inv;
+            L[jj * (kMomSrc + 1)] = (flag > -1) ? (jj == flag ? 1.0 : 0.0) : L[jj * (kMomSrc + 1)] * inv;
+        } else {
+          for (int jj = 0; jj < P1; jj++) L[jj * (kMomSrc + 1)] = 0.0;
         }
-      } else if (tid < 4 * kMomTile) {
-        const int src = tid - 3 * kMomTile;
+      } else {
+        double v[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) v[c] = 0.0;
         if (src < cnt) {
-          const int s = s0 + src;
-          sA[src] = a[s];
-          const double n3[3] = {nx[s], ny[s], nz[s]};
-          const double q3[3] = {qx[s], qy[s], qz[s]};
+          const double A = t.a[s], n0 = A * t.nx[s], n1 = A * t.ny[s], n2 = A * t.nz[s];
+          const double q0 = t.qx[s], q1 = t.qy[s], q2 = t.qz[s];
           if (DL) {
-            for (int l = 0; l < 3; l++)
-              for (int m = 0; m < 3; m++) sQ[3 * l + m][src] = q3[l] * n3[m];
-            for (int m = 0; m < 3; m++) sQ[9 + m][src] = n3[m];
+            v[0] = q0 * n0;
+            v[1] = q1 * n1;
+            v[2] = q2 * n2;
+            v[3] = q0 * n1 + q1 * n0;
+            v[4] = q0 * n2 + q2 * n0;
+            v[5] = q1 * n2 + q2 * n1;
           } else {
-            for (int m = 0; m < 3; m++) {
-              sQ[m][src] = q3[m];
-              sQ[3 + m][src] = n3[m];
-            }
+            v[0] = A * q0;
+            v[1] = A * q1;
+            v[2] = A * q2;
+          }
+          v[C - 3] = n0;
+          v[C - 2] = n1;
+          v[C - 1] = n2;
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) sQ[c * kMomSrc + src] = v[c];
+      }
+    }
+    __syncthreads();
+    // operand fragments (a row or column tile at a time per warp): lane l of a
+    // fragment is row (column) l / 4, source l mod 4 of its quad
+    for (int f = warp; f < sh.nrt + sh.nct; f += nthr / 32) {
+      const bool rows = f < sh.nrt;
+      const int tile = rows ? f : f - sh.nrt, n = rows ? sh.nrt : sh.nct, at = tile * 8 + (lane >> 2);
+      const double *u = nullptr, *v = nullptr;  // the two factors, per source
+      if (rows && at < M2) {
+        const int j = at / P1, k = at - j * P1;
+        u = sL + (P1 + j) * (kMomSrc + 1);
+        v = sL + (2 * P1 + k) * (kMomSrc + 1);
+      } else if (!rows && at < C * P1) {
+        const int c = at / P1, i = at - c * P1;
+        u = sL + i * (kMomSrc + 1);
+        v = sQ + c * kMomSrc;
+      }
+      double* o = (rows ? sA : sB) + tile * 32 + lane;
+#pragma unroll
+      for (int q = 0; q < kMomSrc / 4; q++) {
+        const int src = 4 * q + (lane & 3);
+        o[q * n * 32] = u ? u[src] * v[src] : 0.0;
+      }
+    }
+    __syncthreads();
+    if (has_job) {
+      const int nq = (cnt + 3) / 4;
+      const double *pa = sA + rt0 * 32 + lane, *pb = sB + ct0 * 32 + lane;
+#pragma unroll 2
+      for (int q = 0; q < nq; q++) {
+        double fa[kMomRT], fb[kMomCT];
+#pragma unroll
+        for (int r = 0; r < kMomRT; r++) fa[r] = pa[(q * sh.nrt + r) * 32];
+#pragma unroll
+        for (int c = 0; c < kMomCT; c++) fb[c] = pb[(q * sh.nct + c) * 32];
+#pragma unroll
+        for (int r = 0; r < kMomRT; r++)
+#pragma unroll
+          for (int c = 0; c < kMomCT; c++) mma_f64(acc[r][c], fa[r], fb[c]);
+      }
+    }
+    __syncthreads();
+  }
+  if (!has_job) return;
+  // accumulator of a lane: row l / 4, columns 2 (l mod 4) and the next
+#pragma unroll
+  for (int r = 0; r < kMomRT; r++)
+#pragma unroll
+    for (int c = 0; c < kMomCT; c++)
+    {
+        const int row = (rt0 + r) * 8 + (lane >> 2);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int col = (ct0 + c) * 8 + 2 * (lane & 3) + h;
+          if (row < M2 && col < C * P1) {
+            const int ch = col / P1, i = col - ch * P1;
+            t.partial[((size_t)it.out * C + ch) * Pf + (size_t)i * M2 + row] = acc[r][c][h];
           }
         }
-      }
-      __syncthreads();
-      if (kk < Pf) {
-        for (int s = 0; s < cnt; s++) {
-          const double v = sL[0][i][s] * sL[1][j][s] * sL[2][k][s] * sA[s];
-#pragma unroll
-          for (int c = 0; c < C; c++) acc[c] += v * sQ[c][s];
-        }
-      }
     }
-    if (kk < Pf) {
-#pragma unroll
-      for (int c = 0; c < C; c++) partial[((size_t)it.out * C + c) * Pf + kk] = acc[c];
-    }
-  }
 }
 
 // Sums the partial moments of each node in item order (deterministic) and
-// stores them proxy-major. The stresslet's 12 channels
-// (g (x) n, g-major, then n) enter the far field only through
+// stores them proxy-major. The stresslet's channels (g (x) n) enter the far
+// field only through
 //   d.M.d = M00 d0^2 + M11 d1^2 + M22 d2^2 + (M01 + M10) d0 d1
 //         + (M02 + M20) d0 d2 + (M12 + M21) d1 d2   and   Mn.d,
 // so they are stored as those 6 symmetric combinations and Mn: FP64 10
 // doubles per proxy (the last one zero), FP32 12 floats (the last three zero).
-// The Stokeslet's 6 channels (f, n) are stored as they are: FP64 6 doubles,
-// FP32 8 floats (the last two zero).
-__global__ void moments_reduce_kernel(int C, int Pf, const int* __restrict__ item_start,
-                                      const double* __restrict__ partial, double* __restrict__ mom,
-                                      float* __restrict__ momf) {
-  // one thread per (node, proxy, stored value): a value is one channel, or for
-  // the stresslet's symmetric combinations the sum of two, each summed over
-  // the node's items in item order
-  const int node = blockIdx.y, o = blockIdx.z;
-  const int kk = blockIdx.x * blockDim.x + threadIdx.x;
+// The FP64 upward pass gives the combinations (C = 9), the tensor-core one the
+// 12 products g-major, then n (C = 12). The Stokeslet's 6 channels (f, n) are
+// stored as they are: FP64 6 doubles, FP32 8 floats (the last two zero).
+__global__ void moments_reduce_kernel(int C, int Pf, MomTree t0, MomTree t1) {
+  // one thread per (node, proxy, stored value): a value is one channel, or of
+  // 12 channels the sum of two, each summed over the node's items in item order
+  const bool first = (int)blockIdx.x < t0.nn;
+  const MomTree& t = first ? t0 : t1;
+  const int node = first ? blockIdx.x : blockIdx.x - t0.nn, o = blockIdx.z;
+  const int kk = blockIdx.y * blockDim.x + threadIdx.x;
   if (kk >= Pf) return;
-  const bool dl = C == 12;
-  int c0 = o, c1 = -1;
-  if (dl) {
-    const int first[10] = {0, 4, 8, 1, 2, 5, 9, 10, 11, -1};
-    const int second[10] = {-1, -1, -1, 3, 6, 7, -1, -1, -1, -1};
-    c0 = first[o];
-    c1 = second[o];
+  const bool dl = C != 6;
+  int c0 = o < C ? o : -1, c1 = -1;
+  if (C == 12) {
+    const int first_c[10] = {0, 4, 8, 1, 2, 5, 9, 10, 11, -1};
+    const int second_c[10] = {-1, -1, -1, 3, 6, 7, -1, -1, -1, -1};
+    c0 = first_c[o];
+    c1 = second_c[o];
   }
-  const int a = item_start[node], b = item_start[node + 1];
+  const int a = t.item_start[node], b = t.item_start[node + 1];
   double s0 = 0.0, s1 = 0.0;
-  if (c0 >= 0)
-    for (int q = a; q < b; q++) s0 += partial[((size_t)q * C + c0) * Pf + kk];
-  if (c1 >= 0)
-    for (int q = a; q < b; q++) s1 += partial[((size_t)q * C + c1) * Pf + kk];
+  if (c0 >= 0) {
+#pragma unroll 8
+    for (int q = a; q < b; q++) s0 += t.partial[((size_t)q * C + c0) * Pf + kk];
+  }
+  if (c1 >= 0) {
+#pragma unroll 8
+    for (int q = a; q < b; q++) s1 += t.partial[((size_t)q * C + c1) * Pf + kk];
+  }
   const double v = c1 >= 0 ? s0 + s1 : s0;
   const size_t k = (size_t)node * Pf + kk;
   if (dl) {
-    mom[k * 10 + o] = v;  // o = 9: the zero pad
-    momf[k * 12 + o] = (float)v;
-    if (o == 9) momf[k * 12 + 10] = momf[k * 12 + 11] = 0.f;
+    t.mom[k * 10 + o] = v;  // o = 9: the zero pad
+    t.momf[k * 12 + o] = (float)v;
+    if (o == 9) t.momf[k * 12 + 10] = t.momf[k * 12 + 11] = 0.f;
   } else {
-    mom[k * 6 + o] = v;
-    momf[k * 8 + o] = (float)v;
-    if (o == 5) momf[k * 8 + 6] = momf[k * 8 + 7] = 0.f;
+    t.mom[k * 6 + o] = v;
+    t.momf[k * 8 + o] = (float)v;
+    if (o == 5) t.momf[k * 8 + 6] = t.momf[k * 8 + 7] = 0.f;
   }
 }
 
@@ -356,24 +462,19 @@ inline int nblk(long n, int t) { return (int)std::min<long>((n + t - 1) / t, 148
 
 }  // namespace
 
-void launch_moments(int dl, const MomItem* d_items, int nitems, int P1, const double* tcheb,
-                    const double* x, const double* y, const double* z, const double* nx,
-                    const double* ny, const double* nz, const double* a, const double* qx,
-                    const double* qy, const double* qz, double* partial, cudaStream_t st) {
+void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st) {
+  const int nitems = t0.nitems + t1.nitems;
   if (nitems <= 0) return;
-  if (dl)
-    moments_kernel<true><<<nitems, kMomThreads, 0, st>>>(d_items, P1, tcheb, x, y, z, nx, ny, nz, a,
-                                                         qx, qy, qz, partial);
-  else
-    moments_kernel<false><<<nitems, kMomThreads, 0, st>>>(d_items, P1, tcheb, x, y, z, nx, ny, nz,
-                                                          a, qx, qy, qz, partial);
+  const MomShape m = mom_shape(C, P1);
+  auto* fn = C == 9 ? moments_kernel<9> : moments_kernel<6>;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, m.smem);
+  fn<<<dim3(nitems, m.ctas), m.warps * 32, m.smem, st>>>(t0, t1, m);
 }
 
-void launch_moments_reduce(int C, int Pf, int nnodes_out, const int* d_item_start,
-                           const double* partial, double* mom, float* momf, cudaStream_t st) {
-  if (nnodes_out <= 0) return;
-  dim3 grid((Pf + 127) / 128, nnodes_out, C == 12 ? 10 : 6);
-  moments_reduce_kernel<<<grid, 128, 0, st>>>(C, Pf, d_item_start, partial, mom, momf);
+void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, cudaStream_t st) {
+  if (t0.nn + t1.nn <= 0) return;
+  dim3 grid(t0.nn + t1.nn, (Pf + 127) / 128, C == 6 ? 6 : 10);
+  moments_reduce_kernel<<<grid, 128, 0, st>>>(C, Pf, t0, t1);
 }
 
 void launch_permute(int n, const int* perm, const double* q3, double* qx, double* qy, double* qz,

@@ -679,7 +679,7 @@ void plan_matvec(hr_plan2s& P, const double* x_dev, double* y_dev, int prec) {
   hr_plan2s::Inner* in = (prec != HR_FP64 && P.inner) ? P.inner.get() : nullptr;
   DevTree* trees = in ? in->tree : P.tree;
   plan_ready(P);  // the stencils and the FP64 stresslet batch
-  for (int s = 0; s < 2; s++) trees[s].set_density(C, P.xin.p + P.off[s], PACK_DL, tree, prec != HR_FP64);
+  set_densities(C, &trees[0], &trees[1], P.xin.p + P.off[0], P.xin.p + P.off[1], PACK_DL, tree, prec != HR_FP64);
   for (int t = 0; t < 2; t++) {
     P.tg[t].g0.zero(st);
     launch_interp(P.sten[t].ne, P.sten[t].tgt.p, P.sten[t].idx.p, P.sten[t].pq.p,
@@ -707,7 +707,7 @@ void plan_rhs(hr_plan2s& P, const double* f1_dev, const double* f2_dev, double* 
   if (f2_dev != P.fin.p + P.off[1])
     HR_CHECK_CUDA(cudaMemcpyAsync(P.fin.p + P.off[1], f2_dev, sizeof(double) * 3 * P.nq[1],
                                   cudaMemcpyDeviceToDevice, st));
-  for (int s = 0; s < 2; s++) P.tree[s].set_density(C, P.fin.p + P.off[s], PACK_SL, tree);
+  set_densities(C, &P.tree[0], &P.tree[1], P.fin.p + P.off[0], P.fin.p + P.off[1], PACK_SL, tree, false);
   P.sl.launch(C);
   // SL_1 = on1 + comp2 ; SL_2 = comp1 + on2 ; b = -SL * 2/3
   launch_rhs_combine(3 * P.nq[0], 2.0 / 3.0, P.out_on[0].p, P.out_off[0].p, b_dev + P.off[0], st);

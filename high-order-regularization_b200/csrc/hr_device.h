@@ -109,19 +109,27 @@ void solve_poisson_dev(struct Ctx& C, int N, double L, const uint8_t* band2_dev,
                        const double* p_dev, double* u_dev, int variable, PoissonWork* work = nullptr);
 
 // Tensor-core (tcgen05, 3xTF32) upward pass for the reduced-precision operator:
-// same items and partial layout as launch_moments; a timed-out wait sets *err.
+// the same items; partial moments of 12 (stresslet) or 6 channels per item; a timed-out wait sets *err.
 bool moments_tc_supported(int P1);
 size_t moments_tc_smem(int dl, int P1, int* npad, int* cols);
 void launch_moments_tc(int dl, const MomItem* d_items, int nitems, int P1, const double* tcheb, const double* x,
                        const double* y, const double* z, const double* nx, const double* ny, const double* nz,
                        const double* a, const double* qx, const double* qy, const double* qz, double* partial,
                        int* err, cudaStream_t st);
-void launch_moments(int dl, const MomItem* d_items, int nitems, int P1, const double* tcheb,
-                    const double* x, const double* y, const double* z, const double* nx,
-                    const double* ny, const double* nz, const double* a, const double* qx,
-                    const double* qy, const double* qz, double* partial, cudaStream_t st);
-void launch_moments_reduce(int C, int Pf, int nnodes_out, const int* d_item_start,
-                           const double* partial, double* mom, float* momf, cudaStream_t st);
+// One tree's part of an upward pass.
+struct MomTree {
+  const MomItem* items;
+  int nitems, nn;  // items, nodes
+  const int* item_start;
+  const double *tcheb, *x, *y, *z, *nx, *ny, *nz, *a, *qx, *qy, *qz;
+  double *partial, *mom;
+  float* momf;
+};
+// FP64 upward pass of one or two trees (the second may be empty) of the same
+// degree: C = 9 stresslet, 6 Stokeslet channels; then the reduction per node (C
+// = 12: the layout of launch_moments_tc).
+void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st);
+void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, cudaStream_t st);
 
 // Gathers interleaved reference-order density into tree-order SoA.
 // and fills the density of the packed records pk (xyz, normals and areas of

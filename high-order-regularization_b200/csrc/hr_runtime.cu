@@ -214,26 +214,46 @@ void Ctx::check_tc() {
   }
 }
 
+MomTree DevTree::mom_tree() const {
+  return {items.p, nitems, nn, item_start.p, tcheb.p, x.p, y.p, z.p, nx.p, ny.p, nz.p, a.p, qx.p, qy.p, qz.p,
+          partial.p, mom.p, momf.p};
+}
+
 void DevTree::set_density(Ctx& C, const double* q3_dev, int pack, bool moments, bool tc) {
+  set_densities(C, this, nullptr, q3_dev, nullptr, pack, moments, tc);
+}
+
+void set_densities(Ctx& C, DevTree* t0, DevTree* t1, const double* q0, const double* q1, int pack, bool moments,
+                   bool tc) {
   const bool dl = pack == PACK_DL;
-  launch_permute(n, perm.p, q3_dev, qx.p, qy.p, qz.p, fqx.p, fqy.p, fqz.p,
-                 {x.p, y.p, z.p, nx.p, ny.p, nz.p, a.p, pk.p, pack}, C.stream);
-  C.launches++;
-  if (moments && nitems > 0 && tc && moments_tc_supported(P1)) {
+  for (int s = 0; s < 2; s++) {
+    DevTree* t = s == 0 ? t0 : t1;
+    if (!t) continue;
+    launch_permute(t->n, t->perm.p, s == 0 ? q0 : q1, t->qx.p, t->qy.p, t->qz.p, t->fqx.p, t->fqy.p, t->fqz.p,
+                   {t->x.p, t->y.p, t->z.p, t->nx.p, t->ny.p, t->nz.p, t->a.p, t->pk.p, pack}, C.stream);
+    C.launches++;
+  }
+  if (!moments || t0->nitems + (t1 ? t1->nitems : 0) == 0) return;
+  const MomTree m0 = t0->mom_tree(), m1 = t1 ? t1->mom_tree() : MomTree{};
+  int ch = dl ? 9 : 6;
+  if (tc && moments_tc_supported(t0->P1)) {
     if (!C.tc_err.p) {
       C.tc_err.alloc(1);
       C.tc_err.zero(C.stream);
     }
-    launch_moments_tc(dl ? 1 : 0, items.p, nitems, P1, tcheb.p, x.p, y.p, z.p, nx.p, ny.p, nz.p, a.p, qx.p, qy.p,
-                      qz.p, partial.p, C.tc_err.p, C.stream);
-    launch_moments_reduce(dl ? 12 : 6, Pf, nn, item_start.p, partial.p, mom.p, momf.p, C.stream);
-    C.launches += 2;
-  } else if (moments && nitems > 0) {
-    launch_moments(dl ? 1 : 0, items.p, nitems, P1, tcheb.p, x.p, y.p, z.p, nx.p, ny.p, nz.p, a.p,
-                   qx.p, qy.p, qz.p, partial.p, C.stream);
-    launch_moments_reduce(dl ? 12 : 6, Pf, nn, item_start.p, partial.p, mom.p, momf.p, C.stream);
-    C.launches += 2;
+    for (DevTree* t : {t0, t1}) {
+      if (!t || t->nitems == 0) continue;
+      launch_moments_tc(dl ? 1 : 0, t->items.p, t->nitems, t->P1, t->tcheb.p, t->x.p, t->y.p, t->z.p, t->nx.p, t->ny.p,
+                        t->nz.p, t->a.p, t->qx.p, t->qy.p, t->qz.p, t->partial.p, C.tc_err.p, C.stream);
+      C.launches++;
+    }
+    ch = dl ? 12 : 6;
+  } else {
+    launch_moments(ch, t0->P1, m0, m1, C.stream);
+    C.launches++;
   }
+  launch_moments_reduce(ch, t0->Pf, m0, m1, C.stream);
+  C.launches++;
 }
 
 void DevLists::build(const Tree& T, int nt, const double* txyz, const uint8_t* near,

@@ -138,7 +138,12 @@ struct DevTree {
   // and packed records as `pack` (PACK_DL: stresslet moments, otherwise Stokeslet);
   // tc: the upward pass on the tensor cores (reduced-precision operator)
   void set_density(Ctx& C, const double* q3_dev, int pack, bool moments, bool tc = false);
+  MomTree mom_tree() const;
 };
+
+// set_density of two trees of one degree (t1 may be null), their upward passes in one launch.
+void set_densities(Ctx& C, DevTree* t0, DevTree* t1, const double* q0, const double* q1, int pack, bool moments,
+                   bool tc);
 
 // Target data on the device, reference order.
 struct DevTargets {
