@@ -268,9 +268,11 @@ __global__ void permute_kernel(int n, const int* __restrict__ perm, const double
   qx[p] = a;
   qy[p] = b;
   qz[p] = c;
-  fqx[p] = (float)a;
-  fqy[p] = (float)b;
-  fqz[p] = (float)c;
+  if (fqx) {
+    fqx[p] = (float)a;
+    fqy[p] = (float)b;
+    fqz[p] = (float)c;
+  }
   const double w = ps.a[p], wq = ps.pack == PACK_SL ? w : 1.0;
   if (ps.pack == PACK_E2G) {
     double2* r = reinterpret_cast<double2*>(ps.pk) + 6 * (size_t)p;

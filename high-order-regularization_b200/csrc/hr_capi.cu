@@ -7,6 +7,7 @@
 #include <memory>
 #include <mutex>
 #include <exception>
+#include <numeric>
 #include <random>
 #include <thread>
 #include <vector>
@@ -87,38 +88,17 @@ std::vector<uint8_t> near_flags(int n, const double* b, double delta) {
   return v;
 }
 
+// Target data; an array that is not given is not needed by the sums it is for.
 void upload_targets(DevTargets& tg, int n, const double* xyz, const double* b, const double* x0,
                     const double* n0, const double* f0, const double* nrm,
                     const std::vector<uint8_t>& near, cudaStream_t st) {
   tg.n = n;
   tg.xyz.upload(xyz, 3 * (size_t)n, st);
   if (b) tg.b.upload(b, n, st);
-  else {
-    tg.b.alloc(n);
-    tg.b.zero(st);
-  }
   if (x0) tg.x0.upload(x0, 3 * (size_t)n, st);
-  else {
-    tg.x0.alloc(3 * (size_t)n);
-    tg.x0.zero(st);
-  }
   if (n0) tg.n0.upload(n0, 3 * (size_t)n, st);
-  else {
-    tg.n0.alloc(3 * (size_t)n);
-    tg.n0.zero(st);
-  }
   if (f0) tg.f0.upload(f0, 3 * (size_t)n, st);
-  else {
-    tg.f0.alloc(3 * (size_t)n);
-    tg.f0.zero(st);
-  }
-  tg.g0.alloc(3 * (size_t)n);
-  tg.g0.zero(st);
   if (nrm) tg.nrm.upload(nrm, 3 * (size_t)n, st);
-  else {
-    tg.nrm.alloc(3 * (size_t)n);
-    tg.nrm.zero(st);
-  }
   tg.near.upload(near, st);
 }
 
@@ -173,21 +153,37 @@ void single_eval(Ctx& C, int kind, const hr_eval_opts* opt, double delta, const 
     return;
   }
   HR_REQUIRE(dens, "density missing");
+  // every buffer of the call from the context's workspace, every small upload in one copy
+  WorkspaceScope scope(C);
+  const bool reduced = opt && opt->precision != HR_FP64;
   DevTree tree;
-  tree.build(*S, P, N0, theta, direct, st);
+  tree.build(*S, P, N0, theta, direct, st, reduced);
   DBuf<double> q3;
   q3.upload(dens, 3 * (size_t)S->n, st);
-  tree.set_density(C, q3.p, kind > K_DL_OFF ? PACK_E2G : (dl ? PACK_DL : PACK_SL), !direct,
-                   opt && opt->precision != HR_FP64);
-  std::vector<uint8_t> near =
-      (kind == K_SL_OFF || kind == K_DL_OFF) ? near_flags(nt, b, delta) : std::vector<uint8_t>(nt, 1);
+  const bool off = kind == K_SL_OFF || kind == K_DL_OFF, e2g7 = kind == K_E2G_SL7 || kind == K_E2G_P7;
+  std::vector<uint8_t> near = off ? near_flags(nt, b, delta) : std::vector<uint8_t>(nt, 1);
   DevTargets tg;
-  upload_targets(tg, nt, txyz, on ? nullptr : b, x0, n0,
-                 (kind == K_SL_OFF || kind == K_E2G_SL7 || kind == K_E2G_P7) ? dens0 : nullptr,
-                 on ? S->nrml : nullptr, near, st);
-  if (kind == K_DL_OFF && dens0) tg.g0.upload(dens0, 3 * (size_t)nt, st);
+  upload_targets(tg, nt, txyz, off || e2g7 ? b : nullptr, kind == K_DL_OFF ? x0 : nullptr,
+                 off || e2g7 ? n0 : nullptr, kind == K_SL_OFF || e2g7 ? dens0 : nullptr,
+                 kind == K_SL_ON ? S->nrml : nullptr, near, st);
+  if (kind == K_DL_OFF) tg.g0.upload(dens0, 3 * (size_t)nt, st);
+  // Target blocks. A treecode's lists, and the FP32 sums (coordinates relative
+  // to a block's first target), take the full Morton order. In an FP64 direct
+  // sum the order changes no target's result; it only decides which targets
+  // share a warp's branches, for which 128 cells per axis do (two of the sort's
+  // six passes: 1.9 -> 0.6 ms of host time for 55,298 targets), and the plain
+  // box-face sums have no branches at all.
+  std::vector<int> order;
+  if (direct && !reduced) {
+    if (kind == K_E2G_SL_AWAY || kind == K_E2G_P_AWAY) {
+      order.resize(nt);
+      std::iota(order.begin(), order.end(), 0);
+    } else {
+      order = morton_order(nt, txyz, 7);
+    }
+  }
   DevLists L;
-  L.build(tree.host, nt, txyz, near.data(), st);
+  L.build(tree.host, nt, txyz, near.data(), st, order.empty() ? nullptr : &order);
   DBuf<double> d_out;
   d_out.alloc((size_t)odim * nt);
   double scale;
@@ -208,11 +204,12 @@ void single_eval(Ctx& C, int kind, const hr_eval_opts* opt, double delta, const 
   B.lists.push_back(&L.host);
   B.trees.push_back(&tree.host);
   B.finalize(st, C.num_sms);
+  C.ws.flush(st);
+  tree.set_density(C, q3.p, kind > K_DL_OFF ? PACK_E2G : (dl ? PACK_DL : PACK_SL), !direct, reduced);
   B.launch(C);
   HR_CHECK_CUDA(cudaGetLastError());
-  HR_CHECK_CUDA(cudaMemcpyAsync(out, d_out.p, sizeof(double) * odim * nt, cudaMemcpyDeviceToHost, st));
-  HR_CHECK_CUDA(cudaStreamSynchronize(st));
-  if (opt && opt->precision != HR_FP64) C.check_tc();
+  d2h_staged(C, out, d_out.p, sizeof(double) * odim * nt);
+  if (reduced) C.check_tc();
 }
 
 }  // namespace
@@ -238,6 +235,8 @@ extern "C" int hr_ctx_create(int device, hr_ctx** out) {
     HR_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->c.ev_join, cudaEventDisableTiming));
     ctx->c.counters.alloc(64);
     ctx->c.counters.zero(ctx->c.stream);
+    ctx->c.tc_err.alloc(1);
+    ctx->c.tc_err.zero(ctx->c.stream);
   });
   if (rc != HR_OK) return rc;
   *out = ctx.release();
@@ -254,6 +253,8 @@ extern "C" void hr_ctx_destroy(hr_ctx* ctx) {
   if (ctx->c.stream) {
     cudaStreamSynchronize(ctx->c.stream);
     ctx->c.counters.release();
+    ctx->c.tc_err.release();
+    ctx->c.ws.free_all();
     cudaStreamDestroy(ctx->c.stream);
   }
   if (ctx->c.ev_fork) cudaEventDestroy(ctx->c.ev_fork);
@@ -374,6 +375,7 @@ extern "C" int hr_interpolate_dl_density(hr_ctx* ctx, double h, const hr_surface
     HR_CHECK_CUDA(cudaSetDevice(ctx->c.device));
     cudaStream_t st = ctx->c.stream;
     check_i123(T->n, T->nrst, T->i123);
+    WorkspaceScope scope(ctx->c);
     Stencils s = build_stencils(h, S->center, S->n, S->xyz, T->n, T->nrst, T->x0, T->i123);
     if (S->n == 0) {
       for (size_t e = 0; e < s.tgt.size(); e++) HR_REQUIRE(false, "interpolation from an empty surface");
@@ -384,11 +386,11 @@ extern "C" int hr_interpolate_dl_density(hr_ctx* ctx, double h, const hr_surface
     dg.upload(g, 3 * (size_t)std::max(1, S->n), st);
     dg0.alloc(3 * (size_t)std::max(1, T->n));
     dg0.zero(st);
+    ctx->c.ws.flush(st);
     launch_interp(ds.ne, ds.tgt.p, ds.idx.p, ds.pq.p, dg.p, dg0.p, st);
     ctx->c.launches++;
     HR_CHECK_CUDA(cudaGetLastError());
-    HR_CHECK_CUDA(cudaMemcpyAsync(g0, dg0.p, sizeof(double) * 3 * T->n, cudaMemcpyDeviceToHost, st));
-    HR_CHECK_CUDA(cudaStreamSynchronize(st));
+    d2h_staged(ctx->c, g0, dg0.p, sizeof(double) * 3 * T->n);
   });
 }
 
@@ -397,13 +399,13 @@ extern "C" int hr_dst_poisson3d(hr_ctx* ctx, int n, double* f) {
   return guard(ctx, [&] {
     HR_REQUIRE(n >= 1 && f, "bad DST arguments");
     HR_CHECK_CUDA(cudaSetDevice(ctx->c.device));
-    cudaStream_t st = ctx->c.stream;
     size_t m = (size_t)n * n * n;
+    WorkspaceScope scope(ctx->c);
     DBuf<double> d;
-    d.upload(f, m, st);
+    d.alloc(m);
+    h2d_staged(ctx->c, d.p, f, m * sizeof(double));
     dst_poisson3d_dev(ctx->c, n, d.p);
-    HR_CHECK_CUDA(cudaMemcpyAsync(f, d.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-    HR_CHECK_CUDA(cudaStreamSynchronize(st));
+    d2h_staged(ctx->c, f, d.p, m * sizeof(double));
   });
 }
 
@@ -468,15 +470,21 @@ extern "C" int hr_e2g_solve_poisson(hr_ctx* ctx, int N, double L, const uint8_t*
     HR_CHECK_CUDA(cudaSetDevice(ctx->c.device));
     cudaStream_t st = ctx->c.stream;
     size_t m = (size_t)(N + 1) * (N + 1) * (N + 1);
+    WorkspaceScope scope(ctx->c);
     DBuf<uint8_t> db, dout;
     DBuf<double> dp, du;
-    db.upload(band2, m, st);
-    dout.upload(outside, m, st);
-    if (p) dp.upload(p, m, st);
-    du.upload(u, m, st);
+    db.alloc(m);
+    dout.alloc(m);
+    du.alloc(m);
+    h2d_staged(ctx->c, db.p, band2, m);
+    h2d_staged(ctx->c, dout.p, outside, m);
+    if (p) {
+      dp.alloc(m);
+      h2d_staged(ctx->c, dp.p, p, m * sizeof(double));
+    }
+    h2d_staged(ctx->c, du.p, u, m * sizeof(double));
     solve_poisson_dev(ctx->c, N, L, db.p, dout.p, p ? dp.p : nullptr, du.p, variable);
-    HR_CHECK_CUDA(cudaMemcpyAsync(u, du.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-    HR_CHECK_CUDA(cudaStreamSynchronize(st));
+    d2h_staged(ctx->c, u, du.p, m * sizeof(double));
   });
 }
 
@@ -979,6 +987,8 @@ extern "C" int hr_plan2s_create(hr_ctx* ctx, const hr_scene2s* sc, const hr_eval
       P->near_host[t] = near;
       upload_targets(P->tg[t], T.n, sc->surf[t].xyz, T.b, T.x0, T.n0, sc->f0[t], sc->surf[t].nrml,
                      near, st);
+      P->tg[t].g0.alloc(3 * (size_t)T.n);
+      P->tg[t].g0.zero(st);
       std::vector<uint8_t> all(T.n, 1);
       const std::vector<int> mo = morton_order(T.n, sc->surf[t].xyz);  // shared by both lists
       P->Lon[t].build(P->tree[t].host, T.n, sc->surf[t].xyz, all.data(), st, &mo);

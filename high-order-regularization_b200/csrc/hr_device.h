@@ -26,10 +26,7 @@ struct EvalTask {
   const double *sx, *sy, *sz, *snx, *sny, *snz, *sa;  // sources, tree order
   const double *qx, *qy, *qz;                         // density, tree order
   const double* pk;                                   // packed sources, tree order (Pack), for the FP64 sums
-  double ctr[3];                                      // source surface centre (FP32 frame origin)
-  // FP32 copies for the mixed-precision far field: positions relative to ctr
-  const float *fx, *fy, *fz, *fnx, *fny, *fnz, *fa, *fqx, *fqy, *fqz;
-  const int *node_m0, *node_m1;                       // inclusive member ranges
+  const float *fnx, *fny, *fnz, *fa, *fqx, *fqy, *fqz;  // FP32 copies (reduced-precision sums)
   const double* tcheb;                                // 3*P1 per node
   const double* mom;                                  // Pf*C per node, proxy-major
   const float* momf;                                  // Pf*W32 per node (W32 = 12 DL, 8 SL)
@@ -44,7 +41,6 @@ struct EvalTask {
   double* out2;                                       // nt pressure of K_E2G_UP_AWAY (scaled by scale2)
   double scale2;
   const Entry* entries;                               // interaction entries
-  const int* blk_start;                               // per target block, into entries
   unsigned long long* counters;  // [0] regularized pairs [1] near-target plain [2] far-target [3] proxy
   const int* item_start;  // per target block: its work items' partial slots [start, end)
   double* partial;        // 3 x 128 doubles per work item

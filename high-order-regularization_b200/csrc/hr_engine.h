@@ -85,7 +85,8 @@ struct Stencils {
 Stencils build_stencils(double h, const double ctr[3], int nq, const double* xq, int nt,
                         const int* nrst, const double* x0, const int* i123);
 
-// Morton order of points (stable), used to form spatially coherent target blocks.
-std::vector<int> morton_order(int n, const double* xyz);
+// Morton order of points (stable), used to form spatially coherent target blocks;
+// bits per axis (at most 21).
+std::vector<int> morton_order(int n, const double* xyz, int bits = 21);
 
 }  // namespace hr

@@ -774,6 +774,7 @@ struct DstPlan {
     if (reg_R) lanetab.upload(dst_reg_table(reg_R, t, st), C.stream);
     evc.upload(c, C.stream);
     evs.upload(s, C.stream);
+    if (Workspace* ws = active_workspace()) ws->flush(C.stream);
   }
   // one pass: in [n][n][n] -> out rotated (or into u for mode 2)
   void pass(Ctx& C, const double* in, double* out, int mode, double scale, const double* w, double* u) {
@@ -805,8 +806,9 @@ void dst_poisson3d_dev(Ctx& C, int n, double* f_dev) {
   DstPlan P;
   P.make(C, n);
   P.solve(C, f_dev, 3, 1. / pow(2 * (n + 1), 3), nullptr, nullptr);
-  // the plan's buffers are freed at return and must be idle first
-  HR_CHECK_CUDA(cudaStreamSynchronize(C.stream));
+  // the plan's buffers go at return and must be idle first (in a workspace they
+  // are not used again before the call's own end)
+  if (!active_workspace()) HR_CHECK_CUDA(cudaStreamSynchronize(C.stream));
 }
 
 // A plain 3D DST-I (FFTW's RODFT00 on all three axes, unnormalised) of an

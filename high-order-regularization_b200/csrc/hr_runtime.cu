@@ -69,46 +69,156 @@ void dev_free(void* p) noexcept {
   }
 }
 
-void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
-  cudaStream_t st = C.stream;
-  if (bytes <= 2 * kPinChunk) {
-    HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
-    HR_CHECK_CUDA(cudaStreamSynchronize(st));
-    return;
+Workspace*& active_workspace() {
+  static thread_local Workspace* w = nullptr;
+  return w;
+}
+
+void* Workspace::take(size_t bytes, bool up) {
+  bytes = (bytes + 255) & ~size_t(255);
+  want_dev += bytes;
+  if (up) want_pin += bytes;
+  if (low + bytes > dev_cap - high || (up && low + bytes > pin_cap)) return nullptr;
+  if (up) {
+    low += bytes;
+    return dev + low - bytes;
   }
+  high += bytes;
+  return dev + dev_cap - high;
+}
+
+void Workspace::flush(cudaStream_t st) {
+  if (low > flushed) HR_CHECK_CUDA(cudaMemcpyAsync(dev + flushed, pin + flushed, low - flushed, cudaMemcpyHostToDevice, st));
+  flushed = low;
+}
+
+void Workspace::free_all() {
+  if (dev) dev_free(dev);
+  if (pin) cudaFreeHost(pin);
+  dev = pin = nullptr;
+  dev_cap = pin_cap = 0;
+}
+
+WorkspaceScope::WorkspaceScope(Ctx& c) : C(c) {
+  Workspace& w = C.ws;
+  w.low = w.high = w.flushed = w.want_dev = w.want_pin = 0;
+  active_workspace() = &w;
+}
+
+WorkspaceScope::~WorkspaceScope() {
+  Workspace& w = C.ws;
+  active_workspace() = nullptr;
+  cudaStreamSynchronize(C.side);
+  cudaStreamSynchronize(C.stream);
+  // the buffers of this call are idle; the next call finds room for its like
+  // (powers of two, so that slowly growing calls do not allocate each time)
+  auto grown = [](size_t want, size_t limit) {
+    size_t c = size_t(1) << 20;
+    while (c < want) c *= 2;
+    return std::min(c, limit);
+  };
+  try {
+    if (w.want_dev > w.dev_cap && w.dev_cap < Workspace::kDevMax) {
+      if (w.dev) dev_free(w.dev);
+      w.dev = nullptr;
+      w.dev_cap = 0;
+      const size_t c = grown(w.want_dev, Workspace::kDevMax);
+      w.dev = static_cast<char*>(dev_alloc(c));
+      w.dev_cap = c;
+    }
+    if (w.want_pin > w.pin_cap && w.pin_cap < Workspace::kPinMax) {
+      if (w.pin) cudaFreeHost(w.pin);
+      w.pin = nullptr;
+      w.pin_cap = 0;
+      const size_t c = grown(w.want_pin, Workspace::kPinMax);
+      void* p = nullptr;
+      if (cudaMallocHost(&p, c) == cudaSuccess) {
+        w.pin = static_cast<char*>(p);
+        w.pin_cap = c;
+      } else {
+        cudaGetLastError();
+      }
+    }
+  } catch (...) {  // no memory to keep: the next call allocates as it goes
+  }
+}
+
+namespace {
+
+// The two pinned buffers; chunks of an eighth of the copy, 512 KB to kPinChunk.
+size_t staging(Ctx& C, size_t bytes) {
   if (!C.pin) {
     HR_CHECK_CUDA(cudaMallocHost(&C.pin, 2 * kPinChunk));
     for (auto& e : C.pin_ev) HR_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
+  const size_t c = (bytes / 8 + 4095) & ~size_t(4095);
+  return std::min(kPinChunk, std::max(size_t(512) << 10, c));
+}
+
+void copy_parallel(char* out, const char* in, size_t n) {
+  constexpr size_t kPart = size_t(128) << 10;  // bytes per host thread's piece
+  const long nparts = (long)((n + kPart - 1) / kPart);
+#pragma omp parallel for schedule(static)
+  for (long q = 0; q < nparts; q++) {
+    const size_t o = (size_t)q * kPart;
+    std::memcpy(out + o, in + o, std::min(kPart, n - o));
+  }
+}
+
+constexpr size_t kStageMin = size_t(1) << 20;  // smaller copies gain nothing from staging
+
+}  // namespace
+
+void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
+  cudaStream_t st = C.stream;
+  if (bytes < kStageMin) {
+    HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+    HR_CHECK_CUDA(cudaStreamSynchronize(st));
+    return;
+  }
+  const size_t chunk = staging(C, bytes);
   char* buf[2] = {static_cast<char*>(C.pin), static_cast<char*>(C.pin) + kPinChunk};
   const char* s = static_cast<const char*>(src);
   char* d = static_cast<char*>(dst);
-  const size_t nch = (bytes + kPinChunk - 1) / kPinChunk;
-  auto len = [&](size_t k) { return std::min(kPinChunk, bytes - k * kPinChunk); };
+  const size_t nch = (bytes + chunk - 1) / chunk;
+  auto len = [&](size_t k) { return std::min(chunk, bytes - k * chunk); };
   auto enqueue = [&](size_t k) {
-    HR_CHECK_CUDA(cudaMemcpyAsync(buf[k & 1], s + k * kPinChunk, len(k), cudaMemcpyDeviceToHost, st));
+    HR_CHECK_CUDA(cudaMemcpyAsync(buf[k & 1], s + k * chunk, len(k), cudaMemcpyDeviceToHost, st));
     HR_CHECK_CUDA(cudaEventRecord(C.pin_ev[k & 1], st));
   };
   enqueue(0);
-  enqueue(1);
-  constexpr size_t kPart = size_t(1) << 20;  // bytes per host thread's piece
+  if (nch > 1) enqueue(1);
   for (size_t k = 0; k < nch; k++) {
     HR_CHECK_CUDA(cudaEventSynchronize(C.pin_ev[k & 1]));
-    const size_t n = len(k);
-    char* out = d + k * kPinChunk;
-    const char* in = buf[k & 1];
-    const long nparts = (long)((n + kPart - 1) / kPart);
-#pragma omp parallel for schedule(static)
-    for (long q = 0; q < nparts; q++) {
-      const size_t o = (size_t)q * kPart;
-      std::memcpy(out + o, in + o, std::min(kPart, n - o));
-    }
+    copy_parallel(d + k * chunk, buf[k & 1], len(k));
     if (k + 2 < nch) enqueue(k + 2);
   }
 }
 
+void h2d_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
+  cudaStream_t st = C.stream;
+  if (bytes < kStageMin) {
+    HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+    return;
+  }
+  const size_t chunk = staging(C, bytes);
+  char* buf[2] = {static_cast<char*>(C.pin), static_cast<char*>(C.pin) + kPinChunk};
+  const char* s = static_cast<const char*>(src);
+  char* d = static_cast<char*>(dst);
+  const size_t nch = (bytes + chunk - 1) / chunk;
+  // the buffers may hold the last chunks of an earlier upload
+  for (auto& e : C.pin_ev) HR_CHECK_CUDA(cudaEventSynchronize(e));
+  for (size_t k = 0; k < nch; k++) {
+    const size_t n = std::min(chunk, bytes - k * chunk);
+    HR_CHECK_CUDA(cudaEventSynchronize(C.pin_ev[k & 1]));
+    copy_parallel(buf[k & 1], s + k * chunk, n);
+    HR_CHECK_CUDA(cudaMemcpyAsync(d + k * chunk, buf[k & 1], n, cudaMemcpyHostToDevice, st));
+    HR_CHECK_CUDA(cudaEventRecord(C.pin_ev[k & 1], st));
+  }
+}
+
 void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direct,
-                    cudaStream_t st) {
+                    cudaStream_t st, bool fp32) {
   HR_REQUIRE(S.n >= 0 && (S.n == 0 || (S.xyz && S.nrml && S.area)), "surface arrays missing");
   HR_REQUIRE(P >= 1 && P + 1 <= 16, "treecode degree P must be in [1, 15]");
   HR_REQUIRE(N0 >= 1, "leaf size N0 must be >= 1");
@@ -136,28 +246,19 @@ void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direc
   nz.upload(hnz, st);
   a.upload(ha, st);
   perm.upload(host.perm, st);
-  m0.upload(host.m0, st);
-  m1.upload(host.m1, st);
   tcheb.upload(host.tcheb, st);
   qx.alloc(n);
   qy.alloc(n);
   qz.alloc(n);
   pk.alloc(12 * (size_t)n);
-  for (int k = 0; k < 3; k++) ctr[k] = S.center[k];
-  {
-    std::vector<float> a0(n), a1(n), a2(n), b0(n), b1(n), b2(n), c0(n);
+  if (fp32) {
+    std::vector<float> b0(n), b1(n), b2(n), c0(n);
     for (int p = 0; p < n; p++) {
-      a0[p] = (float)(hx[p] - ctr[0]);
-      a1[p] = (float)(hy[p] - ctr[1]);
-      a2[p] = (float)(hz[p] - ctr[2]);
       b0[p] = (float)hnx[p];
       b1[p] = (float)hny[p];
       b2[p] = (float)hnz[p];
       c0[p] = (float)ha[p];
     }
-    fx.upload(a0, st);
-    fy.upload(a1, st);
-    fz.upload(a2, st);
     fnx.upload(b0, st);
     fny.upload(b1, st);
     fnz.upload(b2, st);
@@ -166,6 +267,7 @@ void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direc
     fqy.alloc(n);
     fqz.alloc(n);
   }
+  if (direct) return;  // no far field
   // upward-pass items: every non-root node (the root's moments stay zero, as
   // in the reference, which skips it: 2S/KITC.cpp:1446), in chunks of sources.
   // Chunks of at most 512 sources, smaller when the tree is small so that the
@@ -181,7 +283,7 @@ void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direc
   moment_terms = 0;
   for (int c = 0; c < nn; c++) {
     start[c] = (int)it.size();
-    if (c == 0 || direct) continue;
+    if (c == 0) continue;
     for (int s = host.m0[c]; s <= host.m1[c]; s += chunk) {
       MomItem m;
       m.node = c;
@@ -237,10 +339,6 @@ void set_densities(Ctx& C, DevTree* t0, DevTree* t1, const double* q0, const dou
   const MomTree m0 = t0->mom_tree(), m1 = t1 ? t1->mom_tree() : MomTree{};
   int ch = dl ? 9 : 6;
   if (tc && moments_tc_supported(t0->P1)) {
-    if (!C.tc_err.p) {
-      C.tc_err.alloc(1);
-      C.tc_err.zero(C.stream);
-    }
     for (DevTree* t : {t0, t1}) {
       if (!t || t->nitems == 0) continue;
       launch_moments_tc(dl ? 1 : 0, t->items.p, t->nitems, t->P1, t->tcheb.p, t->x.p, t->y.p, t->z.p, t->nx.p, t->ny.p,
@@ -260,7 +358,6 @@ void DevLists::build(const Tree& T, int nt, const double* txyz, const uint8_t* n
                      cudaStream_t st, const std::vector<int>* morton) {
   host = build_lists(T, nt, txyz, near, morton);
   tord.upload(host.tord, st);
-  blk_start.upload(host.blk_start, st);
   entries.upload(host.entries, st);
 }
 
@@ -295,10 +392,6 @@ EvalTask make_task(int kind, double DEL, double scale, const DevTree& T, const D
   k.qy = T.qy.p;
   k.qz = T.qz.p;
   k.pk = T.pk.p;
-  for (int c = 0; c < 3; c++) k.ctr[c] = T.ctr[c];
-  k.fx = T.fx.p;
-  k.fy = T.fy.p;
-  k.fz = T.fz.p;
   k.fnx = T.fnx.p;
   k.fny = T.fny.p;
   k.fnz = T.fnz.p;
@@ -306,8 +399,6 @@ EvalTask make_task(int kind, double DEL, double scale, const DevTree& T, const D
   k.fqx = T.fqx.p;
   k.fqy = T.fqy.p;
   k.fqz = T.fqz.p;
-  k.node_m0 = T.m0.p;
-  k.node_m1 = T.m1.p;
   k.tcheb = T.tcheb.p;
   k.mom = T.mom.p;
   k.momf = T.momf.p;
@@ -323,7 +414,6 @@ EvalTask make_task(int kind, double DEL, double scale, const DevTree& T, const D
   k.tnrm = tg.nrm.p;
   k.out = out;
   k.entries = L.entries.p;
-  k.blk_start = L.blk_start.p;
   k.counters = nullptr;
   return k;
 }

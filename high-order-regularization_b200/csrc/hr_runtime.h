@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstring>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -39,14 +40,40 @@ struct Error : std::runtime_error {
 void* dev_alloc(size_t bytes);
 void dev_free(void* p) noexcept;
 
+// The workspace of a context's stateless calls (single sums, interpolation,
+// transforms): device memory handed out front to back and page-locked staging
+// that collects a call's small uploads, both kept between calls. A call of such
+// an entry point made ~55 allocations, as many uploads and as many frees, each
+// with a synchronization: most of the 0.7 ms of a small sum. What does not fit
+// comes from dev_alloc as before and grows the workspace, up to its limits, when
+// the call is over. One call at a time (a context belongs to one thread).
+struct Workspace {
+  static constexpr size_t kDevMax = size_t(256) << 20, kPinMax = size_t(32) << 20;
+  static constexpr size_t kSmall = size_t(4) << 20;  // uploads up to this size are collected
+  char* dev = nullptr;
+  char* pin = nullptr;
+  size_t dev_cap = 0, pin_cap = 0;    // capacities
+  size_t low = 0, high = 0;           // uploads from the front, scratch from the back
+  size_t flushed = 0;                 // uploads already copied
+  size_t want_dev = 0, want_pin = 0;  // this call's total needs
+  // `bytes` of device memory, null if they do not fit; up: among the uploads
+  void* take(size_t bytes, bool up);
+  // copies the uploads collected since the last flush
+  void flush(cudaStream_t st);
+  void free_all();
+};
+// The calling thread's active workspace (null outside a WorkspaceScope).
+Workspace*& active_workspace();
+
 template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
+  bool borrowed = false;  // from the active workspace, not freed here
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) {
+  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), borrowed(o.borrowed) {
     o.p = nullptr;
     o.n = 0;
   }
@@ -55,6 +82,7 @@ struct DBuf {
       release();
       p = o.p;
       n = o.n;
+      borrowed = o.borrowed;
       o.p = nullptr;
       o.n = 0;
     }
@@ -62,23 +90,37 @@ struct DBuf {
   }
   ~DBuf() { release(); }
   void release() {
-    if (p) dev_free(p);
+    if (p && !borrowed) dev_free(p);
     p = nullptr;
     n = 0;
   }
-  void alloc(size_t count) {
-    release();
-    if (count == 0) count = 1;
-    p = static_cast<T*>(dev_alloc(count * sizeof(T)));
-    n = count;
-  }
+  void alloc(size_t count) { get(count, false); }
   void upload(const T* h, size_t count, cudaStream_t st) {
-    alloc(count);
-    if (h && count) HR_CHECK_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, st));
+    const size_t bytes = count * sizeof(T);
+    Workspace* w = active_workspace();
+    const bool small = w && h && count && bytes <= Workspace::kSmall;
+    get(count, small);
+    if (!h || !count) return;
+    if (small && borrowed) {  // collected: copied by flush
+      std::memcpy(w->pin + (reinterpret_cast<char*>(p) - w->dev), h, bytes);
+      return;
+    }
+    HR_CHECK_CUDA(cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, st));
   }
   void upload(const std::vector<T>& v, cudaStream_t st) { upload(v.data(), v.size(), st); }
   void zero(cudaStream_t st) {
     if (p) HR_CHECK_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), st));
+  }
+
+ private:
+  void get(size_t count, bool up) {
+    release();
+    if (count == 0) count = 1;
+    Workspace* w = active_workspace();
+    p = w ? static_cast<T*>(w->take(count * sizeof(T), up)) : nullptr;
+    borrowed = p != nullptr;
+    if (!p) p = static_cast<T*>(dev_alloc(count * sizeof(T)));
+    n = count;
   }
 };
 
@@ -101,8 +143,21 @@ struct Ctx {
   // allocated on first use, and the events that mark each one filled
   void* pin = nullptr;
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
+  Workspace ws;
   // throws if a tensor-core kernel of this context reported a timed-out wait
   void check_tc();
+};
+
+// Makes a context's workspace the calling thread's active one for the duration
+// of a synchronous call; on the way out (also by an exception) it waits for the
+// context's streams, so that the memory is idle, and grows the workspace to the
+// call's needs.
+struct WorkspaceScope {
+  Ctx& C;
+  explicit WorkspaceScope(Ctx& c);
+  ~WorkspaceScope();
+  WorkspaceScope(const WorkspaceScope&) = delete;
+  WorkspaceScope& operator=(const WorkspaceScope&) = delete;
 };
 
 // Bytes of one pinned staging buffer of d2h_staged.
@@ -110,9 +165,12 @@ constexpr size_t kPinChunk = size_t(16) << 20;
 
 // Reads `bytes` from device memory into (pageable) host memory through the
 // context's two pinned buffers: the copy of chunk k + 1 runs while host threads
-// move chunk k into place. Returns when all of it has arrived. Reads of up to
-// two chunks go straight to `dst`.
+// move chunk k into place. Returns when all of it has arrived. Small reads go
+// straight to `dst`.
 void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes);
+// The same the other way: returns when `src` has been read; the last chunk may
+// still be on its way on the context's stream.
+void h2d_staged(Ctx& C, void* dst, const void* src, size_t bytes);
 
 // A surface on the device: sources in tree order, its tree, density buffers
 // and the upward-pass work items.
@@ -120,12 +178,11 @@ struct DevTree {
   Tree host;
   int n = 0, nn = 0, P1 = 0, Pf = 0;
   DBuf<double> x, y, z, nx, ny, nz, a;
-  DBuf<int> perm, m0, m1;
+  DBuf<int> perm;
   DBuf<double> tcheb;
   DBuf<double> qx, qy, qz;
   DBuf<double> pk;  // packed records (Pack), up to 12 doubles per source
-  DBuf<float> fx, fy, fz, fnx, fny, fnz, fa, fqx, fqy, fqz;  // FP32 copies, centre-relative
-  double ctr[3] = {0, 0, 0};
+  DBuf<float> fnx, fny, fnz, fa, fqx, fqy, fqz;  // FP32 copies
   DBuf<double> mom;  // nn * Pf * C, proxy-major (C = 10 DL symmetric form, 6 SL)
   DBuf<float> momf;  // nn * Pf * W32 FP32 copy (W32 = 12 DL, 8 SL)
   DBuf<MomItem> items;
@@ -133,7 +190,8 @@ struct DevTree {
   DBuf<double> partial;
   int nitems = 0;
   long long moment_terms = 0;  // sum over non-root nodes of Pf * members
-  void build(const hr_surface& S, int P, int N0, double theta, bool direct, cudaStream_t st);
+  // fp32: with the FP32 copies that the reduced-precision sums read
+  void build(const hr_surface& S, int P, int N0, double theta, bool direct, cudaStream_t st, bool fp32 = true);
   // density (reference order, interleaved, device) -> tree-order SoA (+ moments)
   // and packed records as `pack` (PACK_DL: stresslet moments, otherwise Stokeslet);
   // tc: the upward pass on the tensor cores (reduced-precision operator)
@@ -155,7 +213,7 @@ struct DevTargets {
 
 struct DevLists {
   Lists host;
-  DBuf<int> tord, blk_start;
+  DBuf<int> tord;
   DBuf<Entry> entries;
   void build(const Tree& T, int nt, const double* txyz, const uint8_t* near, cudaStream_t st,
              const std::vector<int>* morton = nullptr);

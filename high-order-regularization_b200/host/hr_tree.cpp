@@ -175,7 +175,7 @@ Tree build_tree(int n, const double* xyz, const double ctr[3], int P, int N0, do
   return T;
 }
 
-std::vector<int> morton_order(int n, const double* xyz) {
+std::vector<int> morton_order(int n, const double* xyz, int bits) {
   std::vector<int> ord(n);
   std::iota(ord.begin(), ord.end(), 0);
   if (n <= 1) return ord;
@@ -196,6 +196,7 @@ std::vector<int> morton_order(int n, const double* xyz) {
     v = (v | v << 2) & 0x1249249249249249ULL;
     return v;
   };
+  const double cells = (double)((1 << bits) - 1);
   std::vector<uint64_t> code(n), code2(n);
 #pragma omp parallel for schedule(static)
   for (int i = 0; i < n; i++) {
@@ -203,13 +204,13 @@ std::vector<int> morton_order(int n, const double* xyz) {
     for (int k = 0; k < 3; k++) {
       double u = (xyz[3 * i + k] - lo[k]) / ext;
       u = std::min(std::max(u, 0.0), 1.0);
-      q[k] = (uint64_t)(u * 2097151.0);
+      q[k] = (uint64_t)(u * cells);
     }
     code[i] = spread(q[0]) | (spread(q[1]) << 1) | (spread(q[2]) << 2);
   }
-  // stable LSD radix sort of the 63-bit codes, 11 bits per pass
+  // stable LSD radix sort of the codes, 11 bits per pass
   std::vector<int> ord2(n);
-  for (int shift = 0; shift < 63; shift += 11) {
+  for (int shift = 0; shift < 3 * bits; shift += 11) {
     int cnt[2049] = {0};
     for (int i = 0; i < n; i++) cnt[((code[i] >> shift) & 2047) + 1]++;
     for (int d = 0; d < 2048; d++) cnt[d + 1] += cnt[d];
@@ -233,6 +234,29 @@ Lists build_lists(const Tree& T, int nt, const double* txyz, const uint8_t* near
   const int nn = T.nnodes();
   const int P1 = T.P + 1;
   const long long Pf = (long long)P1 * P1 * P1;
+  if (nn == 1 && std::isinf(T.mac[0])) {  // direct sums: every block reads the one node
+    L.blk_start.resize(nb + 1);
+    L.entries.resize(nb);
+    L.blk_cost.resize(nb);
+    long long reg = 0;
+    for (int t = 0; t < nt; t++) reg += near ? near[t] != 0 : 1;
+    for (int b = 0; b < nb; b++) {
+      const int cnt = std::min(kTB, nt - b * kTB);
+      Entry& e = L.entries[b];
+      e.node = 0;
+      e.type = 1;
+      for (int w = 0; w < 4; w++) {
+        const int c = std::min(32, std::max(0, cnt - 32 * w));
+        e.mask[w] = c == 32 ? 0xffffffffu : (1u << c) - 1u;
+      }
+      L.blk_start[b] = b;
+      L.blk_cost[b] = (double)((cnt + 31) / 32) * T.n * 90.0;
+    }
+    L.blk_start[nb] = nb;
+    L.near_pairs_reg = reg * T.n;
+    L.near_pairs_plain = (nt - reg) * (long long)T.n;
+    return L;
+  }
   std::vector<std::vector<Entry>> per(nb);
   std::vector<double> cost(nb, 0.0);
   std::vector<long long> reg(nb, 0), plain(nb, 0), prox(nb, 0);
