@@ -9,18 +9,15 @@
 // output is scaled by out_scale.
 //
 // Kernels:
-//   fwd_bwd_kernel   one thread per sample: forward, loss, backward deltas.
-//                    Weights live in shared memory (broadcast reads, 128-bit
-//                    rows); each thread's hidden activations are a column of a
-//                    shared array, so layer loops never index registers
-//                    dynamically. Pre-activations and deltas go to global
-//                    memory feature-major ([feature][batch], coalesced).
-//   grad_kernel      parameter gradients as the batch contraction
-//                    dW = A^T Delta, split over chunks of 32 samples staged in
-//                    shared memory; each thread owns ~37 parameters.
-//   grad_reduce      sums the chunk partials in chunk order (deterministic).
-//   adam_kernel      Adam with bias correction (Kingma & Ba 2015).
-//   infer_kernel     guess = base + out_scale * MLP(x), FP64 out.
+//   train_kernel     forward, loss, backward and the partial parameter gradient
+//                    of a tile of 128 samples per CTA, everything between the
+//                    samples' inputs and the gradient in shared memory and
+//                    registers (below).
+//   grad_adam_kernel sums the tiles' partial gradients in tile order
+//                    (deterministic) and takes the Adam step with bias
+//                    correction (Kingma & Ba 2015).
+//   infer_kernel     guess = base + out_scale * MLP(x), FP64 out; one thread per
+//                    sample, weights in shared memory.
 // The network is FP32 SIMT arithmetic: about 55 kflop per training sample, so
 // a whole training run is a small fraction of the solves that produce its data.
 #include <cuda_runtime.h>
@@ -40,21 +37,11 @@ constexpr int kIn = 12, kH = 64, kOut = 3;
 constexpr int oW1 = 0, ob1 = oW1 + kIn * kH, oW2 = ob1 + kH, ob2 = oW2 + kH * kH, oW3 = ob2 + kH,
               ob3 = oW3 + kH * kH, oW4 = ob3 + kH, ob4 = oW4 + kH * kOut, kNP = ob4 + kOut;
 static_assert(kNP == 9347, "parameter count");
-constexpr int kZ = 3 * kH;            // stored pre-activations per sample: z1, z2, z3
-constexpr int kD = 3 * kH + kOut;     // stored deltas per sample: d1, d2, d3, d4
-constexpr int kA = kIn + 3 * kH + 1;  // activation row in the gradient: x', s(z1), s(z2), s(z3), 1
 constexpr int kThreads = 128;
-constexpr int kGradThreads = 256;
-constexpr int kPerThread = (kNP + kGradThreads - 1) / kGradThreads;  // 37
-constexpr int kChunk = 32;
 constexpr int kPpad = (kNP + 3) & ~3;
 
 __device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = sigm(z);
-  return s * (1.0f + z * (1.0f - s));
-}
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
   // splitmix64 finalizer (Steele, Lea, Flood 2014)
@@ -96,11 +83,9 @@ __device__ __forceinline__ void dense64(const float* __restrict__ P, int oW, int
   }
 }
 
-// Forward of one sample; on return z holds z3 and col holds s(z3).
-// Zs (optional): feature-major store of z1, z2, z3 at column s of a batch of B.
+// Forward of one sample; col: this thread's activation column.
 __device__ __forceinline__ void forward(const float* __restrict__ P, const float* __restrict__ xin,
-                                        const Norm& nm, float* col, float z[kH], float y[kOut],
-                                        float* __restrict__ Zs, long s, long B) {
+                                        const Norm& nm, float* col, float z[kH], float y[kOut]) {
   float x[kIn];
 #pragma unroll
   for (int i = 0; i < kIn; i++) x[i] = (xin[i] - nm.mean[i]) * nm.inv_std[i];
@@ -120,10 +105,7 @@ __device__ __forceinline__ void forward(const float* __restrict__ P, const float
   }
   for (int layer = 0; layer < 3; layer++) {
 #pragma unroll
-    for (int j = 0; j < kH; j++) {
-      if (Zs) Zs[(size_t)(layer * kH + j) * B + s] = z[j];
-      col[j * kThreads] = silu(z[j]);
-    }
+    for (int j = 0; j < kH; j++) col[j * kThreads] = silu(z[j]);
     if (layer < 2) dense64(P, layer == 0 ? oW2 : oW3, layer == 0 ? ob2 : ob3, col, z);
   }
 #pragma unroll
@@ -136,162 +118,327 @@ __device__ __forceinline__ void forward(const float* __restrict__ P, const float
   }
 }
 
+// All loads of a thread in flight at once (one memory latency, not 37).
+template <int kThr>
 __device__ __forceinline__ void load_params(float* P, const float* __restrict__ params) {
-  for (int i = threadIdx.x; i < kNP; i += blockDim.x) P[i] = params[i];
+  constexpr int kV = kNP / 4, kN = (kV + kThr - 1) / kThr;
+  const float4* src = reinterpret_cast<const float4*>(params);
+  float4 v[kN];
+#pragma unroll
+  for (int i = 0; i < kN; i++) {
+    const int e = threadIdx.x + i * kThr;
+    if (e < kV) v[i] = src[e];
+  }
+#pragma unroll
+  for (int i = 0; i < kN; i++) {
+    const int e = threadIdx.x + i * kThr;
+    if (e < kV) reinterpret_cast<float4*>(P)[e] = v[i];
+  }
+  if (threadIdx.x < kNP - 4 * kV) P[4 * kV + threadIdx.x] = params[4 * kV + threadIdx.x];
 }
 
-// Training pass over a batch: forward, squared-error loss (mean over batch and
-// components of (y - t / out_scale)^2), backward deltas.
-__global__ void __launch_bounds__(kThreads) fwd_bwd_kernel(
-    const float* __restrict__ params, Norm nm, const float* __restrict__ X, const float* __restrict__ T,
-    long n, int batch, unsigned long long seed, long step, int random, long* __restrict__ idx_out,
-    float* __restrict__ Zs, float* __restrict__ Ds, double* __restrict__ loss_part) {
-  extern __shared__ __align__(16) float sm[];
-  float* P = sm;              // kNP weights (padded)
-  float* cols = sm + kPpad;   // kH x kThreads activation / delta columns
-  __shared__ double red[kThreads / 32];
-  load_params(P, params);
+// Training pass over a tile of kS samples: forward, squared-error loss (mean
+// over batch and components of (y - t / out_scale)^2), backward deltas, and the
+// tile's partial gradient dW = A^T Delta.
+//
+// FP32 multiply-adds on the SIMT cores: 27 k per sample, 12 us for 16384
+// samples at their peak rate. One thread per sample with its activations in
+// shared-memory columns, pre-activations and deltas through global memory and a
+// gradient kernel with two shared reads per multiply-add took 150 us. Here
+// every layer is a small matrix product with register tiles, 8 features x 4
+// samples per thread (3 shared reads of 16 bytes per 32 multiply-adds: the
+// shared-memory pipe and the multiply-adds take about equally long), with the
+// activations a_l and the derivatives s'(z_l) in shared memory; the deltas
+// overwrite the derivatives, so a tile's state fits one CTA (213 KB). Lanes run
+// along the samples, so that stores and gathers meet different banks and the
+// weights are broadcast. A batch of 16384 is 128 tiles: one CTA on each of 128
+// SMs. Measured: a step of that batch 148 -> 47 us (batch 300: 111 -> 44, 60000:
+// 474 -> 166); issue slots 52 % busy, shared-memory pipe 52 %, the rest the
+// latencies between barriers with two warps per SM quarter. Four warps with 8 x 8
+// tiles and every layer's code unrolled took 64 us: the code is fetched once
+// per CTA, so the layers loop over one copy of it.
+constexpr int kS = 128, kSP = kS + 4;  // samples per tile; row stride (rows 4 banks apart)
+constexpr int kTrainThreads = 256;
+constexpr int kActR = kH * kSP;        // floats of one [feature][sample] array
+
+// acc[f][q] += sum_k w(k, f) a[k][sample q]: features 8 tx + f, samples 4 ty + q.
+// a: K rows of kSP; w: row k, 64 columns.
+__device__ __forceinline__ void tile_mul(const float* a, const float* w, int K, int tx, int ty, float (&acc)[8][4]) {
+#pragma unroll 4
+  for (int k = 0; k < K; k++) {
+    const float4 av4 = *reinterpret_cast<const float4*>(a + k * kSP + 4 * ty);
+    const float4 w0 = *reinterpret_cast<const float4*>(w + k * kH + 8 * tx);
+    const float4 w1 = *reinterpret_cast<const float4*>(w + k * kH + 8 * tx + 4);
+    const float av[4] = {av4.x, av4.y, av4.z, av4.w};
+    const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (int f = 0; f < 8; f++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[f][q] += av[q] * wv[f];
+  }
+}
+
+// The same with the weights' transpose: acc[f][q] += sum_j W[8 tx + f][j] d[j][sample q].
+__device__ __forceinline__ void tile_mul_t(const float* d, const float* w, int tx, int ty, float (&acc)[8][4]) {
+#pragma unroll 1
+  for (int j = 0; j < kH; j += 4) {
+    float4 wr[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++) wr[f] = *reinterpret_cast<const float4*>(w + (8 * tx + f) * kH + j);
+#pragma unroll
+    for (int jj = 0; jj < 4; jj++) {
+      const float4 dv4 = *reinterpret_cast<const float4*>(d + (j + jj) * kSP + 4 * ty);
+      const float dv[4] = {dv4.x, dv4.y, dv4.z, dv4.w};
+#pragma unroll
+      for (int f = 0; f < 8; f++) {
+        const float wv = jj == 0 ? wr[f].x : (jj == 1 ? wr[f].y : (jj == 2 ? wr[f].z : wr[f].w));
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[f][q] += wv * dv[q];
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void store_row(float* row, int ty, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(row + 4 * ty) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// Partial gradient of one layer over the tile: dW[i][j] = sum_s a[i][s] d[j][s]
+// for kI rows i and the 64 columns j, and db[j] = sum_s d[j][s]. Each half of
+// the CTA sums half of the samples (a thread: rows gx + 8 r, columns gy + 16 c);
+// the second half's sums go to the first through `a`, which nothing reads again.
+template <int kI>
+__device__ __forceinline__ void tile_grad(float* a, const float* d, float* __restrict__ dw, float* __restrict__ db) {
+  constexpr int kR = (kI + 7) / 8;
+  const int half = threadIdx.x >> 7, t = threadIdx.x & 127, lane = t & 31, warp = t >> 5;
+  const int gy = (lane & 7) + 8 * (warp & 1), gx = (lane >> 3) + 4 * (warp >> 1);
+  float acc[kR][4], accb[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    accb[c] = 0.f;
+#pragma unroll
+    for (int r = 0; r < kR; r++) acc[r][c] = 0.f;
+  }
+#pragma unroll 1
+  for (int s = half * (kS / 2); s < (half + 1) * (kS / 2); s += 4) {
+    float4 av[kR], dv[4];
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+      const int i = gx + 8 * r;
+      av[r] = *reinterpret_cast<const float4*>(a + (i < kI ? i : 0) * kSP + s);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++) dv[c] = *reinterpret_cast<const float4*>(d + (gy + 16 * c) * kSP + s);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+#pragma unroll
+      for (int r = 0; r < kR; r++) {
+        acc[r][c] += av[r].x * dv[c].x;
+        acc[r][c] += av[r].y * dv[c].y;
+        acc[r][c] += av[r].z * dv[c].z;
+        acc[r][c] += av[r].w * dv[c].w;
+      }
+      accb[c] += (dv[c].x + dv[c].y) + (dv[c].z + dv[c].w);
+    }
+  }
+  __syncthreads();  // everyone has read a
+  if (half == 1) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+#pragma unroll
+      for (int r = 0; r < kR; r++) a[(c * kR + r) * 128 + t] = acc[r][c];
+      if (gx == 0) a[(4 * kR + c) * 128 + gy] = accb[c];
+    }
+  }
   __syncthreads();
-  float* col = cols + threadIdx.x;
-  const int s = blockIdx.x * kThreads + threadIdx.x;
+  if (half == 0) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+#pragma unroll
+      for (int r = 0; r < kR; r++) {
+        const int i = gx + 8 * r;
+        if (i < kI) dw[i * kH + gy + 16 * c] = acc[r][c] + a[(c * kR + r) * 128 + t];
+      }
+      if (gx == 0) db[gy + 16 * c] = accb[c] + a[(4 * kR + c) * 128 + gy];
+    }
+  }
+}
+static_assert((4 * 8 + 4) * 128 <= kActR && (4 * 2 + 4) * 128 <= kIn * kSP, "a half's sums fit in place of the inputs");
+
+__global__ void __launch_bounds__(kTrainThreads) train_kernel(
+    const float* __restrict__ params, Norm nm, const float* __restrict__ X, const float* __restrict__ T, long n,
+    int batch, unsigned long long seed, long step, int random, float* partial, double* __restrict__ loss_part) {
+  extern __shared__ __align__(16) float sm[];
+  float* P = sm;                    // weights (padded)
+  float* x = P + kPpad;             // normalized inputs, kIn rows
+  float* act = x + kIn * kSP;       // activations a1, a2, a3 (later d3)
+  float* der = act + 3 * kActR;     // derivatives s'(z1), s'(z2), later the deltas d1, d2
+  float* d4 = der + 2 * kActR;      // output deltas, kOut rows
+  __shared__ double red[kTrainThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = (lane & 7) + 8 * (warp & 3), tx = (lane >> 3) + 4 * (warp >> 2);
+  const int s = blockIdx.x * kS + tid;  // this thread's sample in the per-sample parts (tid < kS)
+  const bool valid = tid < kS && s < batch;
+  const long g = valid ? sample_index(s, n, seed, step, random) : 0;
+  load_params<kTrainThreads>(P, params);
+  if (tid < kS) {
+#pragma unroll
+    for (int i = 0; i < kIn; i++) x[i * kSP + tid] = valid ? (X[g * kIn + i] - nm.mean[i]) * nm.inv_std[i] : 0.f;
+  }
+  __syncthreads();
+  float z[8][4];
+  // one copy of the layers' code: it is fetched once per CTA, by one CTA per SM
+#pragma unroll 1
+  for (int l = 0; l < 3; l++) {
+    const int ob = l == 0 ? ob1 : (l == 1 ? ob2 : ob3), oW = l == 0 ? oW1 : (l == 1 ? oW2 : oW3);
+#pragma unroll
+    for (int f = 0; f < 8; f++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) z[f][q] = P[ob + 8 * tx + f];
+    tile_mul(l == 0 ? x : act + (l - 1) * kActR, P + oW, l == 0 ? kIn : kH, tx, ty, z);
+    // a = silu(z), z <- silu'(z), one sigmoid each; the last layer's derivatives
+    // stay in registers
+#pragma unroll
+    for (int f = 0; f < 8; f++) {
+      float av[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float sg = sigm(z[f][q]);
+        av[q] = z[f][q] * sg;
+        z[f][q] = sg * (1.0f + z[f][q] * (1.0f - sg));
+      }
+      store_row(act + l * kActR + (8 * tx + f) * kSP, ty, av);
+      if (l < 2) store_row(der + l * kActR + (8 * tx + f) * kSP, ty, z[f]);
+    }
+    __syncthreads();
+  }
+  float* a3 = act + 2 * kActR;
+  // output, loss and its delta: one sample per thread
   double l2 = 0.0;
-  if (s < batch) {
-    const long g = sample_index(s, n, seed, step, random);
-    idx_out[s] = g;
-    const long B = batch;
-    float z[kH], y[kOut];
-    forward(P, X + g * kIn, nm, col, z, y, Zs, s, B);
-    float d4[kOut];
+  if (tid < kS) {
+    float y[kOut];
+#pragma unroll
+    for (int j = 0; j < kOut; j++) y[j] = P[ob4 + j];
+#pragma unroll 8
+    for (int i = 0; i < kH; i++) {
+      const float ai = a3[i * kSP + tid];
+#pragma unroll
+      for (int j = 0; j < kOut; j++) y[j] += ai * P[oW4 + i * kOut + j];
+    }
     const float inv = 2.0f / (float)((long)batch * kOut);
 #pragma unroll
     for (int j = 0; j < kOut; j++) {
-      const float e = y[j] - T[g * kOut + j] / nm.out_scale;
+      const float e = valid ? y[j] - T[g * kOut + j] / nm.out_scale : 0.f;
       l2 += (double)e * (double)e;
-      d4[j] = e * inv;
-      Ds[(size_t)(3 * kH + j) * B + s] = d4[j];
-    }
-    // d3 = (W4 d4) * s'(z3), z3 still in registers
-    float d[kH];
-#pragma unroll
-    for (int i = 0; i < kH; i++) {
-      float t = 0.f;
-#pragma unroll
-      for (int j = 0; j < kOut; j++) t += P[oW4 + i * kOut + j] * d4[j];
-      d[i] = t * dsilu(z[i]);
-      Ds[(size_t)(2 * kH + i) * B + s] = d[i];
-    }
-    // d2 = (W3 d3) * s'(z2), then d1 = (W2 d2) * s'(z1)
-    for (int layer = 1; layer >= 0; layer--) {
-      const int oW = layer == 1 ? oW3 : oW2;
-#pragma unroll 2
-      for (int i = 0; i < kH; i++) {
-        const float4* w = reinterpret_cast<const float4*>(P + oW + i * kH);
-        float t = 0.f;
-#pragma unroll
-        for (int j4 = 0; j4 < kH / 4; j4++) {
-          const float4 v = w[j4];
-          t += v.x * d[4 * j4] + v.y * d[4 * j4 + 1] + v.z * d[4 * j4 + 2] + v.w * d[4 * j4 + 3];
-        }
-        const float di = t * dsilu(Zs[(size_t)(layer * kH + i) * B + s]);
-        col[i * kThreads] = di;
-        Ds[(size_t)(layer * kH + i) * B + s] = di;
-      }
-#pragma unroll
-      for (int i = 0; i < kH; i++) d[i] = col[i * kThreads];
+      d4[j * kSP + tid] = e * inv;
     }
   }
-  for (int off = 16; off > 0; off >>= 1) l2 += __shfl_down_sync(0xffffffffu, l2, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l2;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  float* out = partial + (size_t)blockIdx.x * kNP;
+  // output layer's gradient: thread i < 64 row i of dW4, threads 64..66 the biases
+  if (tid < kH + kOut) {
+    float acc[kOut] = {0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int q = 0; q < kS; q += 4) {
+      const float4 av = tid < kH ? *reinterpret_cast<const float4*>(a3 + tid * kSP + q) : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+      for (int j = 0; j < kOut; j++) {
+        const float4 dv = *reinterpret_cast<const float4*>(d4 + j * kSP + q);
+        acc[j] += av.x * dv.x;
+        acc[j] += av.y * dv.y;
+        acc[j] += av.z * dv.z;
+        acc[j] += av.w * dv.w;
+      }
+    }
+    if (tid < kH) {
+#pragma unroll
+      for (int j = 0; j < kOut; j++) out[oW4 + tid * kOut + j] = acc[j];
+    } else {
+      const int j = tid - kH;
+      out[ob4 + j] = j == 0 ? acc[0] : (j == 1 ? acc[1] : acc[2]);
+    }
+  }
+  __syncthreads();
+  // d3 = (W4 d4) s'(z3), in place of a3
+#pragma unroll
+  for (int f = 0; f < 8; f++) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < kOut; j++) {
+      const float w = P[oW4 + (8 * tx + f) * kOut + j];
+      const float4 e = *reinterpret_cast<const float4*>(d4 + j * kSP + 4 * ty);
+      v[0] += w * e.x;
+      v[1] += w * e.y;
+      v[2] += w * e.z;
+      v[3] += w * e.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] *= z[f][q];
+    store_row(a3 + (8 * tx + f) * kSP, ty, v);
+  }
+  __syncthreads();
+  // layers 3 and 2: the gradient from a_{l-1} and d_l, then d_{l-1} = (W d_l)
+  // s'(z_{l-1}) in place of the derivatives
+#pragma unroll 1
+  for (int l = 2; l > 0; l--) {
+    const float* d = l == 2 ? a3 : der + kActR;
+    const int oW = l == 2 ? oW3 : oW2, ob = l == 2 ? ob3 : ob2;
+    tile_grad<kH>(act + (l - 1) * kActR, d, out + oW, out + ob);
+#pragma unroll
+    for (int f = 0; f < 8; f++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) z[f][q] = 0.f;
+    tile_mul_t(d, P + oW, tx, ty, z);
+#pragma unroll
+    for (int f = 0; f < 8; f++) {
+      float* row = der + (l - 1) * kActR + (8 * tx + f) * kSP;
+      const float4 sg = *reinterpret_cast<const float4*>(row + 4 * ty);
+      const float v[4] = {z[f][0] * sg.x, z[f][1] * sg.y, z[f][2] * sg.z, z[f][3] * sg.w};
+      store_row(row, ty, v);
+    }
+    __syncthreads();
+  }
+  tile_grad<kIn>(x, der, out + oW1, out + ob1);
+  for (int off = 16; off > 0; off >>= 1) l2 += __shfl_down_sync(0xffffffffu, l2, off);
+  if (lane == 0) red[warp] = l2;
+  __syncthreads();
+  if (tid == 0) {
     double t = 0;
-    for (int w = 0; w < kThreads / 32; w++) t += red[w];
+    for (int w = 0; w < kTrainThreads / 32; w++) t += red[w];
     loss_part[blockIdx.x] = t;
   }
 }
 
-// Activation-row and delta-row index of parameter p, packed (a | d << 16).
-__device__ __forceinline__ int param_rows(int p) {
-  int a, d;
-  if (p < ob1) { a = (p - oW1) / kH; d = (p - oW1) % kH; }
-  else if (p < oW2) { a = kA - 1; d = p - ob1; }
-  else if (p < ob2) { a = kIn + (p - oW2) / kH; d = kH + (p - oW2) % kH; }
-  else if (p < oW3) { a = kA - 1; d = kH + (p - ob2); }
-  else if (p < ob3) { a = kIn + kH + (p - oW3) / kH; d = 2 * kH + (p - oW3) % kH; }
-  else if (p < oW4) { a = kA - 1; d = 2 * kH + (p - ob3); }
-  else if (p < ob4) { a = kIn + 2 * kH + (p - oW4) / kOut; d = 3 * kH + (p - oW4) % kOut; }
-  else { a = kA - 1; d = 3 * kH + (p - ob4); }
-  return a | (d << 16);
-}
+struct Adam {
+  float lr, b1, b2, eps, c1, c2;
+};
 
-// Partial gradient of every parameter over one chunk of samples.
-__global__ void __launch_bounds__(kGradThreads) grad_kernel(Norm nm, const float* __restrict__ X, int batch,
-                                                            const long* __restrict__ idx,
-                                                            const float* __restrict__ Zs,
-                                                            const float* __restrict__ Ds,
-                                                            float* __restrict__ partial) {
-  extern __shared__ __align__(16) float gsm[];
-  float* sAct = gsm;                 // kChunk x kA
-  float* sDel = gsm + kChunk * kA;   // kChunk x kD
-  const int s0 = blockIdx.x * kChunk;
-  const int cs = min(kChunk, batch - s0);
-  for (int e = threadIdx.x; e < kChunk * kA; e += kGradThreads) {
-    const int s = e % kChunk, a = e / kChunk;
-    float v = 0.f;
-    if (s < cs) {
-      const long g = s0 + s;
-      if (a < kIn) v = (X[idx[g] * kIn + a] - nm.mean[a]) * nm.inv_std[a];
-      else if (a < kA - 1) v = silu(Zs[(size_t)(a - kIn) * batch + g]);
-      else v = 1.0f;
-    }
-    sAct[s * kA + a] = v;
+// The gradient, summed over the tiles, and (lr > 0) the Adam step. A CTA of four
+// warps takes 32 parameters; each warp sums a quarter of the tiles in order,
+// then the quarters are added in order (deterministic).
+__global__ void __launch_bounds__(128) grad_adam_kernel(const float* __restrict__ partial, int ntiles,
+                                                        float* __restrict__ grad, float* __restrict__ params,
+                                                        float* __restrict__ m, float* __restrict__ v, Adam o) {
+  __shared__ float part[4][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
+  const int per = (ntiles + 3) / 4, c0 = warp * per, c1 = min(ntiles, c0 + per);
+  float g = 0.f;
+  if (p < kNP) {
+#pragma unroll 16
+    for (int c = c0; c < c1; c++) g += partial[(size_t)c * kNP + p];
   }
-  for (int e = threadIdx.x; e < kChunk * kD; e += kGradThreads) {
-    const int s = e % kChunk, d = e / kChunk;
-    sDel[s * kD + d] = s < cs ? Ds[(size_t)d * batch + s0 + s] : 0.f;
-  }
+  part[warp][lane] = g;
   __syncthreads();
-  int rows[kPerThread];
-  float acc[kPerThread];
-#pragma unroll
-  for (int k = 0; k < kPerThread; k++) {
-    const int p = threadIdx.x + k * kGradThreads;
-    rows[k] = p < kNP ? param_rows(p) : (kA - 1);
-    acc[k] = 0.f;
-  }
-  for (int s = 0; s < cs; s++) {
-    const float* a = sAct + s * kA;
-    const float* dd = sDel + s * kD;
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) acc[k] += a[rows[k] & 0xffff] * dd[rows[k] >> 16];
-  }
-  float* out = partial + (size_t)blockIdx.x * kNP;
-#pragma unroll
-  for (int k = 0; k < kPerThread; k++) {
-    const int p = threadIdx.x + k * kGradThreads;
-    if (p < kNP) out[p] = acc[k];
-  }
-}
-
-__global__ void grad_reduce_kernel(const float* __restrict__ partial, int nchunks, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNP) return;
-  float s = 0.f;
-  for (int c = 0; c < nchunks; c++) s += partial[(size_t)c * kNP + p];
-  grad[p] = s;
-}
-
-__global__ void adam_kernel(float* __restrict__ params, const float* __restrict__ grad, float* __restrict__ m,
-                            float* __restrict__ v, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNP) return;
-  const float g = grad[p];
-  const float mm = b1 * m[p] + (1.0f - b1) * g;
-  const float vv = b2 * v[p] + (1.0f - b2) * g * g;
+  if (warp != 0 || p >= kNP) return;
+  g = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
+  grad[p] = g;
+  if (!(o.lr > 0.f)) return;
+  const float mm = o.b1 * m[p] + (1.0f - o.b1) * g;
+  const float vv = o.b2 * v[p] + (1.0f - o.b2) * g * g;
   m[p] = mm;
   v[p] = vv;
-  params[p] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+  params[p] -= o.lr * (mm / o.c1) / (sqrtf(vv / o.c2) + o.eps);
 }
 
 // Output frames of inference: samples start[f] .. start[f+1]-1 are rotated
@@ -311,12 +458,12 @@ __global__ void __launch_bounds__(kThreads) infer_kernel(const float* __restrict
   extern __shared__ __align__(16) float sm[];
   float* P = sm;
   float* cols = sm + kPpad;
-  load_params(P, params);
+  load_params<kThreads>(P, params);
   __syncthreads();
   const long s = (long)blockIdx.x * kThreads + threadIdx.x;
   if (s >= n) return;
   float z[kH], y[kOut];
-  forward(P, X + s * kIn, nm, cols + threadIdx.x, z, y, nullptr, 0, 0);
+  forward(P, X + s * kIn, nm, cols + threadIdx.x, z, y);
   double v[kOut] = {y[0], y[1], y[2]};
   for (int f = 0; f < fr.n; f++) {
     if (s >= fr.start[f] && s < fr.start[f + 1]) {
@@ -340,7 +487,8 @@ __global__ void sum_kernel(const double* __restrict__ part, int n, double* out) 
 }
 
 constexpr size_t kFwdSmem = sizeof(float) * ((size_t)kPpad + (size_t)kH * kThreads);
-constexpr size_t kGradSmem = sizeof(float) * (size_t)kChunk * (kA + kD);
+constexpr size_t kTrainSmem = sizeof(float) * ((size_t)kPpad + (kIn + kOut) * kSP + 5 * (size_t)kActR);
+static_assert(kTrainSmem + 64 <= 227 * 1024, "a tile's state fits one CTA");
 
 }  // namespace
 
@@ -348,18 +496,14 @@ struct hr_mlp {
   hr_ctx* owner = nullptr;
   Norm nm;
   hr::DBuf<float> params, grad, m, v, partial;
-  hr::DBuf<float> Zs, Ds;
-  hr::DBuf<long> idx;
   hr::DBuf<double> loss_part, loss;
   int cap = 0;
   long step = 0;
   void ensure(int batch) {
     if (batch <= cap) return;
-    Zs.alloc((size_t)batch * kZ);
-    Ds.alloc((size_t)batch * kD);
-    idx.alloc(batch);
-    loss_part.alloc((batch + kThreads - 1) / kThreads);
-    partial.alloc((size_t)((batch + kChunk - 1) / kChunk) * kNP);
+    const size_t tiles = (batch + kS - 1) / kS;
+    loss_part.alloc(tiles);
+    partial.alloc(tiles * kNP);
     cap = batch;
   }
 };
@@ -383,9 +527,8 @@ int mlp_guard(hr_mlp* M, F&& f) {
 void set_smem_attrs() {
   static bool done = false;
   if (done) return;
-  HR_CHECK_CUDA(cudaFuncSetAttribute(fwd_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem));
+  HR_CHECK_CUDA(cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
   HR_CHECK_CUDA(cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem));
-  HR_CHECK_CUDA(cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem));
   done = true;
 }
 
@@ -492,22 +635,15 @@ extern "C" int hr_mlp_train_step(hr_mlp* M, const float* X_dev, const float* T_d
     cudaStream_t st = C.stream;
     set_smem_attrs();
     M->ensure(batch);
-    const int nb = (batch + kThreads - 1) / kThreads;
-    const int nchunks = (batch + kChunk - 1) / kChunk;
+    const int nb = (batch + kS - 1) / kS;
     const long step = M->step + 1;
-    fwd_bwd_kernel<<<nb, kThreads, kFwdSmem, st>>>(M->params.p, M->nm, X_dev, T_dev, n, batch, seed, step, random,
-                                                    M->idx.p, M->Zs.p, M->Ds.p, M->loss_part.p);
-    grad_kernel<<<nchunks, kGradThreads, kGradSmem, st>>>(M->nm, X_dev, batch, M->idx.p, M->Zs.p, M->Ds.p, M->partial.p);
-    grad_reduce_kernel<<<(kNP + 255) / 256, 256, 0, st>>>(M->partial.p, nchunks, M->grad.p);
-    C.launches += 3;
-    if (lr > 0) {
-      M->step = step;
-      const float b1 = 0.9f, b2 = 0.999f;
-      const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-      adam_kernel<<<(kNP + 255) / 256, 256, 0, st>>>(M->params.p, M->grad.p, M->m.p, M->v.p, lr, b1, b2, 1e-8f, c1,
-                                                      c2);
-      C.launches++;
-    }
+    train_kernel<<<nb, kTrainThreads, kTrainSmem, st>>>(M->params.p, M->nm, X_dev, T_dev, n, batch, seed, step, random,
+                                                   M->partial.p, M->loss_part.p);
+    const float b1 = 0.9f, b2 = 0.999f;
+    const Adam o = {lr, b1, b2, 1e-8f, 1.0f - powf(b1, (float)step), 1.0f - powf(b2, (float)step)};
+    grad_adam_kernel<<<(kNP + 31) / 32, 128, 0, st>>>(M->partial.p, nb, M->grad.p, M->params.p, M->m.p, M->v.p, o);
+    C.launches += 2;
+    if (lr > 0) M->step = step;
     HR_CHECK_CUDA(cudaGetLastError());
     if (loss) {
       sum_kernel<<<1, 1, 0, st>>>(M->loss_part.p, nb, M->loss.p);
