@@ -257,47 +257,42 @@ __global__ void moments_reduce_kernel(int C, int Pf, MomTree t0, MomTree t1) {
   }
 }
 
-__global__ void permute_kernel(int n, const int* __restrict__ perm, const double* __restrict__ q3,
-                               double* __restrict__ qx, double* __restrict__ qy,
-                               double* __restrict__ qz, float* __restrict__ fqx,
-                               float* __restrict__ fqy, float* __restrict__ fqz, PackSrc ps) {
+__global__ void permute_kernel(PermTree t0, PermTree t1, int pack) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  int o = perm[p];
-  const double a = q3[3 * o], b = q3[3 * o + 1], c = q3[3 * o + 2];
-  qx[p] = a;
-  qy[p] = b;
-  qz[p] = c;
-  if (fqx) {
-    fqx[p] = (float)a;
-    fqy[p] = (float)b;
-    fqz[p] = (float)c;
+  const bool first = p < t0.n;
+  const PermTree& t = first ? t0 : t1;
+  if (!first) p -= t0.n;
+  if (p >= t.n) return;
+  const int o = t.perm[p];
+  const double a = t.q3[3 * o], b = t.q3[3 * o + 1], c = t.q3[3 * o + 2];
+  t.qx[p] = a;
+  t.qy[p] = b;
+  t.qz[p] = c;
+  if (t.fqx) {
+    t.fqx[p] = (float)a;
+    t.fqy[p] = (float)b;
+    t.fqz[p] = (float)c;
   }
-  const double w = ps.a[p], wq = ps.pack == PACK_SL ? w : 1.0;
-  if (ps.pack == PACK_E2G) {
-    double2* r = reinterpret_cast<double2*>(ps.pk) + 6 * (size_t)p;
-    const double u = ps.nx[p], v = ps.ny[p], z = ps.nz[p];
-    r[0] = make_double2(ps.x[p], ps.y[p]);
-    r[1] = make_double2(ps.z[p], w);
+  if (!t.pk) return;
+  const double w = t.a[p], u = t.nx[p], v = t.ny[p], z = t.nz[p];
+  double2* r = reinterpret_cast<double2*>(t.pk);
+  if (pack == PACK_E2G) {
+    r += 6 * (size_t)p;
+    r[0] = make_double2(t.x[p], t.y[p]);
+    r[1] = make_double2(t.z[p], w);
     r[2] = make_double2(a, b);
     r[3] = make_double2(c, u * u + v * v + z * z);
     r[4] = make_double2(u, v);
     r[5] = make_double2(z, 0.0);
-    return;
+  } else {
+    const double wq = pack == PACK_SL ? w : 1.0;
+    r += 5 * (size_t)p;
+    r[0] = make_double2(t.x[p], t.y[p]);
+    r[1] = make_double2(t.z[p], w);
+    r[2] = make_double2(w * u, w * v);
+    r[3] = make_double2(w * z, wq * a);
+    r[4] = make_double2(wq * b, wq * c);
   }
-  double2* r = reinterpret_cast<double2*>(ps.pk) + 5 * (size_t)p;
-  r[0] = make_double2(ps.x[p], ps.y[p]);
-  r[1] = make_double2(ps.z[p], w);
-  r[2] = make_double2(w * ps.nx[p], w * ps.ny[p]);
-  r[3] = make_double2(w * ps.nz[p], wq * a);
-  r[4] = make_double2(wq * b, wq * c);
-}
-
-__global__ void permute_soa_kernel(int n, const int* __restrict__ perm,
-                                   const double* __restrict__ src, double* __restrict__ dst) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  dst[p] = src[perm[p]];
 }
 
 // sixPoint_coeff (2S/main.cpp:750-757)
@@ -310,61 +305,85 @@ __device__ __forceinline__ void six_coeff(double p, double c[6]) {
   c[5] = p * (p * p - 1.0) * (p * p - 4.0) / 120.0;
 }
 
-// sixPointInterpolate over the precomputed stencil (2S/main.cpp:759-778, 1019-1039)
-__global__ void interp_kernel(int ne, const int* __restrict__ tgt, const int* __restrict__ idx,
-                              const double* __restrict__ pq, const double* __restrict__ g,
-                              double* __restrict__ g0) {
+// sixPointInterpolate over the precomputed stencil (2S/main.cpp:759-778,
+// 1019-1039), one thread per entry and component.
+__global__ void interp_kernel(InterpSet s0, InterpSet s1) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
+  const bool first = e < 3 * s0.ne;
+  const InterpSet& S = first ? s0 : s1;
+  if (!first) e -= 3 * s0.ne;
+  if (e >= 3 * S.ne) return;
+  const int comp = e % 3;
+  e /= 3;
   double a[6], b[6];
-  six_coeff(pq[2 * e], a);
-  six_coeff(pq[2 * e + 1], b);
-  const int* st = idx + 36 * (size_t)e;
-  const int t = tgt[e];
-  for (int comp = 0; comp < 3; comp++) {
-    double ft[6];
-    for (int jj = 0; jj < 6; jj++) {
-      double s = 0.0;
-      for (int ii = 0; ii < 6; ii++) s += a[ii] * g[3 * st[6 * ii + jj] + comp];
-      ft[jj] = s;
-    }
-    double v = 0.0;
-    for (int jj = 0; jj < 6; jj++) v += b[jj] * ft[jj];
-    g0[3 * t + comp] = v;
+  six_coeff(S.pq[2 * e], a);
+  six_coeff(S.pq[2 * e + 1], b);
+  const int* st = S.idx + 36 * (size_t)e;
+  double ft[6];
+#pragma unroll
+  for (int jj = 0; jj < 6; jj++) {
+    double s = 0.0;
+#pragma unroll
+    for (int ii = 0; ii < 6; ii++) s += a[ii] * S.g[3 * st[6 * ii + jj] + comp];
+    ft[jj] = s;
   }
+  double v = 0.0;
+#pragma unroll
+  for (int jj = 0; jj < 6; jj++) v += b[jj] * ft[jj];
+  S.g0[3 * S.tgt[e] + comp] = v;
 }
 
-// u_out = u_in - on*factor; u_out -= comp*factor   (2S/main.cpp:612-676)
-__global__ void matvec_combine_kernel(int n, double factor, const double* __restrict__ x,
-                                      const double* __restrict__ on,
-                                      const double* __restrict__ comp, double* __restrict__ y) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = x[i] - on[i] * factor;
-  v -= comp[i] * factor;
+// u_out = u_in - on*factor; u_out -= comp*factor   (2S/main.cpp:612-676), both
+// target sets (set 1 subtracts comp first: its a is comp, its b is on)
+__global__ void matvec_combine_kernel(CombineSet s0, CombineSet s1, double factor, const double* __restrict__ x,
+                                      double* __restrict__ y) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s0.n + s1.n) return;
+  const CombineSet& S = i < s0.n ? s0 : s1;
+  const int k = i < s0.n ? i : i - s0.n;
+  double v = x[i] - S.a[k] * factor;
+  v -= S.b[k] * factor;
   y[i] = v;
 }
 
-// SL = on; SL += comp; b = -SL * factor   (2S/main.cpp:202-207, 478-536)
-__global__ void rhs_combine_kernel(int n, double factor, const double* __restrict__ on,
-                                   const double* __restrict__ comp, double* __restrict__ b) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = on[i];
-  s += comp[i];
+// SL = a; SL += b; rhs = -SL * factor   (2S/main.cpp:202-207, 478-536)
+__global__ void rhs_combine_kernel(CombineSet s0, CombineSet s1, double factor, double* __restrict__ b) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s0.n + s1.n) return;
+  const CombineSet& S = i < s0.n ? s0 : s1;
+  const int k = i < s0.n ? i : i - s0.n;
+  double s = S.a[k];
+  s += S.b[k];
   b[i] = -s * factor;
 }
 
 constexpr int kDotThreads = 256;
 constexpr int kMaxCols = 64;
 
-// partial[blk][c] = sum over this block's strided range of V[c][i] * w[i]
-__global__ void __launch_bounds__(kDotThreads) dots_kernel(int n, int ncols,
-                                                           const double* __restrict__ V, long ldv,
-                                                           const double* __restrict__ w,
-                                                           double* __restrict__ partial) {
+// One Gram-Schmidt pass: (kSub) w -= sum_c coef[c] V[c] first, then out[c] = U[c] .
+// w for ncols columns (U = V, or the norm's U = w). A thread updates and reads
+// the same elements of w. The blocks' partial sums are added by the last block
+// to finish: one warp per column, lane l the blocks l, l + 32, ... in order,
+// then a fixed shuffle tree (deterministic). One launch instead of three of
+// ~3 us each around microseconds of work.
+template <bool kSub>
+__global__ void __launch_bounds__(kDotThreads) dots_kernel(int n, int nsub, const double* V, long ldv,
+                                                           const double* __restrict__ coef, double* w, int ncols,
+                                                           const double* U, double* __restrict__ partial,
+                                                           unsigned* __restrict__ done, double* __restrict__ out) {
   __shared__ double red[kDotThreads / 32][kMaxCols];
+  __shared__ double sc[kMaxCols];
+  __shared__ bool last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if constexpr (kSub) {
+    if (tid < nsub) sc[tid] = coef[tid];
+    __syncthreads();
+    for (int i = blockIdx.x * kDotThreads + tid; i < n; i += gridDim.x * kDotThreads) {
+      double v = w[i];
+      for (int c = 0; c < nsub; c++) v += -1.0 * sc[c] * V[(size_t)c * ldv + i];
+      w[i] = v;
+    }
+  }
   for (int c0 = 0; c0 < ncols; c0 += 8) {
     double acc[8];
 #pragma unroll
@@ -373,7 +392,7 @@ __global__ void __launch_bounds__(kDotThreads) dots_kernel(int n, int ncols,
       const double wi = w[i];
 #pragma unroll
       for (int q = 0; q < 8; q++)
-        if (c0 + q < ncols) acc[q] += V[(size_t)(c0 + q) * ldv + i] * wi;
+        if (c0 + q < ncols) acc[q] += U[(size_t)(c0 + q) * ldv + i] * wi;
     }
 #pragma unroll
     for (int q = 0; q < 8; q++) {
@@ -387,19 +406,20 @@ __global__ void __launch_bounds__(kDotThreads) dots_kernel(int n, int ncols,
     double s = 0.0;
     for (int wq = 0; wq < kDotThreads / 32; wq++) s += red[wq][tid];
     partial[(size_t)blockIdx.x * kMaxCols + tid] = s;
+    __threadfence();
   }
-}
-
-// One warp per column: lane l sums blocks l, l + 32, ... in order, then a
-// fixed shuffle tree adds the lanes (deterministic).
-__global__ void dots_finalize_kernel(int ncols, int nblk, const double* __restrict__ partial,
-                                     double* __restrict__ out) {
-  const int c = blockIdx.x, lane = threadIdx.x;
-  if (c >= ncols) return;
-  double s = 0.0;
-  for (int b = lane; b < nblk; b += 32) s += partial[(size_t)b * kMaxCols + c];
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if (lane == 0) out[c] = s;
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = warp; c < ncols; c += kDotThreads / 32) {
+    double s = 0.0;
+    for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(&partial[(size_t)b * kMaxCols + c]);
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+    if (lane == 0) out[c] = s;
+  }
+  if (tid == 0) *done = 0u;
 }
 
 // w += sign * sum_c coef[c] V[c]
@@ -416,12 +436,13 @@ __global__ void axpy_multi_kernel(int n, int ncols, const double* __restrict__ V
   }
 }
 
-__global__ void scale_dev_kernel(int n, const double* __restrict__ s, double* __restrict__ w) {
-  const double f = 1.0 / s[0];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] *= f;
-}
-__global__ void scale_kernel(int n, double s, double* __restrict__ w) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] *= s;
+// w *= s, and a copy of the result
+__global__ void scale_kernel(int n, double s, double* __restrict__ w, double* __restrict__ copy) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double v = w[i] * s;
+    w[i] = v;
+    copy[i] = v;
+  }
 }
 __global__ void sub_kernel(int n, const double* __restrict__ a, const double* __restrict__ b,
                            double* __restrict__ o) {
@@ -479,42 +500,36 @@ void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, 
   moments_reduce_kernel<<<grid, 128, 0, st>>>(C, Pf, t0, t1);
 }
 
-void launch_permute(int n, const int* perm, const double* q3, double* qx, double* qy, double* qz,
-                    float* fqx, float* fqy, float* fqz, const PackSrc& ps, cudaStream_t st) {
+void launch_permute(const PermTree& t0, const PermTree& t1, int pack, cudaStream_t st) {
+  const int n = t0.n + t1.n;
   if (n <= 0) return;
-  permute_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, perm, q3, qx, qy, qz, fqx, fqy, fqz, ps);
+  permute_kernel<<<(n + 255) / 256, 256, 0, st>>>(t0, t1, pack);
 }
 
-void launch_permute_soa(int n, const int* perm, const double* src, double* dst, cudaStream_t st) {
+void launch_interp(const InterpSet& s0, const InterpSet& s1, cudaStream_t st) {
+  const int n = 3 * (s0.ne + s1.ne);
   if (n <= 0) return;
-  permute_soa_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, perm, src, dst);
+  interp_kernel<<<(n + 127) / 128, 128, 0, st>>>(s0, s1);
 }
 
-void launch_interp(int ne, const int* tgt, const int* idx, const double* pq, const double* g,
-                   double* g0, cudaStream_t st) {
-  if (ne <= 0) return;
-  interp_kernel<<<(ne + 127) / 128, 128, 0, st>>>(ne, tgt, idx, pq, g, g0);
+void launch_matvec_combine(const CombineSet& s0, const CombineSet& s1, double factor, const double* x, double* y,
+                           cudaStream_t st) {
+  matvec_combine_kernel<<<(s0.n + s1.n + 255) / 256, 256, 0, st>>>(s0, s1, factor, x, y);
 }
 
-void launch_matvec_combine(int n, double factor, const double* x, const double* on,
-                           const double* comp, double* y, cudaStream_t st) {
-  if (n <= 0) return;
-  matvec_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, factor, x, on, comp, y);
+void launch_rhs_combine(const CombineSet& s0, const CombineSet& s1, double factor, double* b, cudaStream_t st) {
+  rhs_combine_kernel<<<(s0.n + s1.n + 255) / 256, 256, 0, st>>>(s0, s1, factor, b);
 }
 
-void launch_rhs_combine(int n, double factor, const double* on, const double* comp, double* b,
-                        cudaStream_t st) {
-  if (n <= 0) return;
-  rhs_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, factor, on, comp, b);
-}
-
-void launch_dots(int n, int ncols, const double* V, long ldv, const double* w, double* partial,
+void launch_dots(int n, int ncols, const double* U, long ldv, const double* w, const DotWork& d, double* out,
                  cudaStream_t st) {
-  dots_kernel<<<kRedBlocks, kDotThreads, 0, st>>>(n, ncols, V, ldv, w, partial);
+  dots_kernel<false><<<kRedBlocks, kDotThreads, 0, st>>>(n, 0, nullptr, ldv, nullptr, const_cast<double*>(w), ncols, U,
+                                                         d.partial, d.done, out);
 }
 
-void launch_dots_finalize(int ncols, const double* partial, double* out, cudaStream_t st) {
-  dots_finalize_kernel<<<ncols, 32, 0, st>>>(ncols, kRedBlocks, partial, out);
+void launch_sub_dots(int n, int nsub, const double* V, long ldv, const double* coef, double* w, int ncols,
+                     const double* U, const DotWork& d, double* out, cudaStream_t st) {
+  dots_kernel<true><<<kRedBlocks, kDotThreads, 0, st>>>(n, nsub, V, ldv, coef, w, ncols, U, d.partial, d.done, out);
 }
 
 void launch_axpy_multi(int n, int ncols, const double* V, long ldv, const double* coef,
@@ -522,11 +537,8 @@ void launch_axpy_multi(int n, int ncols, const double* V, long ldv, const double
   axpy_multi_kernel<<<nblk(n, 256), 256, 0, st>>>(n, ncols, V, ldv, coef, sign, w);
 }
 
-void launch_scale(int n, const double* s_dev, double* w, cudaStream_t st) {
-  scale_dev_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s_dev, w);
-}
-void launch_scale_host(int n, double s, double* w, cudaStream_t st) {
-  scale_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s, w);
+void launch_scale_copy(int n, double s, double* w, double* copy, cudaStream_t st) {
+  scale_kernel<<<nblk(n, 256), 256, 0, st>>>(n, s, w, copy);
 }
 void launch_sub(int n, const double* a, const double* b, double* out, cudaStream_t st) {
   sub_kernel<<<nblk(n, 256), 256, 0, st>>>(n, a, b, out);

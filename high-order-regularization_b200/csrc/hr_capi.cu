@@ -387,7 +387,7 @@ extern "C" int hr_interpolate_dl_density(hr_ctx* ctx, double h, const hr_surface
     dg0.alloc(3 * (size_t)std::max(1, T->n));
     dg0.zero(st);
     ctx->c.ws.flush(st);
-    launch_interp(ds.ne, ds.tgt.p, ds.idx.p, ds.pq.p, dg.p, dg0.p, st);
+    launch_interp({ds.ne, ds.tgt.p, ds.idx.p, ds.pq.p, dg.p, dg0.p}, InterpSet{}, st);
     ctx->c.launches++;
     HR_CHECK_CUDA(cudaGetLastError());
     d2h_staged(ctx->c, g0, dg0.p, sizeof(double) * 3 * T->n);
@@ -509,6 +509,7 @@ struct hr_plan2s {
   // GMRES work space
   int Vcols = 0;
   DBuf<double> V, r, bsave, partial, hbuf, ybuf;
+  DBuf<unsigned> done;  // finished blocks of a reduction, zero between launches
   // Optional treecode of the reduced-precision inner operator of GMRES-IR:
   // trees and interaction lists of its own over the same targets, stencils
   // and output buffers.
@@ -688,20 +689,18 @@ void plan_matvec(hr_plan2s& P, const double* x_dev, double* y_dev, int prec) {
   DevTree* trees = in ? in->tree : P.tree;
   plan_ready(P);  // the stencils and the FP64 stresslet batch
   set_densities(C, &trees[0], &trees[1], P.xin.p + P.off[0], P.xin.p + P.off[1], PACK_DL, tree, prec != HR_FP64);
-  for (int t = 0; t < 2; t++) {
-    P.tg[t].g0.zero(st);
-    launch_interp(P.sten[t].ne, P.sten[t].tgt.p, P.sten[t].idx.p, P.sten[t].pq.p,
-                  P.xin.p + P.off[1 - t], P.tg[t].g0.p, st);
-    C.launches++;
-  }
+  // the other targets' g0 stays zero
+  auto interp = [&](int t) -> InterpSet {
+    return {P.sten[t].ne, P.sten[t].tgt.p, P.sten[t].idx.p, P.sten[t].pq.p, P.xin.p + P.off[1 - t], P.tg[t].g0.p};
+  };
+  launch_interp(interp(0), interp(1), st);
+  C.launches++;
   if (!in && !P.dl[prec].ready) dl_batches(P, P.tree, P.Lon, P.Loff, P.dl, prec, prec + 1, true, st);
   (in ? in->dl[prec] : P.dl[prec]).launch(C);
   // set 0: u - on*f - comp*f ; set 1: u - comp*f - on*f   (2S/main.cpp:612-676)
-  launch_matvec_combine(3 * P.nq[0], 2.0 / 3.0, P.xin.p + P.off[0], P.out_on[0].p, P.out_off[0].p,
-                        y_dev + P.off[0], st);
-  launch_matvec_combine(3 * P.nq[1], 2.0 / 3.0, P.xin.p + P.off[1], P.out_off[1].p, P.out_on[1].p,
-                        y_dev + P.off[1], st);
-  C.launches += 2;
+  launch_matvec_combine({3 * P.nq[0], P.out_on[0].p, P.out_off[0].p}, {3 * P.nq[1], P.out_off[1].p, P.out_on[1].p},
+                        2.0 / 3.0, P.xin.p, y_dev, st);
+  C.launches++;
   HR_CHECK_CUDA(cudaGetLastError());
 }
 
@@ -718,17 +717,16 @@ void plan_rhs(hr_plan2s& P, const double* f1_dev, const double* f2_dev, double* 
   set_densities(C, &P.tree[0], &P.tree[1], P.fin.p + P.off[0], P.fin.p + P.off[1], PACK_SL, tree, false);
   P.sl.launch(C);
   // SL_1 = on1 + comp2 ; SL_2 = comp1 + on2 ; b = -SL * 2/3
-  launch_rhs_combine(3 * P.nq[0], 2.0 / 3.0, P.out_on[0].p, P.out_off[0].p, b_dev + P.off[0], st);
-  launch_rhs_combine(3 * P.nq[1], 2.0 / 3.0, P.out_off[1].p, P.out_on[1].p, b_dev + P.off[1], st);
-  C.launches += 2;
+  launch_rhs_combine({3 * P.nq[0], P.out_on[0].p, P.out_off[0].p}, {3 * P.nq[1], P.out_off[1].p, P.out_on[1].p},
+                     2.0 / 3.0, b_dev, st);
+  C.launches++;
   HR_CHECK_CUDA(cudaGetLastError());
 }
 
 double dev_norm(hr_plan2s& P, const double* v) {
   Ctx& C = *P.C;
-  launch_dots(P.n, 1, v, P.n, v, P.partial.p, C.stream);
-  launch_dots_finalize(1, P.partial.p, P.hbuf.p, C.stream);
-  C.launches += 2;
+  launch_dots(P.n, 1, v, P.n, v, {P.partial.p, P.done.p}, P.hbuf.p, C.stream);
+  C.launches++;
   double h;
   HR_CHECK_CUDA(cudaMemcpyAsync(&h, P.hbuf.p, sizeof(double), cudaMemcpyDeviceToHost, C.stream));
   HR_CHECK_CUDA(cudaStreamSynchronize(C.stream));
@@ -827,7 +825,7 @@ int plan_solve(hr_plan2s& P, const hr_gmres_opts& o, const double* b_dev, double
     const double err_start = error;
     const double cycle_tol = (refine && !fp64_tail) ? std::max(0.5 * o.tol, eta * err_start) : o.tol;
     launch_copy(n, r, P.V.p, st);
-    launch_scale_host(n, 1.0 / r_norm, P.V.p, st);
+    launch_scale_copy(n, 1.0 / r_norm, P.V.p, P.xin.p, st);
     C.launches += 2;
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = r_norm;
@@ -835,31 +833,25 @@ int plan_solve(hr_plan2s& P, const hr_gmres_opts& o, const double* b_dev, double
     while (j < m - 1 && error > cycle_tol && iter < max_iter) {
       j++;
       iter++;
-      double* vj = P.V.p + (size_t)j * n;
       double* w = P.V.p + (size_t)(j + 1) * n;
       const int prec = (refine && !fp64_tail) ? o.precision : HR_FP64;
-      plan_matvec(P, vj, w, prec);
+      plan_matvec(P, P.xin.p, w, prec);  // xin holds V[j] (launch_scale_copy)
       if (prec) R.matvecs_mixed++;
       else R.matvecs_fp64++;
-      // CGS2
-      launch_dots(n, j + 1, P.V.p, n, w, P.partial.p, st);
-      launch_dots_finalize(j + 1, P.partial.p, P.hbuf.p, st);
-      launch_axpy_multi(n, j + 1, P.V.p, n, P.hbuf.p, -1.0, w, st);
-      launch_dots(n, j + 1, P.V.p, n, w, P.partial.p, st);
-      launch_dots_finalize(j + 1, P.partial.p, P.hbuf.p + 64, st);
-      launch_axpy_multi(n, j + 1, P.V.p, n, P.hbuf.p + 64, -1.0, w, st);
-      launch_dots(n, 1, w, n, w, P.partial.p, st);
-      launch_dots_finalize(1, P.partial.p, P.hbuf.p + 128, st);
-      C.launches += 8;
+      // CGS2: h1 = V.w; w -= V h1, h2 = V.w; w -= V h2, |w|^2
+      const DotWork dw{P.partial.p, P.done.p};
+      launch_dots(n, j + 1, P.V.p, n, w, dw, P.hbuf.p, st);
+      launch_sub_dots(n, j + 1, P.V.p, n, P.hbuf.p, w, j + 1, P.V.p, dw, P.hbuf.p + 64, st);
+      launch_sub_dots(n, j + 1, P.V.p, n, P.hbuf.p + 64, w, 1, w, dw, P.hbuf.p + 128, st);
+      C.launches += 3;
       HR_CHECK_CUDA(cudaMemcpyAsync(hh.data(), P.hbuf.p, sizeof(double) * 129, cudaMemcpyDeviceToHost, st));
       HR_CHECK_CUDA(cudaStreamSynchronize(st));
       for (int i = 0; i <= j; i++) Hm(i, j) = hh[i] + hh[64 + i];
       double v_norm = sqrt(hh[128]);
       Hm(j + 1, j) = v_norm;
-      if (v_norm != 0.0) {
-        launch_scale_host(n, 1.0 / v_norm, w, st);
-        C.launches++;
-      }
+      // the next basis vector, also into the operator's input
+      launch_scale_copy(n, v_norm != 0.0 ? 1.0 / v_norm : 1.0, w, P.xin.p, st);
+      C.launches++;
       for (int i = 0; i <= j - 1; i++) {
         double t = Hm(i, j);
         Hm(i, j) = cs[i] * t + sn[i] * Hm(i + 1, j);
@@ -1001,10 +993,13 @@ extern "C" int hr_plan2s_create(hr_ctx* ctx, const hr_scene2s* sc, const hr_eval
       P->out_off[t].alloc(3 * (size_t)T.n);
     };
     run_both(ctx->c.device, [&] { per_target_set(1); }, [&] { per_target_set(0); });
+    for (int s = 0; s < 2; s++) P->tree[s].pk.zero(st);
     P->xin.alloc(P->n);
     P->fin.alloc(P->n);
     P->r.alloc(P->n);
     P->partial.alloc((size_t)kRedBlocks * 64);
+    P->done.alloc(1);
+    P->done.zero(st);
     P->hbuf.alloc(256);
     P->ybuf.alloc(64);
     plan_batches(*P);

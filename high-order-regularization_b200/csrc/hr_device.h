@@ -127,37 +127,53 @@ struct MomTree {
 void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st);
 void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, cudaStream_t st);
 
-// Gathers interleaved reference-order density into tree-order SoA.
-// and fills the density of the packed records pk (xyz, normals and areas of
-// the tree) as `pack` says.
-struct PackSrc {
-  const double *x, *y, *z, *nx, *ny, *nz, *a;
+// Gathers the interleaved reference-order densities of one or two trees into
+// tree-order SoA, FP32 copies (fqx, if not null) and packed records as `pack`
+// says (pk, if not null).
+struct PermTree {
+  int n;
+  const int* perm;
+  const double *q3, *x, *y, *z, *nx, *ny, *nz, *a;
+  double *qx, *qy, *qz;
+  float *fqx, *fqy, *fqz;
   double* pk;
-  int pack;
 };
-void launch_permute(int n, const int* perm, const double* q3, double* qx, double* qy, double* qz,
-                    float* fqx, float* fqy, float* fqz, const PackSrc& ps, cudaStream_t st);
-void launch_permute_soa(int n, const int* perm, const double* src, double* dst, cudaStream_t st);
+void launch_permute(const PermTree& t0, const PermTree& t1, int pack, cudaStream_t st);
 
-// Six-point density interpolation at nearest points.
-void launch_interp(int ne, const int* tgt, const int* idx, const double* pq, const double* g,
-                   double* g0, cudaStream_t st);
+// Six-point density interpolation at nearest points, one or two target sets.
+struct InterpSet {
+  int ne;  // entries
+  const int *tgt, *idx;
+  const double *pq, *g;
+  double* g0;
+};
+void launch_interp(const InterpSet& s0, const InterpSet& s1, cudaStream_t st);
 
-// Two-surface combine steps.
-void launch_matvec_combine(int n, double factor, const double* x, const double* on,
-                           const double* comp, double* y, cudaStream_t st);
-void launch_rhs_combine(int n, double factor, const double* on, const double* comp, double* b,
-                        cudaStream_t st);
+// Two-surface combine steps; a is taken before b.
+struct CombineSet {
+  int n;
+  const double *a, *b;
+};
+void launch_matvec_combine(const CombineSet& s0, const CombineSet& s1, double factor, const double* x, double* y,
+                           cudaStream_t st);
+void launch_rhs_combine(const CombineSet& s0, const CombineSet& s1, double factor, double* b, cudaStream_t st);
 
 // Vector kernels for GMRES (deterministic reductions).
 constexpr int kRedBlocks = 296;
-void launch_dots(int n, int ncols, const double* V, long ldv, const double* w, double* partial,
+struct DotWork {
+  double* partial;  // kRedBlocks x 64
+  unsigned* done;   // zero between launches
+};
+// out[c] = U[c] . w (columns of stride ldv)
+void launch_dots(int n, int ncols, const double* U, long ldv, const double* w, const DotWork& d, double* out,
                  cudaStream_t st);
-void launch_dots_finalize(int ncols, const double* partial, double* out, cudaStream_t st);
+// w -= sum_c coef[c] V[c], then out[c] = U[c] . w
+void launch_sub_dots(int n, int nsub, const double* V, long ldv, const double* coef, double* w, int ncols,
+                     const double* U, const DotWork& d, double* out, cudaStream_t st);
 void launch_axpy_multi(int n, int ncols, const double* V, long ldv, const double* coef,
                        double sign, double* w, cudaStream_t st);
-void launch_scale(int n, const double* s_dev, double* w, cudaStream_t st);
-void launch_scale_host(int n, double s, double* w, cudaStream_t st);
+// w *= s; copy = w
+void launch_scale_copy(int n, double s, double* w, double* copy, cudaStream_t st);
 void launch_sub(int n, const double* a, const double* b, double* out, cudaStream_t st);
 void launch_copy(int n, const double* a, double* out, cudaStream_t st);
 

@@ -1002,12 +1002,14 @@ __global__ void __launch_bounds__(kTB) reduce_kernel(const EvalTask* __restrict_
   const int t = T.tord[k];
   double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
   const int s0 = T.item_start[blk], s1 = T.item_start[blk + 1];
-  for (int s = s0; s < s1; s++) {
-    const double* p = T.partial + ((size_t)s * kTB + tid) * kPartComps;
-    a0 += p[0];
-    a1 += p[1];
-    a2 += p[2];
-    a3 += p[3];
+#pragma unroll 8
+  for (int s = s0; s < s1; s++) {  // eight slots' loads in flight
+    const double2* p = reinterpret_cast<const double2*>(T.partial + ((size_t)s * kTB + tid) * kPartComps);
+    const double2 u = p[0], v = p[1];
+    a0 += u.x;
+    a1 += u.y;
+    a2 += v.x;
+    a3 += v.y;
   }
   const double sc = T.scale;
   double* o = T.out;

@@ -328,13 +328,15 @@ void DevTree::set_density(Ctx& C, const double* q3_dev, int pack, bool moments, 
 void set_densities(Ctx& C, DevTree* t0, DevTree* t1, const double* q0, const double* q1, int pack, bool moments,
                    bool tc) {
   const bool dl = pack == PACK_DL;
-  for (int s = 0; s < 2; s++) {
-    DevTree* t = s == 0 ? t0 : t1;
-    if (!t) continue;
-    launch_permute(t->n, t->perm.p, s == 0 ? q0 : q1, t->qx.p, t->qy.p, t->qz.p, t->fqx.p, t->fqy.p, t->fqz.p,
-                   {t->x.p, t->y.p, t->z.p, t->nx.p, t->ny.p, t->nz.p, t->a.p, t->pk.p, pack}, C.stream);
-    C.launches++;
-  }
+  // the packed records are what the FP64 sums read
+  auto perm = [&](DevTree* t, const double* q) -> PermTree {
+    if (!t) return PermTree{};
+    return {t->n,    t->perm.p, q,       t->x.p,  t->y.p,   t->z.p,   t->nx.p,  t->ny.p,
+            t->nz.p, t->a.p,    t->qx.p, t->qy.p, t->qz.p,  t->fqx.p, t->fqy.p, t->fqz.p,
+            tc ? nullptr : t->pk.p};
+  };
+  launch_permute(perm(t0, q0), perm(t1, q1), pack, C.stream);
+  C.launches++;
   if (!moments || t0->nitems + (t1 ? t1->nitems : 0) == 0) return;
   const MomTree m0 = t0->mom_tree(), m1 = t1 ? t1->mom_tree() : MomTree{};
   int ch = dl ? 9 : 6;
