@@ -214,11 +214,11 @@ __global__ void __launch_bounds__(kMomWarps * 32) moments_kernel(MomTree t0, Mom
 //   d.M.d = M00 d0^2 + M11 d1^2 + M22 d2^2 + (M01 + M10) d0 d1
 //         + (M02 + M20) d0 d2 + (M12 + M21) d1 d2   and   Mn.d,
 // so they are stored as those 6 symmetric combinations and Mn: FP64 10
-// doubles per proxy (the last one zero), FP32 12 floats (the last three zero).
+// doubles per proxy (the last one zero), FP32 as momf_stride says.
 // The FP64 upward pass gives the combinations (C = 9), the tensor-core one the
 // 12 products g-major, then n (C = 12). The Stokeslet's 6 channels (f, n) are
-// stored as they are: FP64 6 doubles, FP32 8 floats (the last two zero).
-__global__ void moments_reduce_kernel(int C, int Pf, MomTree t0, MomTree t1) {
+// stored as they are: FP64 6 doubles, FP32 likewise in pairs.
+__global__ void moments_reduce_kernel(int C, int P1, int Pf, MomTree t0, MomTree t1) {
   // one thread per (node, proxy, stored value): a value is one channel, or of
   // 12 channels the sum of two, each summed over the node's items in item order
   const bool first = (int)blockIdx.x < t0.nn;
@@ -246,14 +246,13 @@ __global__ void moments_reduce_kernel(int C, int Pf, MomTree t0, MomTree t1) {
   }
   const double v = c1 >= 0 ? s0 + s1 : s0;
   const size_t k = (size_t)node * Pf + kk;
+  const int row = kk / P1, pk = kk - row * P1, pair = row * ((P1 + 1) / 2) + pk / 2, half = pk & 1;
   if (dl) {
     t.mom[k * 10 + o] = v;  // o = 9: the zero pad
-    t.momf[k * 12 + o] = (float)v;
-    if (o == 9) t.momf[k * 12 + 10] = t.momf[k * 12 + 11] = 0.f;
+    if (o < 9) t.momf[node * momf_stride(P1, 20) + (size_t)pair * 20 + 2 * o + half] = (float)v;
   } else {
     t.mom[k * 6 + o] = v;
-    t.momf[k * 8 + o] = (float)v;
-    if (o == 5) t.momf[k * 8 + 6] = t.momf[k * 8 + 7] = 0.f;
+    t.momf[node * momf_stride(P1, 12) + (size_t)pair * 12 + 2 * o + half] = (float)v;
   }
 }
 
@@ -494,10 +493,11 @@ void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStr
   fn<<<dim3(nitems, m.ctas), m.warps * 32, m.smem, st>>>(t0, t1, m);
 }
 
-void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, cudaStream_t st) {
+void launch_moments_reduce(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st) {
   if (t0.nn + t1.nn <= 0) return;
+  const int Pf = P1 * P1 * P1;
   dim3 grid(t0.nn + t1.nn, (Pf + 127) / 128, C == 6 ? 6 : 10);
-  moments_reduce_kernel<<<grid, 128, 0, st>>>(C, Pf, t0, t1);
+  moments_reduce_kernel<<<grid, 128, 0, st>>>(C, P1, Pf, t0, t1);
 }
 
 void launch_permute(const PermTree& t0, const PermTree& t1, int pack, cudaStream_t st) {

@@ -29,7 +29,7 @@ struct EvalTask {
   const float *fnx, *fny, *fnz, *fa, *fqx, *fqy, *fqz;  // FP32 copies (reduced-precision sums)
   const double* tcheb;                                // 3*P1 per node
   const double* mom;                                  // Pf*C per node, proxy-major
-  const float* momf;                                  // Pf*W32 per node (W32 = 12 DL, 8 SL)
+  const float* momf;                                  // FP32 copy per node: momf_stride floats
   const int* tord;                                    // target order -> target index
   const double* txyz;                                 // 3nt targets
   const double* tb;                                   // nt signed distances
@@ -53,7 +53,7 @@ struct Seg {
   int s0, s1;
 };
 
-// One CTA's work: a run of consecutive segments of one target block. Each
+// A work item: a run of consecutive segments of one target block. Each
 // item writes its partial sums into its own slot; the reduce kernel adds the
 // slots of a block in order, so results do not depend on scheduling.
 struct BlockRef {
@@ -75,13 +75,13 @@ enum Pack : int {
 
 // The reduced-precision sums of a batch: every work item of a combined list,
 // the first n_on items (lean: on-surface tasks, or the extend-to-grid box-face
-// sums) in one launch on st, the rest in another on side.
+// sums) in one launch on st, the rest in another on side. next: two zeroed work
+// counters (one per launch); launch_reduce zeroes them again.
 void launch_eval(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems, int n_on,
-                 cudaStream_t st, cudaStream_t side);
+                 unsigned* next, int num_sms, cudaStream_t st, cudaStream_t side);
 
-// The FP64 sums of a batch likewise (hr_eval64.cu). next: two zeroed work
-// counters (one per launch); launch_reduce zeroes them again. With count, the
-// per-branch pair counts are added to the tasks' counters.
+// The FP64 sums of a batch likewise (hr_eval64.cu). With count, the per-branch
+// pair counts are added to the tasks' counters.
 void launch_eval64(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems,
                    int n_on, unsigned* next, int num_sms, cudaStream_t st, cudaStream_t side, bool count);
 // The batch's reduction (the items' partial sums per target, in slot order) and
@@ -112,6 +112,12 @@ void launch_moments_tc(int dl, const MomItem* d_items, int nitems, int P1, const
                        const double* y, const double* z, const double* nx, const double* ny, const double* nz,
                        const double* a, const double* qx, const double* qy, const double* qz, double* partial,
                        int* err, cudaStream_t st);
+// The FP32 moments of a node: per Chebyshev row (P+1)/2 pairs of proxies (an
+// odd last one fills half a pair), interleaved value by value: 20 floats per
+// pair of the stresslet's 9 values, 12 of the Stokeslet's 6.
+inline __host__ __device__ size_t momf_stride(int P1, int pair_floats) {
+  return (size_t)P1 * P1 * ((P1 + 1) / 2) * pair_floats;
+}
 // One tree's part of an upward pass.
 struct MomTree {
   const MomItem* items;
@@ -125,7 +131,7 @@ struct MomTree {
 // degree: C = 9 stresslet, 6 Stokeslet channels; then the reduction per node (C
 // = 12: the layout of launch_moments_tc).
 void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st);
-void launch_moments_reduce(int C, int Pf, const MomTree& t0, const MomTree& t1, cudaStream_t st);
+void launch_moments_reduce(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStream_t st);
 
 // Gathers the interleaved reference-order densities of one or two trees into
 // tree-order SoA, FP32 copies (fqx, if not null) and packed records as `pack`

@@ -1,17 +1,31 @@
 // hr_eval.cu — the reduced-precision boundary sums (HR_MIXED, HR_FP32) and the
 // reduction of every batch; the FP64 sums are in hr_eval64.cu.
 //
-// One CTA owns one block of 128 spatially sorted targets (one target per
-// thread, FP64 accumulators in registers) and walks that block's interaction
-// entries in a fixed order, so every result is deterministic:
-//   * near entry  -> direct sum over the node's member sources, staged in
-//                    shared memory in tiles (Call_Ds_*, 2S/KITC.cpp:807-1062;
-//                    in direct mode the single node holds all sources, i.e.
-//                    eval_Stokes_*_{on,off}Surf of 2S/stokeslets.cpp and
-//                    2S/stresslets.cpp, and the sums of E2G/stokes.cpp);
-//   * far entry   -> the node's (P+1)^3 proxy points with their moments staged
-//                    in shared memory (Call_Treecode_*, 2S/KITC.cpp:671-777).
-// A warp whose mask word is zero for an entry skips the arithmetic entirely.
+// Two-surface sums: one persistent CTA of 12 warps per SM; every warp takes
+// units (half a block of 128 spatially sorted targets, two targets per lane,
+// FP64 accumulators in registers) from a common counter, walks the unit's
+// interaction segments in order and writes the unit's own partial sums, so
+// results do not depend on scheduling. Extend-to-grid sums: a CTA per item.
+//   * near segment -> direct sum over the node's member sources, staged in
+//                     shared memory in tiles (Call_Ds_*, 2S/KITC.cpp:807-1062;
+//                     in direct mode the single node holds all sources, i.e.
+//                     eval_Stokes_*_{on,off}Surf of 2S/stokeslets.cpp and
+//                     2S/stresslets.cpp, and the sums of E2G/stokes.cpp);
+//   * far segment  -> the node's (P+1)^3 proxy points with their moments staged
+//                     in shared memory (Call_Treecode_*, 2S/KITC.cpp:671-777).
+//
+// What bounds the two-surface kernels: the issue slots and the FP32 pipe. The
+// packed operations (two sources or two proxies of a target per instruction)
+// have the pipe's FP32 rate at half the issue slots: a probe gives 0.47 packed
+// FMAs per cycle and SM quarter against 1.0 scalar ones (0.38 with three
+// different operands). With them, rsqrt without denormal scaling and units
+// taken by the warp, the stresslet batch's kernels (two-surface problem, h =
+// 1/64, P = 6, N0 = 2000) execute 0.73e9 + 0.69e9 instructions instead of
+// 1.21e9 + 0.90e9; on-surface 1.92 -> 1.18 ms, off-surface 1.71 -> 1.25 ms,
+// the operator application 3.55 -> 2.49 ms against one scalar pair at a time
+// in CTAs per item. Twelve warps: 168 registers, two targets' sums without
+// spills; 8 / 10 / 13 / 14 warps 3.41 (8, before the finer items) / 2.57 /
+// 2.55 / 2.62 ms.
 //
 // Precision. MIXED: FP32 pairs from FP32 coordinates relative to the target
 // block's first target, summed per 16 terms in FP32 and added to the FP64
@@ -35,17 +49,19 @@ namespace {
 #define HR_SMOOTH_STORAGE __device__ const
 #include "hr_smoothing_tables.inc"
 
-constexpr int kSmooth32N = HR_SMOOTH32_PIECES * 8;  // floats per FP32 table
+// The singular kernel takes over at s = kPlainOnSurf32; the tables are staged
+// up to there, in kRep32 copies (a lane reads copy lane & 7).
+constexpr int kPieces32 = (int)(kPlainOnSurf32 * HR_SMOOTH32_PIECES / 64.0f) + 1, kRep32 = 8;
 
 // FP32 piece: (centre, c0, c1, c2) (c3, c4, c5, 0); index floor(s * pieces / 64)
-// for 0 <= s <= 64, formed on the FMA / ALU pipes: adding 1.5 * 2^23 to
-// s * pieces / 64 - 1/2 leaves round-to-nearest of it, i.e. the floor (a tie
+// for 0 <= s <= kPlainOnSurf32, formed on the FMA / ALU pipes: adding 1.5 * 2^23
+// to s * pieces / 64 - 1/2 leaves round-to-nearest of it, i.e. the floor (a tie
 // picks the lower piece, whose polynomial covers its right end), in the low
 // mantissa bits.
 __device__ __forceinline__ float smooth_eval_f(const float4* __restrict__ tab, float s) {
   const float f = fmaf(s, HR_SMOOTH32_PIECES / 64.0f, -0.5f) + 12582912.0f;
-  const int i = min(__float_as_int(f) - 0x4B400000, HR_SMOOTH32_PIECES - 1);
-  const float4 a = tab[2 * i], b = tab[2 * i + 1];
+  const int i = __float_as_int(f) - 0x4B400000;
+  const float4 a = tab[2 * i * kRep32], b = tab[(2 * i + 1) * kRep32];
   const float t = s - a.x;
   return fmaf(fmaf(fmaf(fmaf(fmaf(b.z, t, b.y), t, b.x), t, a.w), t, a.z), t, a.y);
 }
@@ -255,42 +271,7 @@ __device__ __forceinline__ void pair64_band(const double* __restrict__ sm, int j
   }
 }
 
-// ------------------------------------------------------- FP32 plain pairs
-// The singular kernel of a far target (the r/delta > 8 branch of the reference),
-// from FP32 centre-relative coordinates.
-template <int KIND>
-__device__ __forceinline__ void pair32(const float4* __restrict__ s4, int j, const Tgt32& F,
-                                       float& p0, float& p1, float& p2) {
-  const float4 P = s4[j];  // x, y, z, area
-  const float4 N = s4[kNT + j];
-  const float4 Q = s4[2 * kNT + j];
-  const float dx = F.px - P.x, dy = F.py - P.y, dz = F.pz - P.z;
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  const float rinv = rsqrtf(r2);
-  const float rinv2 = rinv * rinv;
-  if (KIND == K_SL_OFF) {
-    const float fx = Q.x - F.f0n0 * N.x;
-    const float fy = Q.y - F.f0n0 * N.y;
-    const float fz = Q.z - F.f0n0 * N.z;
-    const float fdd = fx * dx + fy * dy + fz * dz;
-    const float H1 = P.w * rinv;
-    const float H2 = fdd * H1 * rinv2;
-    p0 += fx * H1 + dx * H2;
-    p1 += fy * H1 + dy * H2;
-    p2 += fz * H1 + dz * H2;
-  } else {  // K_DL_OFF
-    const float gx = Q.x - F.g0[0];
-    const float gy = Q.y - F.g0[1];
-    const float gz = Q.z - F.g0[2];
-    const float gdd = gx * dx + gy * dy + gz * dz;
-    const float ndd = N.x * dx + N.y * dy + N.z * dz;
-    const float kernel = ndd * gdd * (rinv2 * rinv2 * rinv) * P.w;
-    p0 += dx * kernel;
-    p1 += dy * kernel;
-    p2 += dz * kernel;
-  }
-}
-
+// ------------------------------------------------------- FP32 extend-to-grid pairs
 // The box-face sums (E2G/stokes.cpp:13-45, 102-126) in FP32 in one pass, sharing
 // the offset, the distance and f.dx.
 __device__ __forceinline__ void pair32_face(const float4* __restrict__ s4, int j, const Tgt32& F, float& p0,
@@ -346,55 +327,6 @@ __device__ __forceinline__ void pair32r_band(const float4* __restrict__ s4, int 
     const float normal = -(f_dot_n - F.f0n0) * n_dot_dx;
     const float tangential = -(ncf0 * ncd0 + ncf1 * ncd1 + ncf2 * ncd2);
     p3 += (normal + tangential) * H2p * P.w;
-  }
-}
-
-// ------------------------------------- FP32 on-surface pairs, all distances
-// Call_Ds_SL_onSurf / Call_Ds_DL_onSurf (2S/KITC.cpp:807-846, 921-957) in
-// FP32: the smoothing factor from the FP32 table for s = r^2/delta^2 <= 64,
-// the singular kernel beyond (a branch that only warps at the 8 delta
-// boundary split on).
-template <int KIND>
-__device__ __forceinline__ void pair32tab_src(const float4& P, const float4& N, const float4& Q, const Tgt32& F,
-                                              const RegF& gf, const float4* __restrict__ tab, float& p0, float& p1,
-                                              float& p2) {
-  const float dx = F.px - P.x, dy = F.py - P.y, dz = F.pz - P.z;
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  const float sq = r2 * gf.inv_d2;
-  if (KIND == K_SL_ON) {
-    const float fx = Q.x - F.f0n0 * N.x;
-    const float fy = Q.y - F.f0n0 * N.y;
-    const float fz = Q.z - F.f0n0 * N.z;
-    const float fdd = fx * dx + fy * dy + fz * dz;
-    float H1, H2;
-    if (sq <= kPlainOnSurf32) {
-      H1 = smooth_eval_f(tab, sq);
-      H2 = smooth_eval_f(tab + kSmooth32N / 4, sq);
-    } else {
-      H1 = rsqrtf(r2);
-      H2 = H1 * H1 * H1;
-    }
-    const float h2 = H2 * fdd;  // the tile holds area x density and area x normal
-    p0 += fx * H1 + dx * h2;
-    p1 += fy * H1 + dy * h2;
-    p2 += fz * H1 + dz * h2;
-  } else {  // K_DL_ON
-    const float gx = Q.x - F.g0[0];
-    const float gy = Q.y - F.g0[1];
-    const float gz = Q.z - F.g0[2];
-    const float gdd = gx * dx + gy * dy + gz * dz;
-    const float ndd = N.x * dx + N.y * dy + N.z * dz;
-    float H3;
-    if (sq <= kPlainOnSurf32) {
-      H3 = smooth_eval_f(tab, sq);
-    } else {
-      const float ri = rsqrtf(r2), ri2 = ri * ri;
-      H3 = ri2 * ri2 * ri;
-    }
-    const float kernel = ndd * gdd * H3;  // the tile holds area x normal
-    p0 += dx * kernel;
-    p1 += dy * kernel;
-    p2 += dz * kernel;
   }
 }
 
@@ -469,87 +401,640 @@ __device__ __forceinline__ void copy_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Proxy interactions of a run of Chebyshev rows (row r = i (P+1) + j holds
-// proxies (i, j, 0..P)) from the warp's shared copy of the node's proxy-major
-// moments, float4 (DL 3, SL 2 per proxy).
-// Stresslet per proxy: S = (M00, M11, M22, M01 + M10, M02 + M20, M12 + M21),
-// Mn (and padding); Stokeslet: f, n. Every lane reads the same proxy (a
-// shared-memory broadcast). The stresslet kernel uses
+// ------------------------------------------- two-surface sums: packed FP32
+// Two FP32 values in a 64-bit register: the packed operations round each half
+// as the scalar ones do. One instruction serves two sources (or two proxies)
+// of a target; the sums over sources stay scalar, in source order.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float lo(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f2 vfma(f2 a, f2 b, f2 c) {
+  f2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ f2 vmul(f2 a, f2 b) {
+  f2 v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ f2 vsub(f2 a, f2 b) {
+  f2 v;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+// rsqrtf without the scaling of denormal arguments (r below 1.1e-19)
+__device__ __forceinline__ float vrsqrt(float x) {
+  float v;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(v) : "f"(x));
+  return v;
+}
+__device__ __forceinline__ f2 vrsqrt(f2 x) { return pack2(vrsqrt(lo(x)), vrsqrt(hi(x))); }
+template <class V>
+__device__ __forceinline__ V dup(float x);
+template <>
+__device__ __forceinline__ float dup<float>(float x) {
+  return x;
+}
+template <>
+__device__ __forceinline__ f2 dup<f2>(float x) {
+  return pack2(x, x);
+}
+// p + a b and p + a, the halves in order
+__device__ __forceinline__ float sum_mul(float p, float a, float b) { return __fmaf_rn(a, b, p); }
+__device__ __forceinline__ float sum_mul(float p, f2 a, f2 b) {
+  return __fmaf_rn(hi(a), hi(b), __fmaf_rn(lo(a), lo(b), p));
+}
+__device__ __forceinline__ float sum(float p, float a) { return __fadd_rn(p, a); }
+__device__ __forceinline__ float sum(float p, f2 a) { return __fadd_rn(__fadd_rn(p, lo(a)), hi(a)); }
+
+// The FP32 data of a lane's target (offsets from the block's origin): of the
+// Stokeslet -f0.n0, of the stresslet -g0, zero without subtraction.
+struct Tgt2 {
+  float px, py, pz;
+  float m0, m1, m2;
+};
+
+template <bool DL>
+struct Rec {
+  static constexpr int vals = DL ? 9 : 6;          // FP32 moments per proxy
+  static constexpr int pair_b = DL ? 80 : 48;      // bytes of two proxies, interleaved value by value
+};
+
+// One proxy (V = float) or two (V = f2) of a Chebyshev row for one target.
+// Stresslet moments: S = (M00, M11, M22, M01 + M10, M02 + M20, M12 + M21), Mn;
+// Stokeslet: f, n. The stresslet kernel uses
 //   sum_l (sum_k (M[3l+k] - g0_l Mn_k) d_k) d_l = d.M.d - (g0.d)(Mn.d),
 // the reference's proxy sum (Call_Treecode_DL, 2S/KITC.cpp:753-771)
 // regrouped, with d.M.d from the symmetric part and the products of d0, d1
-// taken once per row; Call_Treecode_SL (2S/KITC.cpp:700-714) as written.
-// FP32 proxies, FP64 accumulation per Chebyshev row. P1C > 0 compiles the
-// row length (the proxy loop unrolls and the z coordinates stay in
-// registers); P1C = 0 takes any P1.
-template <bool DL, int P1C>
-__device__ __forceinline__ void proxies32_rows(const float4* __restrict__ s4, int row0, int nrows, int P1rt,
-                                               const float* __restrict__ chebf, const Tgt32& F, double& a0,
-                                               double& a1, double& a2) {
-  constexpr int W = DL ? 3 : 2;  // float4 per proxy
-  const int P1 = P1C > 0 ? P1C : P1rt;
-  float dz[P1C > 0 ? P1C : 1];
-  if constexpr (P1C > 0) {
-#pragma unroll
-    for (int pk = 0; pk < P1C; pk++) dz[pk] = F.pz - chebf[2 * P1C + pk];
+// taken once per row; Call_Treecode_SL (2S/KITC.cpp:700-714) as written. The
+// rounding of each operation, and so each result bit, is that of the scalar
+// loops this replaces, whose on-surface form (ON) sums Mn.d in another order.
+template <bool DL, bool ON, class V>
+struct RowT {
+  V d0, d1, r01, d00, d11, d01, s;  // s: DL the (d0, d1) part of -g0.d, SL -f0.n0
+  V pz, mz;
+  __device__ __forceinline__ RowT(const Tgt2& F, float cx, float cy) {
+    const float e0 = F.px - cx, e1 = F.py - cy;
+    const float e11 = __fmul_rn(e1, e1);
+    d0 = dup<V>(e0);
+    d1 = dup<V>(e1);
+    pz = dup<V>(F.pz);
+    if (DL) {
+      const float e00 = __fmul_rn(e0, e0);
+      d00 = dup<V>(e00);
+      r01 = dup<V>(__fadd_rn(e00, e11));
+      d11 = dup<V>(e11);
+      d01 = dup<V>(__fmul_rn(e0, e1));
+      s = dup<V>(__fmaf_rn(F.m0, e0, __fmul_rn(F.m1, e1)));
+      mz = dup<V>(F.m2);
+    } else {
+      r01 = dup<V>(__fmaf_rn(e0, e0, e11));
+      s = dup<V>(F.m0);
+    }
   }
+  __device__ __forceinline__ void add(const V (&m)[Rec<DL>::vals], V cz, float (&p)[3]) const {
+    const V d2 = vsub(pz, cz);
+    const V rinv = vrsqrt(vfma(d2, d2, r01));
+    if constexpr (DL) {
+      V dmd = vfma(m[0], d00, vmul(m[1], d11));
+      dmd = vfma(m[2], vmul(d2, d2), dmd);
+      dmd = vfma(m[3], d01, dmd);
+      dmd = vfma(m[4], vmul(d0, d2), dmd);
+      dmd = vfma(m[5], vmul(d1, d2), dmd);
+      const V mnd = vfma(m[8], d2, ON ? vfma(m[7], d1, vmul(m[6], d0)) : vfma(m[6], d0, vmul(m[7], d1)));
+      const V g0d = vfma(mz, d2, s);  // negated
+      const V ri2 = vmul(rinv, rinv);
+      const V kernel = vmul(vfma(g0d, mnd, dmd), vmul(vmul(ri2, ri2), rinv));
+      p[0] = sum_mul(p[0], d0, kernel);
+      p[1] = sum_mul(p[1], d1, kernel);
+      p[2] = sum_mul(p[2], d2, kernel);
+    } else {
+      const V m0 = vfma(s, m[3], m[0]), m1 = vfma(s, m[4], m[1]), m2 = vfma(s, m[5], m[2]);
+      const V temp = vmul(vfma(m2, d2, vfma(m0, d0, vmul(m1, d1))), vmul(vmul(rinv, rinv), rinv));
+      p[0] = sum(p[0], vfma(m0, rinv, vmul(temp, d0)));
+      p[1] = sum(p[1], vfma(m1, rinv, vmul(temp, d1)));
+      p[2] = sum(p[2], vfma(m2, rinv, vmul(temp, d2)));
+    }
+  }
+};
+
+// Proxy interactions of a run of Chebyshev rows (row r = i (P+1) + j holds
+// proxies (i, j, 0..P)) from the warp's shared copy of the node's moments,
+// two proxies at a time, an odd last one alone. Every lane reads the same
+// proxies (a shared-memory broadcast). FP32 per row, FP64 across the rows;
+// act: whose sums count. P1C > 0 compiles the row length.
+template <bool DL, bool ON, int NT, int P1C>
+__device__ __forceinline__ void proxy_rows(const char* buf, int row0, int nrows, int P1rt, const float* cheb,
+                                           const Tgt2 (&F)[NT], const bool (&act)[NT], double (&a)[NT][3]) {
+  constexpr int kV = Rec<DL>::vals;
+  const int P1 = P1C > 0 ? P1C : P1rt;
+  const int rowb = ((P1 + 1) / 2) * Rec<DL>::pair_b;
+  int pi = row0 / P1, pj = row0 - pi * P1;
   for (int r = 0; r < nrows; r++) {
-    const int pi = (row0 + r) / P1, pj = (row0 + r) - pi * P1;
-    const float d0 = F.px - chebf[pi];
-    const float d1 = F.py - chebf[P1 + pj];
-    const float r01 = d0 * d0 + d1 * d1;
-    const float d00 = d0 * d0, d11 = d1 * d1, d01 = d0 * d1;
-    const float g0r = F.g0[0] * d0 + F.g0[1] * d1;
-    const float4* row = s4 + r * P1 * W;
-    float p0 = 0.f, p1 = 0.f, p2 = 0.f;
+    const float cx = cheb[pi], cy = cheb[kMaxP1 + pj];
+    if (++pj == P1) pj = 0, pi++;
+    float p[NT][3];
+    const char* row = buf + r * rowb;
+    auto pairs = [&](auto one) {
+      using V = decltype(one);
+      constexpr bool kPair = sizeof(V) == 8;
+      if constexpr (kPair)
+        for (int k = 0; k < NT; k++) p[k][0] = p[k][1] = p[k][2] = 0.f;
+      const RowT<DL, ON, V> R0(F[0], cx, cy), R1(F[NT - 1], cx, cy);
 #pragma unroll
-    for (int pk = 0; pk < (P1C > 0 ? P1C : P1); pk++) {
-      const float d2 = P1C > 0 ? dz[pk] : F.pz - chebf[2 * P1 + pk];
-      const float rinv = rsqrtf(fmaf(d2, d2, r01));
-      const float4 A = row[pk * W];
-      const float4 B = row[pk * W + 1];
-      if (DL) {
-        const float Cx = reinterpret_cast<const float*>(row + pk * W + 2)[0];
-        const float dmd = A.x * d00 + A.y * d11 + A.z * (d2 * d2) + A.w * d01 + B.x * (d0 * d2) + B.y * (d1 * d2);
-        const float mnd = B.z * d0 + B.w * d1 + Cx * d2;
-        const float g0d = fmaf(F.g0[2], d2, g0r);
-        const float ri2 = rinv * rinv;
-        const float kernel = (dmd - g0d * mnd) * (ri2 * ri2 * rinv);
-        p0 += d0 * kernel;
-        p1 += d1 * kernel;
-        p2 += d2 * kernel;
-      } else {
-        const float m0 = A.x - F.f0n0 * A.w;
-        const float m1 = A.y - F.f0n0 * B.x;
-        const float m2 = A.z - F.f0n0 * B.y;
-        const float temp = (m0 * d0 + m1 * d1 + m2 * d2) * (rinv * rinv * rinv);
-        p0 += m0 * rinv + temp * d0;
-        p1 += m1 * rinv + temp * d1;
-        p2 += m2 * rinv + temp * d2;
+      for (int q = kPair ? 0 : P1 / 2; q < (kPair ? P1 / 2 : P1 / 2 + 1); q++) {
+        const ulonglong2* v = reinterpret_cast<const ulonglong2*>(row + q * Rec<DL>::pair_b);
+        f2 w[kV + 1];
+#pragma unroll
+        for (int i = 0; i < kV / 2; i++) {
+          const ulonglong2 u = v[i];
+          w[2 * i] = u.x;
+          w[2 * i + 1] = u.y;
+        }
+        if (kV & 1) w[kV - 1] = reinterpret_cast<const f2*>(v)[kV - 1];
+        V m[kV], cz;
+#pragma unroll
+        for (int i = 0; i < kV; i++)
+          if constexpr (kPair) m[i] = w[i];
+          else m[i] = lo(w[i]);
+        if constexpr (kPair) cz = reinterpret_cast<const f2*>(cheb + 2 * kMaxP1)[q];
+        else cz = cheb[2 * kMaxP1 + 2 * q];
+        R0.add(m, cz, p[0]);
+        if (NT == 2) R1.add(m, cz, p[NT - 1]);
       }
+    };
+    pairs(f2());
+    if (P1 & 1) pairs(float());
+#pragma unroll
+    for (int k = 0; k < NT; k++)
+      if (act[k])
+        for (int c = 0; c < 3; c++) a[k][c] += (double)p[k][c];
+  }
+}
+
+constexpr int kTile = 64;             // sources of a tile
+constexpr int kPairF = 20;            // floats of two sources, interleaved value by value
+constexpr int kBufB = 5120;           // a warp's buffer: two runs of proxy rows, or a tile
+constexpr int kChebB = 3 * kMaxP1 * 4;
+// An off-surface warp's buffer also holds the FP64 tile of the targets that
+// use the regularized forms; their FP32 tile and the pair tile follow.
+constexpr int kNearB = 3 * kTile * 16, kTileB = kTile / 2 * kPairF * 4;
+
+// A far node for the lane's NT targets: its moments stream through the two
+// halves of the warp's buffer in runs of whole Chebyshev rows; the copy of the
+// next run overlaps the interactions of this one.
+template <bool DL, bool ON, int NT>
+__device__ __forceinline__ void far_node(const EvalTask& T, int nd, const Tgt2 (&F)[NT], const bool (&act)[NT],
+                                         const double (&cb)[3], char* buf, float* cheb, double (&a)[NT][3]) {
+  constexpr int kHalf = kBufB / 2;
+  const int lane = threadIdx.x & 31;
+  const int P1 = T.P1, rowb = ((P1 + 1) / 2) * Rec<DL>::pair_b, nr = kHalf / rowb, nrow_all = P1 * P1;
+  const char* src = reinterpret_cast<const char*>(T.momf) + (size_t)nd * nrow_all * rowb;
+  __syncwarp();
+  for (int i = lane; i < 3 * P1; i += 32) {
+    const int c = i / P1;
+    cheb[c * kMaxP1 + i - c * P1] = (float)(T.tcheb[(size_t)nd * 3 * P1 + i] - cb[c]);
+  }
+  const int nch = (nrow_all + nr - 1) / nr;
+  warp_copy_async(buf, src, min(nr, nrow_all) * rowb, lane);
+  for (int ch = 0; ch < nch; ch++) {
+    const int row0 = ch * nr, rows = min(nr, nrow_all - row0);
+    if (ch + 1 < nch) {
+      const int r1 = row0 + nr;
+      warp_copy_async(buf + ((ch + 1) & 1) * kHalf, src + (size_t)r1 * rowb, min(nr, nrow_all - r1) * rowb, lane);
+      copy_async_wait<1>();
+    } else {
+      copy_async_wait<0>();
+    }
+    __syncwarp();
+    const char* b = buf + (ch & 1) * kHalf;
+    switch (P1) {  // the treecode degrees in use: P = 5 (inner), 6 (h = 1/64), 10 (h = 1/256)
+      case 6: proxy_rows<DL, ON, NT, 6>(b, row0, rows, P1, cheb, F, act, a); break;
+      case 7: proxy_rows<DL, ON, NT, 7>(b, row0, rows, P1, cheb, F, act, a); break;
+      case 11: proxy_rows<DL, ON, NT, 11>(b, row0, rows, P1, cheb, F, act, a); break;
+      default: proxy_rows<DL, ON, NT, 0>(b, row0, rows, P1, cheb, F, act, a);
+    }
+    __syncwarp();
+  }
+}
+
+// A tile's sources, two interleaved; an odd last one is followed by a copy of
+// its position without area, normal or density. On-surface: (x, y, z), area x
+// normal, density (SL: area x density); off-surface (x, y, z), area, normal,
+// density.
+template <int KIND>
+__device__ __forceinline__ void stage_pairs(const EvalTask& T, int s0, int cnt, const double (&cb)[3], float* tile) {
+  constexpr bool kOn = KIND == K_SL_ON || KIND == K_DL_ON;
+  for (int i = threadIdx.x & 31; i < ((cnt + 1) & ~1); i += 32) {
+    const int s = s0 + min(i, cnt - 1);
+    float v[10];
+    v[0] = (float)(T.sx[s] - cb[0]);
+    v[1] = (float)(T.sy[s] - cb[1]);
+    v[2] = (float)(T.sz[s] - cb[2]);
+    for (int c = 3; c < 10; c++) v[c] = 0.f;
+    if (i < cnt) {
+      if (kOn) {
+        const double as = T.sa[s];
+        v[3] = (float)(as * T.snx[s]);
+        v[4] = (float)(as * T.sny[s]);
+        v[5] = (float)(as * T.snz[s]);
+        v[6] = KIND == K_SL_ON ? (float)(as * T.qx[s]) : T.fqx[s];
+        v[7] = KIND == K_SL_ON ? (float)(as * T.qy[s]) : T.fqy[s];
+        v[8] = KIND == K_SL_ON ? (float)(as * T.qz[s]) : T.fqz[s];
+      } else {
+        v[3] = T.fnx[s];
+        v[4] = T.fny[s];
+        v[5] = T.fnz[s];
+        v[6] = T.fqx[s];
+        v[7] = T.fqy[s];
+        v[8] = T.fqz[s];
+        v[9] = T.fa[s];
+      }
+    }
+    float* w = tile + (i >> 1) * kPairF + (i & 1);
+#pragma unroll
+    for (int c = 0; c < (kOn ? 9 : 10); c++) w[2 * c] = v[c];
+  }
+}
+
+// Two sources for the lane's NT targets.
+// On-surface (Call_Ds_SL_onSurf / Call_Ds_DL_onSurf, 2S/KITC.cpp:807-846,
+// 921-957): the smoothing factor from the table up to s = kPlainOnSurf32, the
+// singular kernel beyond; the warp looks tables up only where one of its pairs
+// needs them (lim: -1 for a target whose sums do not count).
+// Off-surface, targets beyond 8 delta: the singular kernel.
+template <int KIND, int NT>
+__device__ __forceinline__ void pairs_step(const float* q, const Tgt2 (&F)[NT], const float (&lim)[NT], f2 inv_d2,
+                                           const float4* tab, float (&p)[NT][3]) {
+  constexpr bool kOn = KIND == K_SL_ON || KIND == K_DL_ON, kSL = KIND == K_SL_ON || KIND == K_SL_OFF;
+  f2 w[10];
+  const ulonglong2* v = reinterpret_cast<const ulonglong2*>(q);
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    const ulonglong2 u = v[i];
+    w[2 * i] = u.x;
+    w[2 * i + 1] = u.y;
+  }
+  f2 dx[NT], dy[NT], dz[NT], r2[NT], sq[NT];
+  bool in = false;
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    dx[k] = vsub(dup<f2>(F[k].px), w[0]);
+    dy[k] = vsub(dup<f2>(F[k].py), w[1]);
+    dz[k] = vsub(dup<f2>(F[k].pz), w[2]);
+    r2[k] = vfma(dz[k], dz[k], vfma(dx[k], dx[k], vmul(dy[k], dy[k])));
+    if (kOn) {
+      sq[k] = vmul(r2[k], inv_d2);
+      in = in || lo(sq[k]) <= lim[k] || hi(sq[k]) <= lim[k];
+    }
+  }
+  if constexpr (kOn) in = __any_sync(0xffffffffu, in);
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    f2 H1, H2;
+    const f2 ri = vrsqrt(r2[k]), ri2 = vmul(ri, ri);
+    if (kSL) {
+      H1 = ri;
+      H2 = vmul(ri2, ri);
+    } else {
+      H2 = vmul(vmul(ri2, ri2), ri);
+    }
+    if constexpr (kOn) {
+      if (in) {
+        const float s0 = lo(sq[k]), s1 = hi(sq[k]);
+        const float t0 = fminf(s0, kPlainOnSurf32), t1 = fminf(s1, kPlainOnSurf32);
+        if (kSL) {
+          const float u0 = smooth_eval_f(tab, t0), u1 = smooth_eval_f(tab, t1);
+          H1 = pack2(s0 <= kPlainOnSurf32 ? u0 : lo(H1), s1 <= kPlainOnSurf32 ? u1 : hi(H1));
+          tab += 2 * kPieces32 * kRep32;
+        }
+        const float u0 = smooth_eval_f(tab, t0), u1 = smooth_eval_f(tab, t1);
+        H2 = pack2(s0 <= kPlainOnSurf32 ? u0 : lo(H2), s1 <= kPlainOnSurf32 ? u1 : hi(H2));
+        if (kSL) tab -= 2 * kPieces32 * kRep32;
+      }
+    }
+    if constexpr (kSL) {
+      const f2 nf = dup<f2>(F[k].m0);
+      const f2 fx = vfma(nf, w[3], w[6]), fy = vfma(nf, w[4], w[7]), fz = vfma(nf, w[5], w[8]);
+      const f2 fdd = vfma(fz, dz[k], vfma(fx, dx[k], vmul(fy, dy[k])));
+      f2 h2;
+      if (kOn) {
+        h2 = vmul(H2, fdd);
+      } else {
+        H1 = vmul(w[9], ri);
+        h2 = vmul(vmul(fdd, H1), ri2);
+      }
+      p[k][0] = sum(p[k][0], vfma(fx, H1, vmul(dx[k], h2)));
+      p[k][1] = sum(p[k][1], vfma(fy, H1, vmul(dy[k], h2)));
+      p[k][2] = sum(p[k][2], vfma(fz, H1, vmul(dz[k], h2)));
+    } else {
+      // a far target has no subtraction
+      const f2 gx = kOn ? vsub(w[6], dup<f2>(-F[k].m0)) : w[6], gy = kOn ? vsub(w[7], dup<f2>(-F[k].m1)) : w[7],
+               gz = kOn ? vsub(w[8], dup<f2>(-F[k].m2)) : w[8];
+      const f2 gdd = vfma(gz, dz[k], vfma(gx, dx[k], vmul(gy, dy[k])));
+      const f2 ndd = vfma(w[5], dz[k], vfma(w[3], dx[k], vmul(w[4], dy[k])));
+      f2 kernel = vmul(vmul(ndd, gdd), H2);
+      if (!kOn) kernel = vmul(kernel, w[9]);
+      p[k][0] = sum_mul(p[k][0], dx[k], kernel);
+      p[k][1] = sum_mul(p[k][1], dy[k], kernel);
+      p[k][2] = sum_mul(p[k][2], dz[k], kernel);
+    }
+  }
+}
+
+// A tile of cnt sources for NT targets, FP32 sums of 16 sources added in FP64.
+template <int KIND, int NT>
+__device__ __forceinline__ void tile_pairs(const float* tile, int cnt, const Tgt2 (&F)[NT], const bool (&act)[NT],
+                                           f2 inv_d2, const float4* tab, double (&a)[NT][3]) {
+  constexpr bool kDL = KIND == K_DL_ON || KIND == K_DL_OFF;
+  float lim[NT];
+  for (int k = 0; k < NT; k++) lim[k] = act[k] ? kPlainOnSurf32 : -1.0f;
+  const int np = (cnt + 1) >> 1;
+  for (int j0 = 0; j0 < np; j0 += 8) {
+    float p[NT][3];
+    for (int k = 0; k < NT; k++) p[k][0] = p[k][1] = p[k][2] = 0.f;
+    const int j1 = min(np, j0 + 8);
+#pragma unroll(kDL ? 2 : 1)
+    for (int j = j0; j < j1; j++) pairs_step<KIND, NT>(tile + j * kPairF, F, lim, inv_d2, tab, p);
+#pragma unroll
+    for (int k = 0; k < NT; k++)
+      if (act[k])
+        for (int c = 0; c < 3; c++) a[k][c] += (double)p[k][c];
+  }
+}
+
+// The pairs of one target per lane that uses the regularized forms: FP64 for
+// r <= 3 delta (all-FP32 mode: only the r < 1e-14 limits), FP32 beyond.
+template <int KIND>
+__device__ __noinline__ double3 tile_near(const EvalTask& T, int t, bool act, int cnt, double3 org,
+                                          const double* wsm, const float4* ws4, double3 a) {
+  if (!act) return a;
+  const double cb[3] = {org.x, org.y, org.z};
+  Tgt S;
+  Tgt32 F;
+  load_target<KIND>(T, t, true, cb, S, F);
+  const Reg g = make_reg(T.DEL);
+  RegF gf;
+  gf.inv_d = (float)g.inv_d;
+  gf.d64 = (float)g.d64;
+  gf.inv_d2 = (float)g.inv_d2;
+  gf.inv_d3 = (float)g.inv_d3;
+  gf.inv_d5 = (float)g.inv_d5;
+  const float cut2f = T.mixed == 2 ? 1e-28f : (float)(9.0 * T.DEL * T.DEL);
+  double a0 = a.x, a1 = a.y, a2 = a.z;
+  for (int j0 = 0; j0 < cnt; j0 += 16) {
+    float p0 = 0.f, p1 = 0.f, p2 = 0.f;
+    const int j1 = min(cnt, j0 + 16);
+    for (int j = j0; j < j1; j++) {
+      const float4 Pj = ws4[j];
+      const float dx = F.px - Pj.x, dy = F.py - Pj.y, dz = F.pz - Pj.z;
+      if (dx * dx + dy * dy + dz * dz > cut2f) pair32r<KIND>(ws4, j, F, gf, p0, p1, p2);
+      else pair64<KIND>(wsm, j, S, g, a0, a1, a2);
     }
     a0 += (double)p0;
     a1 += (double)p1;
     a2 += (double)p2;
   }
+  return make_double3(a0, a1, a2);
 }
 
-template <bool DL>
-__device__ __forceinline__ void proxies32_any(const float4* __restrict__ s4, int row0, int nrows, int P1,
-                                              const float* __restrict__ chebf, const Tgt32& F, double& a0,
-                                              double& a1, double& a2) {
-  switch (P1) {  // the treecode degrees in use: P = 5 (inner), 6 (h = 1/64), 10 (h = 1/256)
-    case 6: proxies32_rows<DL, 6>(s4, row0, nrows, P1, chebf, F, a0, a1, a2); break;
-    case 7: proxies32_rows<DL, 7>(s4, row0, nrows, P1, chebf, F, a0, a1, a2); break;
-    case 11: proxies32_rows<DL, 11>(s4, row0, nrows, P1, chebf, F, a0, a1, a2); break;
-    default: proxies32_rows<DL, 0>(s4, row0, nrows, P1, chebf, F, a0, a1, a2);
+// The FP64 and FP32 tiles of tile_near.
+__device__ __forceinline__ void stage_near(const EvalTask& T, int s0, int cnt, const double (&cb)[3], double* wsm,
+                                           float4* ws4) {
+  for (int i = threadIdx.x & 31; i < cnt; i += 32) {
+    const int s = s0 + i;
+    const double x = T.sx[s], y = T.sy[s], z = T.sz[s];
+    double2* w2 = reinterpret_cast<double2*>(wsm) + 5 * i;
+    w2[0] = make_double2(x, y);
+    w2[1] = make_double2(z, T.sa[s]);
+    w2[2] = make_double2(T.snx[s], T.sny[s]);
+    w2[3] = make_double2(T.snz[s], T.qx[s]);
+    w2[4] = make_double2(T.qy[s], T.qz[s]);
+    ws4[i] = make_float4((float)(x - cb[0]), (float)(y - cb[1]), (float)(z - cb[2]), T.fa[s]);
+    ws4[kNT + i] = make_float4(T.fnx[s], T.fny[s], T.fnz[s], 0.f);
+    ws4[2 * kNT + i] = make_float4(T.fqx[s], T.fqy[s], T.fqz[s], 0.f);
   }
 }
 
-// One item of an off-surface or extend-to-grid task.
+// A near segment [s0, s0 + n) for NT targets; near: which of them use the
+// regularized forms (off-surface kinds).
+template <int KIND, int NT>
+__device__ __forceinline__ void near_segment(const EvalTask& T, int s0, int n, const Tgt2 (&F)[NT],
+                                             const int (&t)[NT], const bool (&act)[NT], const bool (&near)[NT],
+                                             const double (&cb)[3], f2 inv_d2, const float4* tab, char* buf,
+                                             double (&a)[NT][3]) {
+  constexpr bool kOn = KIND == K_SL_ON || KIND == K_DL_ON;
+  bool far[NT], any_far = kOn, any_near = false;
+  for (int k = 0; k < NT; k++) {
+    far[k] = act[k] && (kOn || !near[k]);
+    if (!kOn) {
+      any_far = any_far || __any_sync(0xffffffffu, far[k]);
+      any_near = any_near || __any_sync(0xffffffffu, act[k] && near[k]);
+    }
+  }
+  float* tile = reinterpret_cast<float*>(buf + (kOn ? 0 : kBufB + kNearB));
+  double* wsm = reinterpret_cast<double*>(buf);
+  float4* ws4 = reinterpret_cast<float4*>(buf + kBufB);
+  for (int b = 0; b < n; b += kTile) {
+    const int cnt = min(kTile, n - b);
+    __syncwarp();
+    if (any_far) stage_pairs<KIND>(T, s0 + b, cnt, cb, tile);
+    if constexpr (!kOn)
+      if (any_near) stage_near(T, s0 + b, cnt, cb, wsm, ws4);
+    __syncwarp();
+    if (any_far) tile_pairs<KIND, NT>(tile, cnt, F, far, inv_d2, tab, a);
+    if constexpr (!kOn) {
+#pragma unroll
+      for (int k = 0; k < NT; k++)
+        if (__any_sync(0xffffffffu, act[k] && near[k])) {
+          const double3 v = tile_near<KIND>(T, t[k], act[k] && near[k], cnt, make_double3(cb[0], cb[1], cb[2]), wsm, ws4,
+                                            make_double3(a[k][0], a[k][1], a[k][2]));
+          a[k][0] = v.x;
+          a[k][1] = v.y;
+          a[k][2] = v.z;
+        }
+    }
+  }
+  __syncwarp();
+}
+
+// One unit: half h (64 targets, two per lane: lane and lane + 32) of an item's
+// target block, all its segments in order.
+template <int KIND>
+__device__ __forceinline__ void run_unit(const EvalTask& T, const BlockRef& it, int h, const Seg* __restrict__ segs,
+                                         const float4* tab, char* buf, float* cheb) {
+  constexpr bool kOn = KIND == K_SL_ON || KIND == K_DL_ON, DL = KIND == K_DL_ON || KIND == K_DL_OFF;
+  const int lane = threadIdx.x & 31;
+  const int k0 = it.blk * kTB + h * 64 + lane;
+  const bool valid[2] = {k0 < T.nt, k0 + 32 < T.nt};
+  if (!__any_sync(0xffffffffu, valid[0])) return;  // the block's tail: no slot of these targets is read
+  // origin of the FP32 coordinates: the block's first target (the sources a
+  // block meets lie within a few leaf sizes of it, so FP32 offsets stay small)
+  double cb[3];
+  {
+    const int t0 = T.tord[it.blk * kTB];
+    cb[0] = T.txyz[3 * t0];
+    cb[1] = T.txyz[3 * t0 + 1];
+    cb[2] = T.txyz[3 * t0 + 2];
+  }
+  Tgt2 F[2];
+  int t[2];
+  bool near[2];
+  double a[2][3];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    t[k] = valid[k] ? T.tord[k0 + 32 * k] : 0;
+    Tgt S;
+    Tgt32 f;
+    load_target<KIND>(T, t[k], valid[k], cb, S, f);
+    near[k] = !kOn && S.near != 0;
+    F[k] = {f.px, f.py, f.pz, DL ? -f.g0[0] : -f.f0n0, DL ? -f.g0[1] : 0.f, DL ? -f.g0[2] : 0.f};
+    for (int c = 0; c < 3; c++) a[k][c] = 0.0;
+  }
+  const f2 inv_d2 = dup<f2>((float)make_reg(T.DEL).inv_d2);
+  for (int base = it.seg0; base < it.seg1; base += 32) {
+    // 32 segments at a time, one per lane; those without a target of this half drop out
+    const int q = base + lane;
+    Seg sg{0, 0, 0};
+    int node = 0, type = 0;
+    uint32_t w0 = 0, w1 = 0;
+    if (q < it.seg1) {
+      sg = segs[q];
+      const Entry* E = T.entries + sg.entry;
+      node = E->node;
+      type = E->type;
+      w0 = E->mask[2 * h];
+      w1 = E->mask[2 * h + 1];
+    }
+    unsigned live = __ballot_sync(0xffffffffu, (w0 | w1) != 0u);
+    while (live) {
+      const int l = __ffs(live) - 1;
+      live &= live - 1;
+      const uint32_t m0 = __shfl_sync(0xffffffffu, w0, l), m1 = __shfl_sync(0xffffffffu, w1, l);
+      const int ty = __shfl_sync(0xffffffffu, type, l), nd = __shfl_sync(0xffffffffu, node, l);
+      const int s0 = __shfl_sync(0xffffffffu, sg.s0, l), n = __shfl_sync(0xffffffffu, sg.s1, l) - s0;
+      const bool act[2] = {valid[0] && ((m0 >> lane) & 1u), valid[1] && ((m1 >> lane) & 1u)};
+      if (m0 != 0u && m1 != 0u) {
+        if (ty == 1) {
+          near_segment<KIND, 2>(T, s0, n, F, t, act, near, cb, inv_d2, tab, buf, a);
+        } else if (kOn) {  // a node's rows are summed by themselves
+          double p[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+          far_node<DL, kOn, 2>(T, nd, F, act, cb, buf, cheb, p);
+          for (int k = 0; k < 2; k++)
+            if (act[k])
+              for (int c = 0; c < 3; c++) a[k][c] += p[k][c];
+        } else {
+          far_node<DL, kOn, 2>(T, nd, F, act, cb, buf, cheb, a);
+        }
+      } else {  // one target per lane
+        const int k = m0 != 0u ? 0 : 1;
+        const Tgt2 F1[1] = {k == 0 ? F[0] : F[1]};
+        const int t1[1] = {k == 0 ? t[0] : t[1]};
+        const bool act1[1] = {k == 0 ? act[0] : act[1]}, near1[1] = {k == 0 ? near[0] : near[1]};
+        double a1[1][3], p1[1][3] = {{0.0, 0.0, 0.0}};
+        for (int c = 0; c < 3; c++) a1[0][c] = k == 0 ? a[0][c] : a[1][c];
+        if (ty == 1) {
+          near_segment<KIND, 1>(T, s0, n, F1, t1, act1, near1, cb, inv_d2, tab, buf, a1);
+        } else if (kOn) {
+          far_node<DL, kOn, 1>(T, nd, F1, act1, cb, buf, cheb, p1);
+          if (act1[0])
+            for (int c = 0; c < 3; c++) a1[0][c] += p1[0][c];
+        } else {
+          far_node<DL, kOn, 1>(T, nd, F1, act1, cb, buf, cheb, a1);
+        }
+        for (int c = 0; c < 3; c++) {
+          a[0][c] = k == 0 ? a1[0][c] : a[0][c];
+          a[1][c] = k == 1 ? a1[0][c] : a[1][c];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    double2* o = reinterpret_cast<double2*>(T.partial + ((size_t)it.slot * kTB + h * 64 + 32 * k + lane) * kPartComps);
+    o[0] = make_double2(a[k][0], a[k][1]);
+    o[1] = make_double2(a[k][2], 0.0);
+  }
+}
+
+template <int KIND>
+struct Shape32 {
+  static constexpr bool on = KIND == K_SL_ON || KIND == K_DL_ON;
+  static constexpr int warps = 12;
+  static constexpr int warp_b = kBufB + (on ? 0 : kNearB + kTileB) + kChebB;
+  static constexpr int tab_b = !on ? 0 : (KIND == K_SL_ON ? 2 : 1) * 2 * kPieces32 * kRep32 * 16;
+  static constexpr int smem = tab_b + warps * warp_b;
+};
+
+// A launch's items, one persistent CTA per SM: every warp takes units from a
+// common counter (the first by position, the rest in the items' order of
+// decreasing cost); a unit's sums go to its own slot.
+template <int KIND>
+__global__ void __launch_bounds__(Shape32<KIND>::warps * 32, 1)
+    units_kernel(const EvalTask* __restrict__ tasks, const BlockRef* __restrict__ items,
+                 const Seg* __restrict__ segs, unsigned nunits, unsigned* __restrict__ next) {
+  using SH = Shape32<KIND>;
+  extern __shared__ __align__(16) char smc[];
+  float4* tab = reinterpret_cast<float4*>(smc);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  char* buf = smc + SH::tab_b + warp * SH::warp_b;
+  float* cheb = reinterpret_cast<float*>(buf + SH::warp_b - kChebB);
+  if constexpr (SH::on) {
+    // the tables with the powers of 1/delta in the coefficients, eight copies
+    // (all tasks of a batch share one delta)
+    const Reg gs = make_reg(tasks[items[0].task].DEL);
+    float* t32 = reinterpret_cast<float*>(tab);
+    for (int i = threadIdx.x; i < kPieces32 * 8; i += blockDim.x) {
+      const bool centre = (i & 7) == 0;
+      for (int c = 0; c < kRep32; c++) {
+        float* o = t32 + ((i >> 2) * kRep32 + c) * 4 + (i & 3);
+        if (KIND == K_SL_ON) {
+          o[0] = kSmooth32G1[i] * (centre ? 1.0f : (float)gs.inv_d);
+          o[2 * kPieces32 * kRep32 * 4] = kSmooth32G2[i] * (centre ? 1.0f : (float)gs.inv_d3);
+        } else {
+          o[0] = kSmooth32G3[i] * (centre ? 1.0f : (float)gs.inv_d5);
+        }
+      }
+    }
+    __syncthreads();
+    tab += lane & (kRep32 - 1);
+  }
+  for (unsigned u = warp * gridDim.x + blockIdx.x; u < nunits;) {
+    unsigned nx = 0;
+    if (lane == 0) nx = atomicAdd(next, 1u);  // returns while the unit runs
+    const BlockRef it = items[u >> 1];
+    run_unit<KIND>(tasks[it.task], it, u & 1, segs, tab, buf, cheb);
+    u = __shfl_sync(0xffffffffu, nx, 0) + gridDim.x * SH::warps;
+  }
+}
+
+template <int KIND>
+void launch_units(const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems, unsigned* next,
+                  int num_sms, cudaStream_t st) {
+  if (nitems <= 0) return;
+  static_assert(Shape32<KIND>::smem <= 227 * 1024, "the table and the buffers fit one CTA");
+  // set on every launch: the attribute belongs to the current device's context
+  cudaFuncSetAttribute(units_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape32<KIND>::smem);
+  const unsigned nunits = 2u * (unsigned)nitems;
+  const unsigned grid = nunits < (unsigned)num_sms ? nunits : (unsigned)num_sms;
+  units_kernel<KIND><<<grid, Shape32<KIND>::warps * 32, Shape32<KIND>::smem, st>>>(d_tasks, d_items, d_segs, nunits, next);
+}
+
+// ------------------------------------------------- extend-to-grid sums
+
+// One item of an extend-to-grid task.
 template <int KIND>
 __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, const Seg* __restrict__ segs,
-                                         double* sm, float4* s4, float* chebf) {
+                                         double* sm, float4* s4) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blk = it.blk;
   const int k = blk * kTB + tid;
@@ -578,15 +1063,13 @@ __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, 
   // only the r < 1e-14 limits of the reference stay in FP64
   const float cut2f = T.mixed == 2 ? 1e-28f : (float)(9.0 * T.DEL * T.DEL);
   double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;  // a3: the pressure of the extend-to-grid sums
-  constexpr bool kFace = KIND == K_E2G_UP_AWAY, kBand = KIND == K_E2G_UP7;
+  constexpr bool kFace = KIND == K_E2G_UP_AWAY;
   constexpr bool kSrcNrm = !kFace;
-  const bool all32 = kFace || ((KIND == K_SL_OFF || KIND == K_DL_OFF) && !S.near);
   // Each warp walks the item's segments on its own: its own source tiles in
   // shared memory, __syncwarp only, and an entry whose mask is zero for this
   // warp is skipped outright.
   double* wsm = sm + warp * kWarpSm;
   float4* ws4 = s4 + warp * 3 * kNT;
-  float* wchebf = chebf + warp * 3 * kMaxP1;
   for (int q = it.seg0; q < it.seg1; q++) {
     const Seg sg = segs[q];
     const Entry E = T.entries[sg.entry];
@@ -628,7 +1111,7 @@ __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, 
             a2 += (double)p2;
             a3 += (double)p3;
           }
-        } else if constexpr (kBand) {
+        } else {
           for (int j0 = 0; j0 < cnt; j0 += 16) {
             float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
             const int j1 = min(cnt, j0 + 16);
@@ -644,69 +1127,7 @@ __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, 
             a2 += (double)p2;
             a3 += (double)p3;
           }
-        } else if (all32) {
-          for (int j0 = 0; j0 < cnt; j0 += 16) {
-            float p0 = 0.f, p1 = 0.f, p2 = 0.f;
-            const int j1 = min(cnt, j0 + 16);
-            if (j1 - j0 == 16) {  // a full run: a compile-time trip count
-#pragma unroll 4
-              for (int j = j0; j < j0 + 16; j++) pair32<KIND>(ws4, j, F, p0, p1, p2);
-            } else {
-              for (int j = j0; j < j1; j++) pair32<KIND>(ws4, j, F, p0, p1, p2);
-            }
-            a0 += (double)p0;
-            a1 += (double)p1;
-            a2 += (double)p2;
-          }
-        } else {
-          for (int j0 = 0; j0 < cnt; j0 += 16) {
-            float p0 = 0.f, p1 = 0.f, p2 = 0.f;
-            const int j1 = min(cnt, j0 + 16);
-            for (int j = j0; j < j1; j++) {
-              const float4 Pj = ws4[j];
-              const float dx = F.px - Pj.x, dy = F.py - Pj.y, dz = F.pz - Pj.z;
-              if (dx * dx + dy * dy + dz * dz > cut2f) pair32r<KIND>(ws4, j, F, gf, p0, p1, p2);
-              else pair64<KIND>(wsm, j, S, g, a0, a1, a2);
-            }
-            a0 += (double)p0;
-            a1 += (double)p1;
-            a2 += (double)p2;
-          }
         }
-      }
-    } else if constexpr (!kFace && !kBand) {
-      constexpr bool DL = KIND == K_DL_OFF;
-      const int P1 = T.P1, Pf = T.Pf;
-      // The node's proxy-major moments stream through the warp's tile in
-      // runs of whole Chebyshev rows, double-buffered: the asynchronous copy
-      // of the next run overlaps the interactions of this one.
-      constexpr int kBpp = DL ? 48 : 32;  // bytes per proxy
-      constexpr int kHalf = kWarpSm * 4;  // bytes per buffer
-      const char* src = reinterpret_cast<const char*>(T.momf + (size_t)E.node * Pf * (DL ? 12 : 8));
-      char* buf = reinterpret_cast<char*>(wsm);
-      const int rowb = P1 * kBpp;
-      const int nr = max(1, kHalf / rowb);
-      const int nrow_all = P1 * P1;
-      const int nch = (nrow_all + nr - 1) / nr;
-      __syncwarp();
-      for (int i = lane; i < 3 * P1; i += 32)
-        wchebf[i] = (float)(T.tcheb[(size_t)E.node * 3 * P1 + i] - cb[i / P1]);
-      warp_copy_async(buf, src, min(nr, nrow_all) * rowb, lane);
-      for (int ch = 0; ch < nch; ch++) {
-        const int row0 = ch * nr, rows = min(nr, nrow_all - row0);
-        if (ch + 1 < nch) {
-          const int r1 = row0 + nr;
-          warp_copy_async(buf + ((ch + 1) & 1) * kHalf, src + (size_t)r1 * rowb, min(nr, nrow_all - r1) * rowb,
-                          lane);
-          copy_async_wait<1>();
-        } else {
-          copy_async_wait<0>();
-        }
-        __syncwarp();
-        if (act)
-          proxies32_any<DL>(reinterpret_cast<const float4*>(buf + (ch & 1) * kHalf), row0, rows, P1, wchebf, F, a0,
-                            a1, a2);
-        __syncwarp();
       }
     }
   }
@@ -718,274 +1139,21 @@ __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, 
   o[3] = a3;
 }
 
-// ------------------------------------- two targets per thread (mixed, on-surface)
-
-// FP32 proxies of a run of Chebyshev rows for two targets: each shared-memory
-// read of a proxy serves both. Sums per row go to acc (FP64). P1C as in
-// proxies32_rows.
-template <bool DL, int P1C>
-__device__ __forceinline__ void proxies32_rows2(const float4* __restrict__ s4, int row0, int nrows, int P1rt,
-                                                const float* __restrict__ chebf, const Tgt32 (&F)[2],
-                                                double (&acc)[2][3]) {
-  constexpr int W = DL ? 3 : 2;  // float4 per proxy
-  const int P1 = P1C > 0 ? P1C : P1rt;
-  float czr[P1C > 0 ? P1C : 1];
-  if constexpr (P1C > 0) {
-#pragma unroll
-    for (int pk = 0; pk < P1C; pk++) czr[pk] = chebf[2 * P1C + pk];
-  }
-  for (int r = 0; r < nrows; r++) {
-    const int pi = (row0 + r) / P1, pj = (row0 + r) - pi * P1;
-    const float cx = chebf[pi], cy = chebf[P1 + pj];
-    float d0[2], d1[2], r01[2], d00[2], d11[2], d01[2], g0r[2];
-    float p[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      d0[q] = F[q].px - cx;
-      d1[q] = F[q].py - cy;
-      r01[q] = d0[q] * d0[q] + d1[q] * d1[q];
-      d00[q] = d0[q] * d0[q];
-      d11[q] = d1[q] * d1[q];
-      d01[q] = d0[q] * d1[q];
-      g0r[q] = F[q].g0[0] * d0[q] + F[q].g0[1] * d1[q];
-    }
-    const float4* row = s4 + r * P1 * W;
-#pragma unroll
-    for (int pk = 0; pk < (P1C > 0 ? P1C : P1); pk++) {
-      const float cz = P1C > 0 ? czr[pk] : chebf[2 * P1 + pk];
-      const float4 A = row[pk * W];
-      const float4 B = row[pk * W + 1];
-      const float Cx = DL ? reinterpret_cast<const float*>(row + pk * W + 2)[0] : 0.f;
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const float d2 = F[q].pz - cz;
-        const float rinv = rsqrtf(fmaf(d2, d2, r01[q]));
-        if (DL) {
-          const float dmd = A.x * d00[q] + A.y * d11[q] + A.z * (d2 * d2) + A.w * d01[q] + B.x * (d0[q] * d2) +
-                            B.y * (d1[q] * d2);
-          const float mnd = B.z * d0[q] + B.w * d1[q] + Cx * d2;
-          const float g0d = fmaf(F[q].g0[2], d2, g0r[q]);
-          const float ri2 = rinv * rinv;
-          const float kernel = (dmd - g0d * mnd) * (ri2 * ri2 * rinv);
-          p[q][0] += d0[q] * kernel;
-          p[q][1] += d1[q] * kernel;
-          p[q][2] += d2 * kernel;
-        } else {
-          const float m0 = A.x - F[q].f0n0 * A.w;
-          const float m1 = A.y - F[q].f0n0 * B.x;
-          const float m2 = A.z - F[q].f0n0 * B.y;
-          const float temp = (m0 * d0[q] + m1 * d1[q] + m2 * d2) * (rinv * rinv * rinv);
-          p[q][0] += m0 * rinv + temp * d0[q];
-          p[q][1] += m1 * rinv + temp * d1[q];
-          p[q][2] += m2 * rinv + temp * d2;
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-      for (int c = 0; c < 3; c++) acc[q][c] += (double)p[q][c];
-  }
-}
-
-template <bool DL>
-__device__ __forceinline__ void proxies32_any2(const float4* __restrict__ s4, int row0, int nrows, int P1,
-                                               const float* __restrict__ chebf, const Tgt32 (&F)[2],
-                                               double (&acc)[2][3]) {
-  switch (P1) {  // the treecode degrees in use: P = 5 (inner), 6 (h = 1/64), 10 (h = 1/256)
-    case 6: proxies32_rows2<DL, 6>(s4, row0, nrows, P1, chebf, F, acc); break;
-    case 7: proxies32_rows2<DL, 7>(s4, row0, nrows, P1, chebf, F, acc); break;
-    case 11: proxies32_rows2<DL, 11>(s4, row0, nrows, P1, chebf, F, acc); break;
-    default: proxies32_rows2<DL, 0>(s4, row0, nrows, P1, chebf, F, acc);
-  }
-}
-
-// The reduced-precision on-surface items (K_SL_ON / K_DL_ON, every pair in
-// FP32 with the tabulated smoothing factors) with two targets per thread: a
-// CTA of kTB2 = 64 threads covers the block's 128 targets — warp w holds
-// targets 64 w + lane and 64 w + 32 + lane, i.e. mask words 2 w and 2 w + 1 —
-// so every source and proxy read from shared memory serves two pairs.
-constexpr int kTB2 = 64;
-template <int KIND>
-__device__ __forceinline__ void run_item_on2(const EvalTask& T, const BlockRef& it, const Seg* __restrict__ segs,
-                                             double* sm, float4* s4, float* chebf, const float4* stab32) {
-  constexpr bool DL = (KIND == K_DL_ON);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int blk = it.blk;
-  double cb[3];
-  {
-    const int t0 = T.tord[blk * kTB];
-    cb[0] = T.txyz[3 * t0];
-    cb[1] = T.txyz[3 * t0 + 1];
-    cb[2] = T.txyz[3 * t0 + 2];
-  }
-  Tgt32 F[2];
-  bool valid[2];
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const int k = blk * kTB + warp * 64 + q * 32 + lane;
-    valid[q] = k < T.nt;
-    Tgt S;
-    load_target<KIND>(T, valid[q] ? T.tord[k] : 0, valid[q], cb, S, F[q]);
-  }
-  const Reg g = make_reg(T.DEL);
-  RegF gf;
-  gf.inv_d = (float)g.inv_d;
-  gf.d64 = (float)g.d64;
-  gf.inv_d2 = (float)g.inv_d2;
-  gf.inv_d3 = (float)g.inv_d3;
-  gf.inv_d5 = (float)g.inv_d5;
-  double a[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-  double* wsm = sm + warp * kWarpSm;
-  float4* ws4 = s4 + warp * 3 * kNT;
-  float* wchebf = chebf + warp * 3 * kMaxP1;
-  for (int qs = it.seg0; qs < it.seg1; qs++) {
-    const Seg sg = segs[qs];
-    const Entry E = T.entries[sg.entry];
-    const uint32_t mA = E.mask[2 * warp], mB = E.mask[2 * warp + 1];
-    if ((mA | mB) == 0u) continue;
-    const bool actA = valid[0] && ((mA >> lane) & 1u);
-    const bool actB = valid[1] && ((mB >> lane) & 1u);
-    if (E.type == 1) {
-      const int m0 = sg.s0, m1 = sg.s1 - 1;
-      for (int s0 = m0; s0 <= m1; s0 += kNT) {
-        const int cnt = min(kNT, m1 - s0 + 1);
-        __syncwarp();
-        for (int i = lane; i < cnt; i += 32) {
-          const int s = s0 + i;
-          const double as = T.sa[s];
-          ws4[i] = make_float4((float)(T.sx[s] - cb[0]), (float)(T.sy[s] - cb[1]), (float)(T.sz[s] - cb[2]),
-                               (float)as);
-          ws4[kNT + i] = make_float4((float)(as * T.snx[s]), (float)(as * T.sny[s]), (float)(as * T.snz[s]), 0.f);
-          if (KIND == K_SL_ON)
-            ws4[2 * kNT + i] = make_float4((float)(as * T.qx[s]), (float)(as * T.qy[s]), (float)(as * T.qz[s]), 0.f);
-          else
-            ws4[2 * kNT + i] = make_float4(T.fqx[s], T.fqy[s], T.fqz[s], 0.f);
-        }
-        __syncwarp();
-        if (!actA && !actB) continue;
-        for (int j0 = 0; j0 < cnt; j0 += 16) {
-          float pA[3] = {0.f, 0.f, 0.f}, pB[3] = {0.f, 0.f, 0.f};
-          const int j1 = min(cnt, j0 + 16);
-          if (j1 - j0 == 16) {  // a full run: a compile-time trip count
-#pragma unroll 4
-            for (int j = j0; j < j0 + 16; j++) {
-              const float4 P = ws4[j], N = ws4[kNT + j], Q = ws4[2 * kNT + j];
-              pair32tab_src<KIND>(P, N, Q, F[0], gf, stab32, pA[0], pA[1], pA[2]);
-              pair32tab_src<KIND>(P, N, Q, F[1], gf, stab32, pB[0], pB[1], pB[2]);
-            }
-          } else {
-#pragma unroll 2
-            for (int j = j0; j < j1; j++) {
-              const float4 P = ws4[j], N = ws4[kNT + j], Q = ws4[2 * kNT + j];
-              pair32tab_src<KIND>(P, N, Q, F[0], gf, stab32, pA[0], pA[1], pA[2]);
-              pair32tab_src<KIND>(P, N, Q, F[1], gf, stab32, pB[0], pB[1], pB[2]);
-            }
-          }
-          if (actA)
-            for (int c = 0; c < 3; c++) a[0][c] += (double)pA[c];
-          if (actB)
-            for (int c = 0; c < 3; c++) a[1][c] += (double)pB[c];
-        }
-      }
-    } else {
-      // far node: the proxy-major FP32 moments through the warp's tile, double-buffered
-      const int P1 = T.P1, Pf = T.Pf;
-      constexpr int kBpp = DL ? 48 : 32;  // bytes per proxy
-      constexpr int kHalf = kWarpSm * 4;  // bytes per buffer
-      const char* src = reinterpret_cast<const char*>(T.momf + (size_t)E.node * Pf * (DL ? 12 : 8));
-      char* buf = reinterpret_cast<char*>(wsm);
-      const int rowb = P1 * kBpp;
-      const int nr = max(1, kHalf / rowb);
-      const int nrow_all = P1 * P1;
-      const int nch = (nrow_all + nr - 1) / nr;
-      __syncwarp();
-      for (int i = lane; i < 3 * P1; i += 32)
-        wchebf[i] = (float)(T.tcheb[(size_t)E.node * 3 * P1 + i] - cb[i / P1]);
-      warp_copy_async(buf, src, min(nr, nrow_all) * rowb, lane);
-      double acc[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-      for (int ch = 0; ch < nch; ch++) {
-        const int row0 = ch * nr, rows = min(nr, nrow_all - row0);
-        if (ch + 1 < nch) {
-          const int r1 = row0 + nr;
-          warp_copy_async(buf + ((ch + 1) & 1) * kHalf, src + (size_t)r1 * rowb, min(nr, nrow_all - r1) * rowb,
-                          lane);
-          copy_async_wait<1>();
-        } else {
-          copy_async_wait<0>();
-        }
-        __syncwarp();
-        if (actA || actB)
-          proxies32_any2<DL>(reinterpret_cast<const float4*>(buf + (ch & 1) * kHalf), row0, rows, P1, wchebf, F,
-                              acc);
-        __syncwarp();
-      }
-      if (actA)
-        for (int c = 0; c < 3; c++) a[0][c] += acc[0][c];
-      if (actB)
-        for (int c = 0; c < 3; c++) a[1][c] += acc[1][c];
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    double* o = T.partial + ((size_t)it.slot * kTB + warp * 64 + q * 32 + lane) * kPartComps;
-    o[0] = a[q][0];
-    o[1] = a[q][1];
-    o[2] = a[q][2];
-    o[3] = 0.0;
-  }
-}
-
-template <int FAM>
-__global__ void __launch_bounds__(kTB2, 8) eval_kernel_on2(const EvalTask* __restrict__ tasks,
-                                                           const BlockRef* __restrict__ items,
-                                                           const Seg* __restrict__ segs) {
-  constexpr int kW2 = kTB2 / 32;
-  __shared__ __align__(16) double sm[kW2 * kWarpSm];
-  __shared__ float4 sf[kW2 * 3 * kNT];
-  __shared__ float chebf[kW2 * 3 * kMaxP1];
-  __shared__ EvalTask sT;
-  __shared__ float4 stab32[FAM == F_SL ? 2 * kSmooth32N / 4 : kSmooth32N / 4];
-  const BlockRef it = items[blockIdx.x];
-  if (threadIdx.x == 0) sT = tasks[it.task];
-  {
-    // FP32 tables with the powers of 1/delta in the coefficients (as in eval_kernel)
-    const Reg gs = make_reg(tasks[it.task].DEL);
-    float* t32 = reinterpret_cast<float*>(stab32);
-    for (int i = threadIdx.x; i < kSmooth32N; i += blockDim.x) {
-      const bool centre = (i & 7) == 0;
-      if (FAM == F_SL) {
-        t32[i] = kSmooth32G1[i] * (centre ? 1.0f : (float)gs.inv_d);
-        t32[kSmooth32N + i] = kSmooth32G2[i] * (centre ? 1.0f : (float)gs.inv_d3);
-      } else {
-        t32[i] = kSmooth32G3[i] * (centre ? 1.0f : (float)gs.inv_d5);
-      }
-    }
-  }
-  __syncthreads();
-  if (FAM == F_SL) run_item_on2<K_SL_ON>(sT, it, segs, sm, sf, chebf, stab32);
-  else run_item_on2<K_DL_ON>(sT, it, segs, sm, sf, chebf, stab32);
-}
-
-// The batch's other items: off-surface tasks, or one of the extend-to-grid
-// passes. ON = true: the box-face sums, whose code path needs fewer registers
-// (no nearest-point data, no per-target coefficients), six CTAs per SM; the
-// others four.
-template <int FAM, bool ON>
-__global__ void __launch_bounds__(kTB, ON ? 6 : 4)
-    eval_kernel(const EvalTask* __restrict__ tasks, const BlockRef* __restrict__ items,
-                const Seg* __restrict__ segs) {
+// The extend-to-grid items, a CTA each. FACE: the box-face sums, whose code
+// path needs fewer registers (no nearest-point data, no per-target
+// coefficients), six CTAs per SM; the band's four.
+template <bool FACE>
+__global__ void __launch_bounds__(kTB, FACE ? 6 : 4)
+    eval_kernel_e2g(const EvalTask* __restrict__ tasks, const BlockRef* __restrict__ items,
+                    const Seg* __restrict__ segs) {
   __shared__ __align__(16) double sm[kSmem];
   // per-warp FP32 source tiles: (x, y, z, area), (n, 0), (q, 0) per source
   __shared__ float4 sf[kWarps * 3 * kNT];
-  __shared__ float chebf[kWarps * 3 * kMaxP1];
   __shared__ EvalTask sT;
   const BlockRef it = items[blockIdx.x];
   if (threadIdx.x == 0) sT = tasks[it.task];
   __syncthreads();
-  if (FAM == F_SL) run_item<K_SL_OFF>(sT, it, segs, sm, sf, chebf);
-  else if (FAM == F_DL) run_item<K_DL_OFF>(sT, it, segs, sm, sf, chebf);
-  else if (ON) run_item<K_E2G_UP_AWAY>(sT, it, segs, sm, sf, chebf);
-  else run_item<K_E2G_UP7>(sT, it, segs, sm, sf, chebf);
+  run_item<FACE ? K_E2G_UP_AWAY : K_E2G_UP7>(sT, it, segs, sm, sf);
 }
 
 // Sums a target block's item partials in slot order and applies the
@@ -1073,18 +1241,18 @@ __global__ void __launch_bounds__(kTB) reduce_kernel(const EvalTask* __restrict_
 }  // namespace
 
 void launch_eval(int family, const EvalTask* d_tasks, const BlockRef* d_items, const Seg* d_segs, int nitems, int n_on,
-                 cudaStream_t st, cudaStream_t side) {
+                 unsigned* next, int num_sms, cudaStream_t st, cudaStream_t side) {
   const int n_off = nitems - n_on;
   const BlockRef* off = d_items + n_on;
   if (family == F_SL) {
-    if (n_on > 0) eval_kernel_on2<F_SL><<<n_on, kTB2, 0, st>>>(d_tasks, d_items, d_segs);
-    if (n_off > 0) eval_kernel<F_SL, false><<<n_off, kTB, 0, side>>>(d_tasks, off, d_segs);
+    launch_units<K_SL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, st);
+    launch_units<K_SL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, side);
   } else if (family == F_DL) {
-    if (n_on > 0) eval_kernel_on2<F_DL><<<n_on, kTB2, 0, st>>>(d_tasks, d_items, d_segs);
-    if (n_off > 0) eval_kernel<F_DL, false><<<n_off, kTB, 0, side>>>(d_tasks, off, d_segs);
+    launch_units<K_DL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, st);
+    launch_units<K_DL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, side);
   } else {
-    if (n_on > 0) eval_kernel<F_E2G, true><<<n_on, kTB, 0, st>>>(d_tasks, d_items, d_segs);
-    if (n_off > 0) eval_kernel<F_E2G, false><<<n_off, kTB, 0, side>>>(d_tasks, off, d_segs);
+    if (n_on > 0) eval_kernel_e2g<true><<<n_on, kTB, 0, st>>>(d_tasks, d_items, d_segs);
+    if (n_off > 0) eval_kernel_e2g<false><<<n_off, kTB, 0, side>>>(d_tasks, off, d_segs);
   }
 }
 

@@ -301,7 +301,7 @@ void DevTree::build(const hr_surface& S, int P, int N0, double theta, bool direc
   partial.alloc((size_t)std::max(1, nitems) * 12 * Pf);
   mom.alloc((size_t)nn * 12 * Pf);
   mom.zero(st);
-  momf.alloc((size_t)nn * 12 * Pf);
+  momf.alloc((size_t)nn * momf_stride(host.P + 1, 20));
   momf.zero(st);
 }
 
@@ -352,7 +352,7 @@ void set_densities(Ctx& C, DevTree* t0, DevTree* t1, const double* q0, const dou
     launch_moments(ch, t0->P1, m0, m1, C.stream);
     C.launches++;
   }
-  launch_moments_reduce(ch, t0->Pf, m0, m1, C.stream);
+  launch_moments_reduce(ch, t0->P1, m0, m1, C.stream);
   C.launches++;
 }
 
@@ -428,11 +428,18 @@ bool lean_kind(int k) {
 }
 
 // Cost of one target-source pair and of one target-proxy pair for a warp, in
-// FP64 instructions of the kernels of hr_eval64.cu.
+// FP64 instructions of the kernels of hr_eval64.cu, or issue slots of the
+// reduced-precision two-surface kernels of hr_eval.cu (an off-surface pair: the
+// mean of the singular kernel and of the regularized forms).
 struct PairCost {
   double direct, proxy;
 };
-PairCost pair_cost(int kind) {
+PairCost pair_cost(int kind, int mixed) {
+  const bool dl = kind == K_DL_ON || kind == K_DL_OFF, sl = kind == K_SL_ON || kind == K_SL_OFF;
+  if (mixed) {
+    if (dl || sl) return {kind == K_DL_ON || kind == K_SL_ON ? 24.0 : 60.0, 15.0};
+    return {2.0, 1.5};  // the extend-to-grid sums, in relative units
+  }
   switch (kind) {
     case K_DL_ON: return {36, 25};
     case K_DL_OFF: return {75, 25};
@@ -452,8 +459,9 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     Seg s;
     double cost;
   };
-  // The FP64 kernels take work by the warp (hr_eval64.cu); the others by the CTA.
-  const bool by_warp = !tasks.empty() && !tasks[0].mixed;
+  // The two-surface kernels and the FP64 extend-to-grid ones take work by the
+  // warp; the reduced-precision extend-to-grid ones by the CTA.
+  const bool mixed = !tasks.empty() && tasks[0].mixed, by_warp = !mixed || family != F_E2G;
   auto entry_warps = [](const Entry& E) {
     int warps = 0;
     for (int w = 0; w < 4; w++) warps += E.mask[w] != 0u;
@@ -465,7 +473,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     const Lists& L = *lists[t];
     const Tree& T = *trees[t];
     const double Pf = (double)(T.P + 1) * (T.P + 1) * (T.P + 1);
-    const PairCost pc = by_warp ? pair_cost(tasks[t].kind) : PairCost{2.0, 1.5};
+    const PairCost pc = pair_cost(tasks[t].kind, tasks[t].mixed);
     double sum = 0.0;
     // every cost is a multiple of 1/2 far below 2^52: exact in any order
 #pragma omp parallel for schedule(dynamic, 16) reduction(+ : sum)
@@ -481,13 +489,18 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   //    CTAs x 16 waves), never below two tiles. By the warp: each launch on its
   //    own and with its kinds' costs, in segments no longer than an item and
   //    never below kMinSrc sources (stresslet batch at h = 1/64, P = 6, with
-  //    kWaves = 8 / 16 / 24 / 48: 4.06 / 3.87 / 3.89 / 3.92 ms; one partition
-  //    for both launches 4.14 ms).
+  //    kWaves = 8 / 16 / 24 / 48: FP64 4.06 / 3.87 / 3.89 / 3.92 ms; one
+  //    partition for both launches 4.14 ms; the reduced-precision operator 8 /
+  //    16 / 32 / 64: 2.80 / 2.61 / 2.64 / 2.68 ms).
   constexpr double kWaves = 16, kMinSrc = 128;
+  // Segment lengths are a multiple of this. Reduced precision: of its tiles, so
+  // that the FP32 sums of 16 sources do not depend on how the work is cut.
+  const int cut = mixed ? 64 : 32;
   double target[2];
   for (int c = 0; c < 2; c++) target[c] = std::max((total[0] + total[1]) / (num_sms * 4.0 * 16.0), 2.0 * 256.0 * 2.0);
   if (by_warp)
-    for (int c = 0; c < 2; c++) target[c] = std::max(4.0 * total[c] / (num_sms * 16.0 * kWaves), 4.0 * kMinSrc * 36.0);
+    for (int c = 0; c < 2; c++) target[c] = std::max(4.0 * total[c] / (num_sms * 16.0 * kWaves),
+                                                      4.0 * kMinSrc * (mixed ? 24.0 : 36.0));
   // 3. segments: a far entry whole, a near entry cut into source ranges of at
   //    most 512; cost ~ active warps x pair evaluations.
   std::vector<std::vector<std::vector<HSeg>>> per(tasks.size());
@@ -495,9 +508,10 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     const Lists& L = *lists[t];
     const Tree& T = *trees[t];
     const double Pf = (double)(T.P + 1) * (T.P + 1) * (T.P + 1);
-    const PairCost pc = by_warp ? pair_cost(tasks[t].kind) : PairCost{2.0, 1.5};
+    const PairCost pc = pair_cost(tasks[t].kind, tasks[t].mixed);
     const double want = target[lean_kind(tasks[t].kind) ? 0 : 1];
-    const int seg = by_warp ? std::min(512, std::max((int)kMinSrc, (int)(want / (4.0 * pc.direct)) / 32 * 32)) : 512;
+    const int seg =
+        by_warp ? std::min(512, std::max((int)kMinSrc, (int)(want / (4.0 * pc.direct)) / cut * cut)) : 512;
     per[t].resize(L.nblocks());
 #pragma omp parallel for schedule(dynamic, 16)
     for (int b = 0; b < L.nblocks(); b++) {
@@ -615,7 +629,7 @@ void Batch::launch(Ctx& C) {
     HR_CHECK_CUDA(cudaEventRecord(C.ev_fork, C.stream));
     HR_CHECK_CUDA(cudaStreamWaitEvent(C.side, C.ev_fork, 0));
   }
-  if (!tasks.empty() && tasks[0].mixed) launch_eval(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, C.stream, side);
+  if (!tasks.empty() && tasks[0].mixed) launch_eval(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, d_next.p, C.num_sms, C.stream, side);
   else
     launch_eval64(family, d_tasks.p, d_items.p, d_segs.p, nitems, n_on, d_next.p, C.num_sms, C.stream, side,
                   C.count_work);

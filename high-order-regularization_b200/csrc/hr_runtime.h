@@ -184,7 +184,7 @@ struct DevTree {
   DBuf<double> pk;  // packed records (Pack), up to 12 doubles per source
   DBuf<float> fnx, fny, fnz, fa, fqx, fqy, fqz;  // FP32 copies
   DBuf<double> mom;  // nn * Pf * C, proxy-major (C = 10 DL symmetric form, 6 SL)
-  DBuf<float> momf;  // nn * Pf * W32 FP32 copy (W32 = 12 DL, 8 SL)
+  DBuf<float> momf;  // FP32 copy, momf_stride floats per node
   DBuf<MomItem> items;
   DBuf<int> item_start;
   DBuf<double> partial;
@@ -239,7 +239,7 @@ struct Batch {
   DBuf<int> d_item_start;
   DBuf<int2> d_task_blocks;
   DBuf<double> d_partial;
-  DBuf<unsigned> d_next;  // work counters of the FP64 launches, zero between launches
+  DBuf<unsigned> d_next;  // work counters of the launches, zero between launches
   int nitems = 0, ntask_blocks = 0;
   int n_on = 0;  // leading lean items (on-surface / box-face tasks, launched on their own)
   bool ready = false;  // finalize has run
