@@ -99,7 +99,7 @@ struct Shape<C_DL_ON> {
 };
 template <>
 struct Shape<C_DL_OFF> {
-  static constexpr int pieces = HR_T64_F0_PIECES, coef = HR_T64_F0_COEF, warps = 8, tile = 32, rec = 10, unroll = 2;
+  static constexpr int pieces = HR_T64_F0_PIECES, coef = HR_T64_F0_COEF, warps = 8, tile = 32, rec = 10, unroll = 4;
   static constexpr bool exp = true, pair = false;
 };
 template <>
@@ -245,15 +245,24 @@ __device__ __forceinline__ void load_target(const EvalTask& T, int t, Tgt<KIND =
 // polynomials the rest.
 struct NearDL {  // an off-surface stresslet target's data for its direct pairs, loaded per segment
   int near;
-  double b, x0[3], n0[3], Q[3], R[3];
+  // The target is x0 + b n0 with |n0| = 1, up to 1e-13 delta (true for any
+  // target without subtraction): beyond 8 delta, where s2 = r^2 s3, its pairs
+  // are plain stresslets of g - g0.
+  bool foot;
+  double b, x0[3], n0[3], g0[3], Q[3], R[3];  // g0: zero without subtraction
   template <int KIND>
   __device__ __forceinline__ void load(const EvalTask& T, int t, const Len& g) {
     near = T.tnear[t];
     b = T.tb[t];
+    double off = 0.0, nn = -1.0;
     for (int k = 0; k < 3; k++) {
       x0[k] = T.tx0[3 * t + k];
       n0[k] = T.tn0[3 * t + k];
+      g0[k] = near ? T.tg0[3 * t + k] : 0.0;
+      off = fmax(off, fabs(fma(-b, n0[k], T.txyz[3 * t + k] - x0[k])));
+      nn = fma(n0[k], n0[k], nn);
     }
+    foot = !near || (off <= 1e-13 * T.DEL && fabs(nn) <= 1e-13);
     Coef c;
     c.c1 = c.c2 = c.c3 = 0.0;
     if (near) c = reg_coeff(b / T.DEL);
@@ -385,11 +394,20 @@ __device__ __forceinline__ void pairs_dl_on(const double2* s, const Tgt<true> (&
 // stresslet for the others. With m1 = d c1a - n0 c1b and m2 = -sig m1 + d c2a +
 // xh c2b the reference's m1 s2 + m2 s3 is d (c1a al + c2a s3) + xh c2b s3 -
 // n0 c1b al, al = s2 - sig s3; the n0 terms add up in a scalar (a[3]). The
-// tile holds area x normal.
+// tile holds area x normal. A step without a near pair inside 8 delta (by a
+// count over all sources four of five of the near warps' pairs of sources at h
+// = 1/32, 92 % at h = 1/64) takes the subtraction form's pairs as plain
+// stresslets too, where every target of the warp allows it (plain): with x =
+// x0 + b n0, d = b n0 - xh and r^2 = sig + b^2 the two are the same, and the
+// plain one takes 30 FP64 operations instead of 75. Operator application at h
+// = 1/64 3.90 -> 3.73 ms, at h = 1/32 0.811 -> 0.749 ms (steps of 2 / 3 / 4
+// sources 3.75 / 3.74 / 3.73; 4 for the plain pairs and 2 for the others
+// 3.77). Measured and not kept: whole tiles beyond 8 delta of the box around
+// the unit's near targets first, both targets of a lane at once, 3.84 ms.
 template <int U, bool COUNT>
 __device__ __forceinline__ void pairs_dl_off(const double2* s, const Tgt<true>& P, const NearDL& S, const Len& g,
-                                             const double2* tab, const double* ex, bool act, bool any_near, bool any_far, const EvalTask& T,
-                                             Count& cnt, double (&a)[4]) {
+                                             const double2* tab, const double* ex, bool act, bool any_near, bool any_far, bool plain,
+                                             const EvalTask& T, Count& cnt, double (&a)[4]) {
   double dx[U], dy[U], dz[U], r2[U], s2[U], s3[U];
   bool tb[U], any_t = false, any_p = false;
 #pragma unroll
@@ -405,7 +423,24 @@ __device__ __forceinline__ void pairs_dl_off(const double2* s, const Tgt<true>& 
     any_p |= !tb[u];
     s2[u] = s3[u] = 0.0;
   }
-  if (__any_sync(kFull, act && any_t)) {
+  const bool tables = __any_sync(kFull, act && any_t);
+  if (!tables && plain) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const Src q = load_src(s + 5 * u);
+      const double xr = cap(r2[u]), y = rsqrt20(xr), y2 = y * y;
+      const double e = fma(-xr, y2, 1.0);
+      const double p5 = fma(fma(4.375, e, 2.5), e, 1.0) * (y2 * y2 * y);
+      const double gdd = fma(q.qx - S.g0[0], dx[u], fma(q.qy - S.g0[1], dy[u], (q.qz - S.g0[2]) * dz[u]));
+      const double ndd = fma(q.nx, dx[u], fma(q.ny, dy[u], q.nz * dz[u]));
+      const double k = gdd * ndd * p5;
+      a[0] = fma(dx[u], k, a[0]);
+      a[1] = fma(dy[u], k, a[1]);
+      a[2] = fma(dz[u], k, a[2]);
+    }
+    return;
+  }
+  if (tables) {
 #pragma unroll
     for (int u = 0; u < U; u++) {
       double t, c[2 * Lay<C_DL_OFF>::pairs], f, df;
@@ -437,7 +472,7 @@ __device__ __forceinline__ void pairs_dl_off(const double2* s, const Tgt<true>& 
     for (int u = 0; u < U; u++) {
       const Src q = load_src(s + 5 * u);
       const double xh = q.x - S.x0[0], yh = q.y - S.x0[1], zh = q.z - S.x0[2];
-      const double gx = q.qx - P.g0[0], gy = q.qy - P.g0[1], gz = q.qz - P.g0[2];
+      const double gx = q.qx - S.g0[0], gy = q.qy - S.g0[1], gz = q.qz - S.g0[2];
       const double xhn0 = fma(xh, S.n0[0], fma(yh, S.n0[1], zh * S.n0[2]));
       const double sig = fma(-2.0 * S.b, xhn0, fma(xh, xh, fma(yh, yh, zh * zh)));
       const double gn0 = fma(gx, S.n0[0], fma(gy, S.n0[1], gz * S.n0[2]));
@@ -782,8 +817,9 @@ __device__ __forceinline__ void near_segment(const EvalTask& T, int s0, int n,
   using NEAR = std::conditional_t<CLS == C_DL_OFF, NearDL, std::conditional_t<CLS == C_SL_OFF || CLS == C_BAND, NearSL, NearNone>>;
   NEAR N[NT];
   for (int k = 0; k < NT; k++) N[k].template load<KIND>(T, t[k], g);
-  bool any_near = true, any_far = false;
+  bool any_near = true, any_far = false, plain = false;
   if constexpr (KIND == K_DL_OFF) {
+    plain = !__any_sync(kFull, act[0] && !N[0].foot);
     any_near = __any_sync(kFull, act[0] && N[0].near);
     any_far = __any_sync(kFull, act[0] && !N[0].near);
   }
@@ -803,7 +839,7 @@ __device__ __forceinline__ void near_segment(const EvalTask& T, int s0, int n,
       const double2* q = s + (kRec / 2) * j;
       if constexpr (KIND == K_DL_ON) pairs_dl_on<NT, V, COUNT>(q, S, g, tab, act, T, cnt, p);
       else if constexpr (KIND == K_DL_OFF)
-        pairs_dl_off<V, COUNT>(q, S[0], N[0], g, tab, ex, act[0], any_near, any_far, T, cnt, p[0]);
+        pairs_dl_off<V, COUNT>(q, S[0], N[0], g, tab, ex, act[0], any_near, any_far, plain, T, cnt, p[0]);
       else if constexpr (KIND == K_SL_ON || KIND == K_SL_OFF) pairs_sl<CLS, NT, V, COUNT>(q, S, N, g, tab, ex, act, T, cnt, p);
       else if constexpr (CLS == C_FACE) pairs_face<KIND, NT, V>(q, S, p);
       else pairs_band<KIND, NT, V>(q, S, N, g, tab, ex, act, T.DEL, p);

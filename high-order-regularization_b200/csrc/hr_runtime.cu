@@ -430,7 +430,10 @@ bool lean_kind(int k) {
 // Cost of one target-source pair and of one target-proxy pair for a warp, in
 // FP64 instructions of the kernels of hr_eval64.cu, or issue slots of the
 // reduced-precision two-surface kernels of hr_eval.cu (an off-surface pair: the
-// mean of the singular kernel and of the regularized forms).
+// mean of the singular kernel and of the regularized forms). The off-surface
+// stresslet's pairs cost 30 or 75, or both where lanes differ; 100 leaves its
+// items short (operator at h = 1/32 with 55 / 75 / 100 / 130: 0.760 / 0.752 /
+// 0.743 / 0.746 ms).
 struct PairCost {
   double direct, proxy;
 };
@@ -442,7 +445,7 @@ PairCost pair_cost(int kind, int mixed) {
   }
   switch (kind) {
     case K_DL_ON: return {36, 25};
-    case K_DL_OFF: return {75, 25};
+    case K_DL_OFF: return {100, 25};
     case K_SL_ON: return {40, 22};
     case K_SL_OFF: return {50, 22};
     case K_E2G_SL_AWAY:
