@@ -24,7 +24,7 @@
 //     128-byte phase without bank conflict, 10 from random pieces of a table.
 // Measured for the two launches of a batch (two-surface problem, h = 1/64, P =
 // 6, N0 = 2000), against one-thread-per-target CTAs with a table each and
-// CUDA's rsqrt, erf and exp: stresslet 4.91 -> 3.78 ms (on-surface 2.98 -> 2.32,
+// CUDA's rsqrt, erf and exp: stresslet 4.91 -> 3.60 ms (on-surface 2.98 -> 2.31,
 // FP64 pipe 57 -> 67 %, data pipe 70 -> 54 %), Stokeslet 4.91 -> 3.58 ms;
 // extend-to-grid sums at N = 96 / 192 2.36 / 29.0 -> 1.79 / 22.8 ms (box faces
 // 81 % of the FP64 pipe). What they do for that:
