@@ -1271,12 +1271,15 @@ void launch_eval(int family, const EvalTask* d_tasks, const BlockRef* d_items, c
                  unsigned* next, int num_sms, cudaStream_t st, cudaStream_t side) {
   const int n_off = nitems - n_on;
   const BlockRef* off = d_items + n_on;
+  // the off-surface items first: their units' times differ most (near targets),
+  // and the other launch fills their tail (operator at h = 1/32 0.735 -> 0.665 ms,
+  // h = 1/24 0.42 -> 0.39)
   if (family == F_SL) {
-    launch_units<K_SL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, st);
-    launch_units<K_SL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, side);
+    launch_units<K_SL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, st);
+    launch_units<K_SL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, side);
   } else if (family == F_DL) {
-    launch_units<K_DL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, st);
-    launch_units<K_DL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, side);
+    launch_units<K_DL_OFF>(d_tasks, off, d_segs, n_off, next + 1, num_sms, st);
+    launch_units<K_DL_ON>(d_tasks, d_items, d_segs, n_on, next, num_sms, side);
   } else {
     if (n_on > 0) eval_kernel_e2g<true><<<n_on, kTB, 0, st>>>(d_tasks, d_items, d_segs);
     if (n_off > 0) eval_kernel_e2g<false><<<n_off, kTB, 0, side>>>(d_tasks, off, d_segs);

@@ -495,7 +495,12 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   //    kWaves = 8 / 16 / 24 / 48: FP64 4.06 / 3.87 / 3.89 / 3.92 ms; one
   //    partition for both launches 4.14 ms; the reduced-precision operator 8 /
   //    16 / 32 / 64: 2.80 / 2.61 / 2.64 / 2.68 ms).
-  constexpr double kWaves = 16, kMinSrc = 128;
+  //    kMinSrc: 64 instead of 128 sources take the reduced-precision operator
+  //    at h = 1/16 / 1/24 / 1/32 / 1/64 from 0.305 / 0.427 / 0.666 / 2.47 to
+  //    0.223 / 0.330 / 0.644 / 2.46 ms (a near target's FP64 pairs make long
+  //    units).
+  constexpr double kWaves = 16;
+  const int kMinSrc = mixed ? 64 : 128;
   // Segment lengths are a multiple of this. Reduced precision: of its tiles, so
   // that the FP32 sums of 16 sources do not depend on how the work is cut.
   const int cut = mixed ? 64 : 32;
@@ -514,7 +519,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     const PairCost pc = pair_cost(tasks[t].kind, tasks[t].mixed);
     const double want = target[lean_kind(tasks[t].kind) ? 0 : 1];
     const int seg =
-        by_warp ? std::min(512, std::max((int)kMinSrc, (int)(want / (4.0 * pc.direct)) / cut * cut)) : 512;
+        by_warp ? std::min(512, std::max(kMinSrc, (int)(want / (4.0 * pc.direct)) / cut * cut)) : 512;
     per[t].resize(L.nblocks());
 #pragma omp parallel for schedule(dynamic, 16)
     for (int b = 0; b < L.nblocks(); b++) {
