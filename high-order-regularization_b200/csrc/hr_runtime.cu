@@ -491,24 +491,30 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   //    Small items keep the tail short. By the CTA: total / (SMs x 4 resident
   //    CTAs x 16 waves), never below two tiles. By the warp: each launch on its
   //    own and with its kinds' costs, in segments no longer than an item and
-  //    never below kMinSrc sources (stresslet batch at h = 1/64, P = 6, with
+  //    never below min_src sources (stresslet batch at h = 1/64, P = 6, with
   //    kWaves = 8 / 16 / 24 / 48: FP64 4.06 / 3.87 / 3.89 / 3.92 ms; one
   //    partition for both launches 4.14 ms; the reduced-precision operator 8 /
   //    16 / 32 / 64: 2.80 / 2.61 / 2.64 / 2.68 ms).
-  //    kMinSrc: 64 instead of 128 sources take the reduced-precision operator
-  //    at h = 1/16 / 1/24 / 1/32 / 1/64 from 0.305 / 0.427 / 0.666 / 2.47 to
-  //    0.223 / 0.330 / 0.644 / 2.46 ms (a near target's FP64 pairs make long
-  //    units).
-  constexpr double kWaves = 16;
-  const int kMinSrc = mixed ? 64 : 128;
+  //    The least item: FP64 128 sources, where that leaves a warp fewer than
+  //    kFew items fewer, down to 64 (operator at h = 1/14 / 1/18 / 1/24 / 1/32
+  //    with 128 throughout 0.174 / 0.220 / 0.343 / 0.738 ms, so 0.136 / 0.192 /
+  //    0.322 / 0.740; 64 throughout 0.760 at h = 1/32; kFew = 3 0.341 at h =
+  //    1/24, 8 the same as 5). Reduced precision 64: 128 took the operator at h
+  //    = 1/16 / 1/24 / 1/32 / 1/64 0.305 / 0.427 / 0.666 / 2.47 ms, 64 0.223 /
+  //    0.330 / 0.644 / 2.46 (a near target's FP64 pairs make long units).
+  constexpr double kWaves = 16, kFew = 5;
+  int min_src[2];
   // Segment lengths are a multiple of this. Reduced precision: of its tiles, so
   // that the FP32 sums of 16 sources do not depend on how the work is cut.
   const int cut = mixed ? 64 : 32;
   double target[2];
   for (int c = 0; c < 2; c++) target[c] = std::max((total[0] + total[1]) / (num_sms * 4.0 * 16.0), 2.0 * 256.0 * 2.0);
-  if (by_warp)
-    for (int c = 0; c < 2; c++) target[c] = std::max(4.0 * total[c] / (num_sms * 16.0 * kWaves),
-                                                      4.0 * kMinSrc * (mixed ? 24.0 : 36.0));
+  for (int c = 0; c < 2; c++) {
+    const double few = 4.0 * total[c] / (num_sms * 16.0 * kFew) / (4.0 * 36.0);  // sources
+    min_src[c] = mixed ? 64 : std::max(64, (int)std::min(128.0, few) / 32 * 32);
+    if (by_warp)
+      target[c] = std::max(4.0 * total[c] / (num_sms * 16.0 * kWaves), 4.0 * min_src[c] * (mixed ? 24.0 : 36.0));
+  }
   // 3. segments: a far entry whole, a near entry cut into source ranges of at
   //    most 512; cost ~ active warps x pair evaluations.
   std::vector<std::vector<std::vector<HSeg>>> per(tasks.size());
@@ -518,8 +524,8 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     const double Pf = (double)(T.P + 1) * (T.P + 1) * (T.P + 1);
     const PairCost pc = pair_cost(tasks[t].kind, tasks[t].mixed);
     const double want = target[lean_kind(tasks[t].kind) ? 0 : 1];
-    const int seg =
-        by_warp ? std::min(512, std::max(kMinSrc, (int)(want / (4.0 * pc.direct)) / cut * cut)) : 512;
+    const int least = min_src[lean_kind(tasks[t].kind) ? 0 : 1];
+    const int seg = by_warp ? std::min(512, std::max(least, (int)(want / (4.0 * pc.direct)) / cut * cut)) : 512;
     per[t].resize(L.nblocks());
 #pragma omp parallel for schedule(dynamic, 16)
     for (int b = 0; b < L.nblocks(); b++) {
