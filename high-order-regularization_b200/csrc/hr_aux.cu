@@ -9,7 +9,6 @@ namespace hr {
 
 namespace {
 
-constexpr int kMaxP1 = 16;
 
 // Upward pass: the barycentric Lagrange proxy moments of Panel_Moments_SL /
 // Panel_Moments_DL (2S/KITC.cpp:351-668) of one (node, source range) item,

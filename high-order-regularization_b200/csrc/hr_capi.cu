@@ -468,7 +468,6 @@ extern "C" int hr_e2g_solve_poisson(hr_ctx* ctx, int N, double L, const uint8_t*
     HR_REQUIRE(N >= 6 && L > 0 && band2 && outside && u, "bad Poisson arguments");
     HR_REQUIRE(!(variable >= 1 && variable <= 3) || p, "pressure grid missing");
     HR_CHECK_CUDA(cudaSetDevice(ctx->c.device));
-    cudaStream_t st = ctx->c.stream;
     size_t m = (size_t)(N + 1) * (N + 1) * (N + 1);
     WorkspaceScope scope(ctx->c);
     DBuf<uint8_t> db, dout;

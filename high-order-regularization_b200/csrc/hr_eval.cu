@@ -21,8 +21,8 @@
 // different operands). With them, rsqrt without denormal scaling and units
 // taken by the warp, the stresslet batch's kernels (two-surface problem, h =
 // 1/64, P = 6, N0 = 2000) execute 0.73e9 + 0.69e9 instructions instead of
-// 1.21e9 + 0.90e9; on-surface 1.92 -> 1.18 ms, off-surface 1.71 -> 1.25 ms,
-// the operator application 3.55 -> 2.49 ms against one scalar pair at a time
+// 1.21e9 + 0.90e9; on-surface 1.92 -> 1.17 ms, off-surface 1.71 -> 1.15 ms,
+// the operator application 3.53 -> 2.47 ms against one scalar pair at a time
 // in CTAs per item. Twelve warps: 168 registers, two targets' sums without
 // spills; 8 / 10 / 13 / 14 warps 3.41 (8, before the finer items) / 2.57 /
 // 2.55 / 2.62 ms.
