@@ -849,8 +849,9 @@ __device__ __forceinline__ void near_segment(const EvalTask& T, int s0, int n,
     for (; j < c; j++) step(std::integral_constant<int, 1>(), j);
     __syncwarp();
   }
-  if constexpr (KIND == K_DL_OFF) {  // the n0 terms
-    for (int c = 0; c < 3; c++) p[0][c] = fma(-N[0].n0[c], p[0][3], p[0][c]);
+  if constexpr (KIND == K_DL_OFF) {  // the n0 terms; a far target's n0 is never used and may hold anything
+    if (N[0].near)
+      for (int c = 0; c < 3; c++) p[0][c] = fma(-N[0].n0[c], p[0][3], p[0][c]);
     p[0][3] = 0.0;
   }
 }
