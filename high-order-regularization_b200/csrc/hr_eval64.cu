@@ -39,8 +39,10 @@
 //     derivative; off-surface factors add a polynomial with the target's
 //     coefficients times e^-s, which is a table value e^{-i/4} times a
 //     constant-coefficient polynomial in the piece's offset.
-//   * The pieces are addressed in r^2 itself (their offsets and coefficients
-//     carry the powers of delta), which saves the scaling of r^2.
+//   * A piece's polynomial is in the offset from its centre in pieces, which
+//     one multiply-add forms from r^2. Offsets in r^2 with the powers of delta
+//     in the coefficients cost the same and lose the high-order coefficients
+//     to underflow from delta = 1e12 on (delta^-23).
 //   * 1/r^3 and 1/r^5 come from the hardware's approximate reciprocal square
 //     root y (rsqrt.approx.ftz.f64: a 20-bit result, so y^2 is exact) and the
 //     binomial series (1 - e)^{-k/2} in e = 1 - r^2 y^2 (|e| < 2^-18) to second
@@ -129,9 +131,10 @@ struct Lay : Shape<CLS> {
 // Constants of a task's regularization length.
 struct Len {
   double inv_d2;
-  double inv_w, w;  // 4 / delta^2 and delta^2 / 4: pieces per unit of r^2 and back
-  int hi_tab;       // high word of the largest tabulated r^2
-  int hi_zero;      // high word of the reference's r < 1e-14 limit, squared
+  double inv_w;    // 4 / delta^2: pieces per unit of r^2
+  double df, dt;   // -2 and -2/3 d(pieces)/d(r^2): from a derivative by the piece's offset to G2, F and T
+  int hi_tab;      // high word of the largest tabulated r^2
+  int hi_zero;     // high word of the reference's r < 1e-14 limit, squared
 };
 
 template <int CLS>
@@ -139,8 +142,11 @@ __device__ __forceinline__ Len make_len(double d) {
   Len g;
   const double inv = 1.0 / d;
   g.inv_d2 = inv * inv;
-  g.inv_w = 4.0 * g.inv_d2;
-  g.w = 0.25 * (d * d);
+  // correctly rounded but for the last step: its relative error is that of every s
+  const double d2 = d * d, q = 4.0 / d2;
+  g.inv_w = fma(fma(-q, fma(d, d, -d2), fma(-q, d2, 4.0)), 0.25 * q, q);
+  g.df = -2.0 * g.inv_w;
+  g.dt = -2.0 / 3.0 * g.inv_w;
   // on the surface the factors equal the singular kernel's to 2^-54 from s = 51
   // on (hr_pairs.cuh); off it the reference's switch at r = 8 delta
   const bool on = CLS == C_SL_ON || CLS == C_DL_ON;
@@ -162,11 +168,11 @@ __device__ __forceinline__ double cap(double r2) {
   return __hiloint2double(min(__double2hiint(r2), 0x7fb00000), __double2loint(r2));
 }
 
-// The piece of r^2 and the offset from its centre (in r^2).
+// The piece of r^2 and the offset from its centre (in pieces: |t| <= 1/2).
 template <int CLS>
 __device__ __forceinline__ const double2* piece(const double2* tab, const Len& g, double r2, double& t, int& i) {
   const double f = fma(r2, g.inv_w, kRoundMagic);
-  t = fma(kRoundMagic - f, g.w, r2);
+  t = fma(r2, g.inv_w, kRoundMagic - f);
   i = (int)min((unsigned)__double2loint(f), (unsigned)(Shape<CLS>::pieces - 1));
   return tab + (size_t)i * (Lay<CLS>::pairs * kRep);
 }
@@ -202,12 +208,13 @@ __device__ __forceinline__ void poly2(const double (&c)[2 * Lay<CLS>::pairs], do
   }
 }
 
-// e^{-s} at s = i / 4 + t (|t| <= 1/8).
+// e^{-s} at s = (i + t) / 4.
 __device__ __forceinline__ double exp_piece(const double* ex, int i, double t) {
   constexpr double c[] = {HR_T64_EXP_COEFS};
-  double v = c[9];
+  constexpr double q[] = {1.0, 0x1p-2, 0x1p-4, 0x1p-6, 0x1p-8, 0x1p-10, 0x1p-12, 0x1p-14, 0x1p-16, 0x1p-18};
+  double v = c[9] * q[9];
 #pragma unroll
-  for (int k = 8; k >= 0; k--) v = fma(v, t, c[k]);
+  for (int k = 8; k >= 0; k--) v = fma(v, t, c[k] * q[k]);
   return v * ex[i];
 }
 
@@ -447,9 +454,9 @@ __device__ __forceinline__ void pairs_dl_off(const double2* s, const Tgt<true>& 
       int i;
       load_piece<C_DL_OFF>(piece<C_DL_OFF>(tab, g, r2[u], t, i), c);
       poly2<C_DL_OFF>(c, t, f, df);
-      const double x = exp_piece(ex, i, t * g.inv_d2);
+      const double x = exp_piece(ex, i, t);
       s2[u] = fma(fma(fma(S.Q[2], r2[u], S.Q[1]), r2[u], S.Q[0]), x, f);
-      s3[u] = fma(fma(fma(S.R[2], r2[u], S.R[1]), r2[u], S.R[0]), x, -2.0 / 3.0 * df);
+      s3[u] = fma(fma(fma(S.R[2], r2[u], S.R[1]), r2[u], S.R[0]), x, g.dt * df);
       if (__double2hiint(r2[u]) < g.hi_zero) {  // the reference's values for r < 1e-14
         s2[u] = 256.0 / 15.0 / d_rootpi() / (T.DEL * T.DEL * T.DEL);
         s3[u] = 0.0;
@@ -523,9 +530,9 @@ __device__ __forceinline__ void factors_off(double r2, const NearSL& N, const Le
   int i;
   load_piece<CLS>(piece<CLS>(tab, g, r2, t, i), c);
   poly2<CLS>(c, t, v, dv);
-  const double x = exp_piece(ex, i, t * g.inv_d2);
+  const double x = exp_piece(ex, i, t);
   s1 = fma(fma(fma(N.P[2], r2, N.P[1]), r2, N.P[0]), x, v);
-  s2 = fma(fma(fma(N.Q[2], r2, N.Q[1]), r2, N.Q[0]), x, -2.0 * dv);
+  s2 = fma(fma(fma(N.Q[2], r2, N.Q[1]), r2, N.Q[0]), x, g.df * dv);
   if (__double2hiint(r2) < g.hi_zero) {  // the reference's values for r < 1e-14
     s1 = 32.0 / 5.0 / d_rootpi() / del;
     s2 = 256.0 / 15.0 / d_rootpi() / (del * del * del);
@@ -571,7 +578,7 @@ __device__ __forceinline__ void pairs_sl(const double2* s, const Tgt<false> (&S)
           int i;
           load_piece<CLS>(piece<CLS>(tab, g, r2[u][k], t, i), c);
           poly2<CLS>(c, t, s1[u][k], dv);
-          s2[u][k] = -2.0 * dv;
+          s2[u][k] = g.df * dv;
         } else {
           factors_off<CLS>(r2[u][k], N[k], g, T.DEL, tab, ex, s1[u][k], s2[u][k]);
         }
@@ -983,8 +990,8 @@ __global__ void __launch_bounds__(Shape<CLS>::warps * 32, 1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* wsm = ex + Lay<CLS>::exp_d + warp * Lay<CLS>::warp_d;
   // the smoothing table, eight copies, its coefficients scaled to offsets in
-  // r^2 and to the power of 1/delta of the factor (all tasks of a batch share
-  // one delta)
+  // pieces (exactly, by powers of four) and to the power of 1/delta of the factor
+  // (all tasks of a batch share one delta)
   if constexpr (Shape<CLS>::pieces > 0) {
     const double inv = 1.0 / tasks[items[0].task].DEL, i2 = inv * inv;
     const double lead = CLS == C_DL_ON ? i2 * i2 * inv : (CLS == C_DL_OFF ? i2 * inv : inv);
@@ -993,7 +1000,7 @@ __global__ void __launch_bounds__(Shape<CLS>::warps * 32, 1)
     double scale[2 * kP];
     scale[0] = lead;
 #pragma unroll
-    for (int k = 1; k < 2 * kP; k++) scale[k] = scale[k - 1] * i2;
+    for (int k = 1; k < 2 * kP; k++) scale[k] = scale[k - 1] * 0.25;
     for (int i = threadIdx.x; i < Shape<CLS>::pieces; i += blockDim.x) {
 #pragma unroll
       for (int k = 0; k < kP; k++) {
