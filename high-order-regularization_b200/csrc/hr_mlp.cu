@@ -279,11 +279,14 @@ __global__ void __launch_bounds__(kTrainThreads) train_kernel(
   const int ty = (lane & 7) + 8 * (warp & 3), tx = (lane >> 3) + 4 * (warp >> 2);
   const int s = blockIdx.x * kS + tid;  // this thread's sample in the per-sample parts (tid < kS)
   const bool valid = tid < kS && s < batch;
-  const long g = valid ? sample_index(s, n, seed, step, random) : 0;
+  // past the batch's end a tile repeats its first sample with output deltas of
+  // zero: what a sample without input (the biases alone) gives may overflow where
+  // no sample of the batch does, and 0 x inf would reach the gradient
+  const long g = tid < kS ? sample_index(valid ? s : blockIdx.x * kS, n, seed, step, random) : 0;
   load_params<kTrainThreads>(P, params);
   if (tid < kS) {
 #pragma unroll
-    for (int i = 0; i < kIn; i++) x[i * kSP + tid] = valid ? (X[g * kIn + i] - nm.mean[i]) * nm.inv_std[i] : 0.f;
+    for (int i = 0; i < kIn; i++) x[i * kSP + tid] = (X[g * kIn + i] - nm.mean[i]) * nm.inv_std[i];
   }
   __syncthreads();
   float z[8][4];
@@ -428,7 +431,7 @@ __global__ void __launch_bounds__(128) grad_adam_kernel(const float* __restrict_
   const int per = (ntiles + 3) / 4, c0 = warp * per, c1 = min(ntiles, c0 + per);
   double sum = 0.0;
   if (p < kNP) {
-int c = c0;
+    int c = c0;
     for (; c + 8 <= c1; c += 8) {
       float t[8];
 #pragma unroll
