@@ -752,10 +752,7 @@ int plan_solve(hr_plan2s& P, const hr_gmres_opts& o, const double* b_dev, double
   hr_gmres_report R;
   memset(&R, 0, sizeof(R));
   R.true_residual = -1.0;
-  if (P.Vcols < m + 1) {
-    P.V.alloc((size_t)(m + 1) * n);
-    P.Vcols = m + 1;
-  }
+  grow(P.Vcols, m + 1, [&] { P.V.alloc((size_t)(m + 1) * n); });
   cudaEvent_t e0, e1;
   HR_CHECK_CUDA(cudaEventCreate(&e0));
   HR_CHECK_CUDA(cudaEventCreate(&e1));

@@ -512,11 +512,11 @@ struct hr_mlp {
   int cap = 0;
   long step = 0;
   void ensure(int batch) {
-    if (batch <= cap) return;
-    const size_t tiles = (batch + kS - 1) / kS;
-    loss_part.alloc(tiles);
-    partial.alloc(tiles * kNP);
-    cap = batch;
+    hr::grow(cap, batch, [&] {
+      const size_t tiles = ((size_t)batch + kS - 1) / kS;
+      loss_part.alloc(tiles);
+      partial.alloc(tiles * kNP);
+    });
   }
 };
 

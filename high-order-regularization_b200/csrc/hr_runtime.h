@@ -20,11 +20,15 @@ struct Error : std::runtime_error {
   Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
 
+// The error is taken from the runtime when it is thrown, so that a later call
+// does not report it again for a launch of its own.
 #define HR_CHECK_CUDA(call)                                                                  \
   do {                                                                                       \
     cudaError_t e_ = (call);                                                                 \
-    if (e_ != cudaSuccess)                                                                   \
+    if (e_ != cudaSuccess) {                                                                 \
+      cudaGetLastError();                                                                    \
       throw ::hr::Error(HR_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));    \
+    }                                                                                        \
   } while (0)
 
 #define HR_REQUIRE(cond, msg)                                   \
@@ -123,6 +127,18 @@ struct DBuf {
     n = count;
   }
 };
+
+// Grows buffers that are kept between calls: alloc allocates them anew for `want`,
+// `have` is what they hold now. It is zero while alloc runs, which lets go of
+// the old memory first: after a failed allocation the next call, of any size,
+// allocates again.
+template <class N, class F>
+void grow(N& have, N want, F&& alloc) {
+  if (want <= have) return;
+  have = 0;
+  alloc();
+  have = want;
+}
 
 struct Ctx {
   int device = 0;
