@@ -8,6 +8,7 @@ Only tests/, the smoke test and bench.py's CPU-baseline leg import this module.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import numpy as np
@@ -372,12 +373,15 @@ class Ref2S:
 
 
 class RefE2G:
-    """The unmodified reference extend-to-grid program (oracle/_ref)."""
+    """The unmodified reference extend-to-grid program (oracle/_ref), loaded on
+    first use: an object can be made before ref_available() is asked."""
 
-    def __init__(self):
-        self.lib = ctypes.CDLL(os.path.join(REF_DIR, "librefe2g.so"))
-        self.lib.refe2g_log.restype = ctypes.c_char_p
-        self.lib.refe2g_p_exact.restype = ctypes.c_double
+    @functools.cached_property
+    def lib(self):
+        lib = ctypes.CDLL(os.path.join(REF_DIR, "librefe2g.so"))
+        lib.refe2g_log.restype = ctypes.c_char_p
+        lib.refe2g_p_exact.restype = ctypes.c_double
+        return lib
 
     def setup(self, N):
         self.N = N
