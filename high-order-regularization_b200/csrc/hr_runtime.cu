@@ -167,11 +167,26 @@ void copy_parallel(char* out, const char* in, size_t n) {
 
 constexpr size_t kStageMin = size_t(1) << 20;  // smaller copies gain nothing from staging
 
+// Whether the copy engines reach the caller's array themselves (page-locked or
+// managed memory): a copy by way of the pinned buffers is slower there (21.9 MB
+// of grids 719 us instead of 397, a Poisson transform of 95^3 points 560 and 373).
+bool page_locked(const void* p, size_t bytes) {
+  for (const void* q : {p, static_cast<const void*>(static_cast<const char*>(p) + bytes - 1)}) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type == cudaMemoryTypeUnregistered) return false;
+  }
+  return true;
+}
+
 }  // namespace
 
 void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
   cudaStream_t st = C.stream;
-  if (bytes < kStageMin) {
+  if (bytes < kStageMin || page_locked(dst, bytes)) {
     HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     HR_CHECK_CUDA(cudaStreamSynchronize(st));
     return;
@@ -197,7 +212,7 @@ void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
 
 void h2d_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
   cudaStream_t st = C.stream;
-  if (bytes < kStageMin) {
+  if (bytes < kStageMin || page_locked(src, bytes)) {
     HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     return;
   }

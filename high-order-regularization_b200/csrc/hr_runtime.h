@@ -181,11 +181,12 @@ constexpr size_t kPinChunk = size_t(16) << 20;
 
 // Reads `bytes` from device memory into (pageable) host memory through the
 // context's two pinned buffers: the copy of chunk k + 1 runs while host threads
-// move chunk k into place. Returns when all of it has arrived. Small reads go
-// straight to `dst`.
+// move chunk k into place. Returns when all of it has arrived. Small reads and
+// those into page-locked memory go straight to `dst`.
 void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes);
-// The same the other way: returns when `src` has been read; the last chunk may
-// still be on its way on the context's stream.
+// The same the other way: returns when a pageable `src` has been read (the last
+// chunk may still be on its way on the context's stream); a page-locked one is
+// read until the stream has passed the copy.
 void h2d_staged(Ctx& C, void* dst, const void* src, size_t bytes);
 
 // A surface on the device: sources in tree order, its tree, density buffers

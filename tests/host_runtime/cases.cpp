@@ -50,9 +50,36 @@ void failed_growth() {
   CHECK(a.p && b.p && b.n == 7000 && cap == 7);
 }
 
+// A copy between page-locked memory and the device is one copy, of pageable memory
+// one per chunk; what arrives is the same.
+void page_locked_copies() {
+  Ctx C;
+  const size_t n = size_t(5) << 20;
+  void *a, *b, *d;
+  cudaMallocHost(&a, n);
+  cudaMallocHost(&b, n);
+  d = dev_alloc(n);
+  std::vector<char> u(n), v(n);
+  for (size_t i = 0; i < n; i++) u[i] = static_cast<char*>(a)[i] = (char)(i * 7 + i / 1000);
+  auto copies = [&](const void* src, void* dst) {
+    memset(d, 0, n);
+    memset(dst, 0, n);
+    const int c0 = fake.copies;
+    h2d_staged(C, d, src, n);
+    const int c1 = fake.copies;
+    d2h_staged(C, dst, d, n);
+    CHECK(!memcmp(dst, u.data(), n));
+    return std::make_pair(c1 - c0, fake.copies - c1);
+  };
+  CHECK(copies(a, b) == std::make_pair(1, 1));
+  CHECK(copies(u.data(), v.data()).first > 1 && copies(u.data(), v.data()).second > 1);
+  CHECK(copies(a, v.data()).first == 1 && copies(u.data(), b).second == 1);
+}
+
 int main(int, char** argv) {
   const std::string c = argv[1];
   if (c == "failed_growth") failed_growth();
+  else if (c == "page_locked_copies") page_locked_copies();
   else return 2;
   return 0;
 }
