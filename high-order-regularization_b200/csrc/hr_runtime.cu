@@ -146,10 +146,14 @@ WorkspaceScope::~WorkspaceScope() {
 namespace {
 
 // The two pinned buffers; chunks of an eighth of the copy, 512 KB to kPinChunk.
+// 0 where the host gives no page-locked memory: the copy is then a plain one.
 size_t staging(Ctx& C, size_t bytes) {
-  if (!C.pin) {
-    HR_CHECK_CUDA(cudaMallocHost(&C.pin, 2 * kPinChunk));
-    for (auto& e : C.pin_ev) HR_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  for (auto& e : C.pin_ev)
+    if (!e) HR_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!C.pin && cudaMallocHost(&C.pin, 2 * kPinChunk) != cudaSuccess) {
+    cudaGetLastError();
+    C.pin = nullptr;
+    return 0;
   }
   const size_t c = (bytes / 8 + 4095) & ~size_t(4095);
   return std::min(kPinChunk, std::max(size_t(512) << 10, c));
@@ -186,12 +190,12 @@ bool page_locked(const void* p, size_t bytes) {
 
 void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
   cudaStream_t st = C.stream;
-  if (bytes < kStageMin || page_locked(dst, bytes)) {
+  const size_t chunk = bytes < kStageMin || page_locked(dst, bytes) ? 0 : staging(C, bytes);
+  if (!chunk) {
     HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     HR_CHECK_CUDA(cudaStreamSynchronize(st));
     return;
   }
-  const size_t chunk = staging(C, bytes);
   char* buf[2] = {static_cast<char*>(C.pin), static_cast<char*>(C.pin) + kPinChunk};
   const char* s = static_cast<const char*>(src);
   char* d = static_cast<char*>(dst);
@@ -212,11 +216,11 @@ void d2h_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
 
 void h2d_staged(Ctx& C, void* dst, const void* src, size_t bytes) {
   cudaStream_t st = C.stream;
-  if (bytes < kStageMin || page_locked(src, bytes)) {
+  const size_t chunk = bytes < kStageMin || page_locked(src, bytes) ? 0 : staging(C, bytes);
+  if (!chunk) {
     HR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     return;
   }
-  const size_t chunk = staging(C, bytes);
   char* buf[2] = {static_cast<char*>(C.pin), static_cast<char*>(C.pin) + kPinChunk};
   const char* s = static_cast<const char*>(src);
   char* d = static_cast<char*>(dst);

@@ -76,10 +76,29 @@ void page_locked_copies() {
   CHECK(copies(a, v.data()).first == 1 && copies(u.data(), b).second == 1);
 }
 
+// Without page-locked memory large copies are plain ones; once there is some
+// they are staged.
+void no_page_locked_memory() {
+  Ctx C;
+  const size_t n = size_t(3) << 20;
+  std::vector<char> u(n, 5), v(n);
+  void* d = dev_alloc(n);
+  fake.no_pinned = true;
+  h2d_staged(C, d, u.data(), n);
+  d2h_staged(C, v.data(), d, n);
+  CHECK(u == v && fake.copies == 2);
+  CHECK(cudaGetLastError() == cudaSuccess);
+  fake.no_pinned = false;
+  v.assign(n, 0);
+  d2h_staged(C, v.data(), d, n);
+  CHECK(u == v && fake.copies > 4);
+}
+
 int main(int, char** argv) {
   const std::string c = argv[1];
   if (c == "failed_growth") failed_growth();
   else if (c == "page_locked_copies") page_locked_copies();
+  else if (c == "no_page_locked_memory") no_page_locked_memory();
   else return 2;
   return 0;
 }
