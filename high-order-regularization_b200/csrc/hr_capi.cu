@@ -394,10 +394,12 @@ extern "C" int hr_interpolate_dl_density(hr_ctx* ctx, double h, const hr_surface
   });
 }
 
-extern "C" int hr_dst_poisson3d(hr_ctx* ctx, int n, double* f) {
+extern "C" int hr_dst_poisson3d(hr_ctx* ctx, int n, double* f) { return hr_dst_poisson3d_to(ctx, n, f, f); }
+
+extern "C" int hr_dst_poisson3d_to(hr_ctx* ctx, int n, const double* f, double* out) {
   if (!ctx) return HR_ERR_ARG;
   return guard(ctx, [&] {
-    HR_REQUIRE(n >= 1 && f, "bad DST arguments");
+    HR_REQUIRE(n >= 1 && f && out, "bad DST arguments");
     HR_CHECK_CUDA(cudaSetDevice(ctx->c.device));
     size_t m = (size_t)n * n * n;
     WorkspaceScope scope(ctx->c);
@@ -405,7 +407,7 @@ extern "C" int hr_dst_poisson3d(hr_ctx* ctx, int n, double* f) {
     d.alloc(m);
     h2d_staged(ctx->c, d.p, f, m * sizeof(double));
     dst_poisson3d_dev(ctx->c, n, d.p);
-    d2h_staged(ctx->c, f, d.p, m * sizeof(double));
+    d2h_staged(ctx->c, out, d.p, m * sizeof(double));
   });
 }
 

@@ -126,6 +126,9 @@ int hr_e2g_pressure_7ord(hr_ctx* ctx, double delta, const hr_surface* S, const d
  * n^3 host array: DST-I, divide by the eigenvalues of the 4th-order compact
  * Laplacian, DST-I, scale 1/(2(n+1))^3. */
 int hr_dst_poisson3d(hr_ctx* ctx, int n, double* f);
+/* The same from f to out (which may be f): a caller that keeps f needs no copy
+ * of it. */
+int hr_dst_poisson3d_to(hr_ctx* ctx, int n, const double* f, double* out);
 /* A plain 3D DST-I, FFTW's RODFT00 on all three axes, unnormalised
  * (Y = 2 sum X_j sin(pi (j+1)(k+1)/(n+1)) per axis), of a row-major n^3 host
  * array: what fftw_plan_r2r_3d(n, n, n, in, out, FFTW_RODFT00 x3, ...) +
