@@ -76,8 +76,11 @@ Workspace*& active_workspace() {
 
 void* Workspace::take(size_t bytes, bool up) {
   bytes = (bytes + 255) & ~size_t(255);
-  want_dev += bytes;
-  if (up) want_pin += bytes;
+  // a buffer that would not fit a workspace at its limits is no reason to grow it
+  if (want_dev + bytes <= kDevMax && (!up || want_pin + bytes <= kPinMax)) {
+    want_dev += bytes;
+    if (up) want_pin += bytes;
+  }
   if (low + bytes > dev_cap - high || (up && low + bytes > pin_cap)) return nullptr;
   if (up) {
     low += bytes;
@@ -118,7 +121,7 @@ WorkspaceScope::~WorkspaceScope() {
     return std::min(c, limit);
   };
   try {
-    if (w.want_dev > w.dev_cap && w.dev_cap < Workspace::kDevMax) {
+    if (w.want_dev > w.dev_cap) {
       if (w.dev) dev_free(w.dev);
       w.dev = nullptr;
       w.dev_cap = 0;
@@ -126,7 +129,7 @@ WorkspaceScope::~WorkspaceScope() {
       w.dev = static_cast<char*>(dev_alloc(c));
       w.dev_cap = c;
     }
-    if (w.want_pin > w.pin_cap && w.pin_cap < Workspace::kPinMax) {
+    if (w.want_pin > w.pin_cap) {
       if (w.pin) cudaFreeHost(w.pin);
       w.pin = nullptr;
       w.pin_cap = 0;

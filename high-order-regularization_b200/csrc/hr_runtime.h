@@ -59,7 +59,7 @@ struct Workspace {
   size_t dev_cap = 0, pin_cap = 0;    // capacities
   size_t low = 0, high = 0;           // uploads from the front, scratch from the back
   size_t flushed = 0;                 // uploads already copied
-  size_t want_dev = 0, want_pin = 0;  // this call's total needs
+  size_t want_dev = 0, want_pin = 0;  // this call's total needs that fit the limits
   // `bytes` of device memory, null if they do not fit; up: among the uploads
   void* take(size_t bytes, bool up);
   // copies the uploads collected since the last flush

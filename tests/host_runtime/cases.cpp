@@ -1,4 +1,5 @@
 // Host logic of csrc/hr_runtime.{h,cu} against fake_cudart.cpp; one case per run.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -94,11 +95,48 @@ void no_page_locked_memory() {
   CHECK(u == v && fake.copies > 4);
 }
 
+// The workspace grows to what a call's buffers can use of it, not for those that
+// no workspace holds; the others fit it from the next call on.
+void workspace_growth() {
+  Ctx C;
+  const size_t big = Workspace::kDevMax + 1, mid = size_t(40) << 20;
+  auto call = [&](std::vector<size_t> sizes, bool up = false) {
+    WorkspaceScope scope(C);
+    std::vector<DBuf<char>> b(sizes.size());
+    std::vector<char> h(1000000);
+    std::vector<bool> borrowed;
+    for (size_t i = 0; i < sizes.size(); i++) {
+      if (up) b[i].upload(h.data(), sizes[i], 0);
+      else b[i].alloc(sizes[i]);
+      borrowed.push_back(b[i].borrowed);
+    }
+    return borrowed;
+  };
+  const std::vector<bool> none(1, false), yes(1, true);
+  CHECK(call({big}) == none && C.ws.dev_cap == 0 && fake.device == 0);
+  CHECK(call({big, 1000}) == std::vector<bool>(2, false) && C.ws.dev_cap == size_t(1) << 20);
+  CHECK(call({big, 1000}) == std::vector<bool>({false, true}));
+  CHECK(call({mid, big, mid}) == std::vector<bool>(3, false) && C.ws.dev_cap == size_t(128) << 20);
+  CHECK(call({mid, big, mid}) == std::vector<bool>({true, false, true}));
+  // seven of 40 MB: six fit
+  CHECK(call(std::vector<size_t>(7, mid)).back() == false && C.ws.dev_cap == Workspace::kDevMax);
+  CHECK(call(std::vector<size_t>(7, mid)) == std::vector<bool>({true, true, true, true, true, true, false}));
+  // uploads need page-locked room as well: 33 of 1 MB fit its 32 MB
+  call(std::vector<size_t>(40, 1000000), true);
+  CHECK(C.ws.pin_cap == Workspace::kPinMax);
+  auto b = call(std::vector<size_t>(40, 1000000), true);
+  CHECK(std::count(b.begin(), b.end(), true) == 33 && b[0] && !b[39]);
+  CHECK(fake.device == C.ws.dev_cap);
+  C.ws.free_all();
+  CHECK(fake.device == 0 && fake.locked.empty());
+}
+
 int main(int, char** argv) {
   const std::string c = argv[1];
   if (c == "failed_growth") failed_growth();
   else if (c == "page_locked_copies") page_locked_copies();
   else if (c == "no_page_locked_memory") no_page_locked_memory();
+  else if (c == "workspace_growth") workspace_growth();
   else return 2;
   return 0;
 }
