@@ -40,6 +40,24 @@ DevPool& pool_of(int dev) {
   return P;
 }
 
+// The workspaces that hold device memory, so that an allocation for which the
+// device has no room can have that of contexts which are in no stateless call.
+std::mutex g_ws_mu;  // also guards Workspace::busy
+std::vector<Workspace*>& g_ws = *new std::vector<Workspace*>;  // never destroyed: a context may outlive static objects
+
+bool release_idle_workspaces(int dev) {
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  bool any = false;
+  for (Workspace* w : g_ws) {
+    if (w->busy || !w->dev || w->device != dev) continue;
+    dev_free(w->dev);
+    w->dev = nullptr;
+    w->dev_cap = 0;
+    any = true;
+  }
+  return any;
+}
+
 }  // namespace
 
 void* dev_alloc(size_t bytes) {
@@ -47,7 +65,12 @@ void* dev_alloc(size_t bytes) {
   HR_CHECK_CUDA(cudaGetDevice(&dev));
   DevPool& P = pool_of(dev);
   void* p = nullptr;
-  HR_CHECK_CUDA(cudaMallocFromPoolAsync(&p, bytes, P.pool, P.st));
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, P.pool, P.st);
+  if (e == cudaErrorMemoryAllocation && release_idle_workspaces(dev)) {
+    cudaGetLastError();
+    e = cudaMallocFromPoolAsync(&p, bytes, P.pool, P.st);
+  }
+  HR_CHECK_CUDA(e);
   // complete before any other stream sees the pointer
   HR_CHECK_CUDA(cudaStreamSynchronize(P.st));
   return p;
@@ -96,6 +119,8 @@ void Workspace::flush(cudaStream_t st) {
 }
 
 void Workspace::free_all() {
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  g_ws.erase(std::remove(g_ws.begin(), g_ws.end(), this), g_ws.end());
   if (dev) dev_free(dev);
   if (pin) cudaFreeHost(pin);
   dev = pin = nullptr;
@@ -104,6 +129,12 @@ void Workspace::free_all() {
 
 WorkspaceScope::WorkspaceScope(Ctx& c) : C(c) {
   Workspace& w = C.ws;
+  {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    w.device = C.device;
+    w.busy = true;
+    if (std::find(g_ws.begin(), g_ws.end(), &w) == g_ws.end()) g_ws.push_back(&w);
+  }
   w.low = w.high = w.flushed = w.want_dev = w.want_pin = 0;
   active_workspace() = &w;
 }
@@ -144,6 +175,8 @@ WorkspaceScope::~WorkspaceScope() {
     }
   } catch (...) {  // no memory to keep: the next call allocates as it goes
   }
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  w.busy = false;
 }
 
 namespace {

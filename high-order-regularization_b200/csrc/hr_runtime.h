@@ -50,10 +50,14 @@ void dev_free(void* p) noexcept;
 // an entry point made ~55 allocations, as many uploads and as many frees, each
 // with a synchronization: most of the 0.7 ms of a small sum. What does not fit
 // comes from dev_alloc as before and grows the workspace, up to its limits, when
-// the call is over. One call at a time (a context belongs to one thread).
+// the call is over. One call at a time (a context belongs to one thread). An
+// allocation for which the device has no room gets the memory of the workspaces
+// that are between calls.
 struct Workspace {
   static constexpr size_t kDevMax = size_t(256) << 20, kPinMax = size_t(32) << 20;
   static constexpr size_t kSmall = size_t(4) << 20;  // uploads up to this size are collected
+  int device = 0;
+  bool busy = false;  // in a WorkspaceScope: otherwise dev_alloc may take the device memory back
   char* dev = nullptr;
   char* pin = nullptr;
   size_t dev_cap = 0, pin_cap = 0;    // capacities

@@ -131,12 +131,44 @@ void workspace_growth() {
   CHECK(fake.device == 0 && fake.locked.empty());
 }
 
+// An allocation that does not fit gets the memory of the contexts between calls,
+// not that of one in a call; the next call has its workspace again.
+void workspace_given_back() {
+  Ctx A, B;
+  const size_t mb = size_t(1) << 20;
+  auto call = [&](Ctx& C, auto&& inside) {
+    WorkspaceScope scope(C);
+    DBuf<char> b;
+    b.alloc(3 * mb);
+    b.zero(0);
+    inside();
+    return b.borrowed;
+  };
+  auto nothing = [] {};
+  for (Ctx* C : {&A, &B})
+    for (int i = 0; i < 2; i++) call(*C, nothing);
+  CHECK(fake.device == 8 * mb && call(A, nothing) && call(B, nothing));
+  fake.device_limit = 10 * mb;
+  void* p = nullptr;
+  const bool had = call(B, [&] { p = dev_alloc(5 * mb); });  // takes A's, leaves B's
+  CHECK(had && p && !A.ws.dev && B.ws.dev && fake.device == 9 * mb);
+  CHECK(throws([&] { call(B, [&] { dev_alloc(5 * mb); }); }));
+  CHECK(B.ws.dev && cudaGetLastError() == cudaSuccess);
+  dev_free(p);
+  CHECK(!call(A, nothing) && call(A, nothing) && call(B, nothing));
+  A.ws.free_all();
+  B.ws.free_all();
+  CHECK(fake.device == 0);
+  CHECK(throws([&] { dev_alloc(11 * mb); }));
+}
+
 int main(int, char** argv) {
   const std::string c = argv[1];
   if (c == "failed_growth") failed_growth();
   else if (c == "page_locked_copies") page_locked_copies();
   else if (c == "no_page_locked_memory") no_page_locked_memory();
   else if (c == "workspace_growth") workspace_growth();
+  else if (c == "workspace_given_back") workspace_given_back();
   else return 2;
   return 0;
 }
