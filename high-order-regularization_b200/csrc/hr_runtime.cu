@@ -512,6 +512,35 @@ PairCost pair_cost(int kind, int mixed) {
 
 }  // namespace
 
+std::vector<int> item_order(const std::vector<double>& cost, const std::vector<uint8_t>& lean) {
+  // Stable LSD radix sort, 11 bits per pass, of 2 cost (an integer, cut to 31
+  // bits) downwards below a bit for the others, the item's number in the low half.
+  // A comparison sort of the items took half of finalize; with it and larger
+  // records the first reduced-precision application at h = 1/32 (17,822 items)
+  // was 1.62 ms instead of 1.20.
+  const size_t n = cost.size();
+  double most = 0.0;
+  for (double c : cost) most = std::max(most, c);
+  uint64_t top = (uint64_t)(2.0 * most);
+  int drop = 0, bits = 0;
+  while (top >> drop >> 31) drop++;
+  top >>= drop;
+  while (top >> bits) bits++;
+  std::vector<uint64_t> a(n), b(n);
+  for (size_t i = 0; i < n; i++)
+    a[i] = ((top - ((uint64_t)(2.0 * cost[i]) >> drop)) | (uint64_t)(lean[i] ? 0 : 1) << bits) << 32 | i;
+  for (int shift = 32; shift <= 32 + bits; shift += 11) {
+    int cnt[2049] = {0};
+    for (uint64_t r : a) cnt[((r >> shift) & 2047) + 1]++;
+    for (int d = 0; d < 2048; d++) cnt[d + 1] += cnt[d];
+    for (uint64_t r : a) b[cnt[(r >> shift) & 2047]++] = r;
+    a.swap(b);
+  }
+  std::vector<int> order(n);
+  for (size_t i = 0; i < n; i++) order[i] = (int)(uint32_t)a[i];
+  return order;
+}
+
 void Batch::finalize(cudaStream_t st, int num_sms) {
   struct HSeg {
     Seg s;
@@ -584,6 +613,7 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     per[t].resize(L.nblocks());
 #pragma omp parallel for schedule(dynamic, 16)
     for (int b = 0; b < L.nblocks(); b++) {
+      per[t][b].reserve(2 * (L.blk_start[b + 1] - L.blk_start[b]));
       for (int e = L.blk_start[b]; e < L.blk_start[b + 1]; e++) {
         const Entry& E = L.entries[e];
         const int warps = entry_warps(E);
@@ -632,7 +662,9 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   }
   HR_REQUIRE(seg_off[nbt] < (1L << 31) && slot_off[nbt] < (1L << 31), "batch too large for 32-bit segment indices");
   std::vector<Seg> segs(seg_off[nbt]);
-  std::vector<std::pair<double, BlockRef>> items(slot_off[nbt]);
+  std::vector<BlockRef> items(slot_off[nbt]);
+  std::vector<double> cost(slot_off[nbt]);
+  std::vector<uint8_t> lean(slot_off[nbt]);
 #pragma omp parallel for schedule(dynamic, 64)
   for (long q = 0; q < nbt; q++) {
     const int t = tblocks[q].x, b = tblocks[q].y;
@@ -642,7 +674,9 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
     for (const auto& r : runs[q]) {
       BlockRef ref{t, b, sg, sg + r.first, it};
       for (int k = 0; k < r.first; k++) segs[sg++] = v[i++].s;
-      items[it++] = {r.second, ref};
+      items[it] = ref;
+      lean[it] = lean_kind(tasks[t].kind);
+      cost[it++] = r.second;
     }
   }
   // per task: the slot of each block's first item, then the task's end
@@ -659,19 +693,10 @@ void Batch::finalize(cudaStream_t st, int num_sms) {
   }
   // lean items first (their own launch: on-surface kinds, or the extend-to-grid
   // box-face sums), each part by decreasing cost
-  auto on_kind = [&](const BlockRef& r) { return lean_kind(tasks[r.task].kind); };
-  std::stable_sort(items.begin(), items.end(),
-                   [&](const std::pair<double, BlockRef>& a, const std::pair<double, BlockRef>& b) {
-                     const bool oa = on_kind(a.second), ob = on_kind(b.second);
-                     if (oa != ob) return oa;
-                     return a.first > b.first;
-                   });
+  const std::vector<int> order = item_order(cost, lean);
   std::vector<BlockRef> br(items.size());
-  n_on = 0;
-  for (size_t i = 0; i < items.size(); i++) {
-    br[i] = items[i].second;
-    n_on += on_kind(br[i]) ? 1 : 0;
-  }
+  for (size_t i = 0; i < items.size(); i++) br[i] = items[order[i]];
+  n_on = (int)std::count(lean.begin(), lean.end(), 1);
   nitems = (int)br.size();
   ntask_blocks = (int)tblocks.size();
   d_items.upload(br, st);

@@ -247,6 +247,11 @@ struct DevStencils {
   void build(const Stencils& S, cudaStream_t st);
 };
 
+// The order of a batch's items: the lean ones first, each part by decreasing cost,
+// equal costs as they stand. Costs are multiples of 1/2 (from 2^30 on compared to
+// 31 bits).
+std::vector<int> item_order(const std::vector<double>& cost, const std::vector<uint8_t>& lean);
+
 // A batch of boundary sums evaluated together (one or two kernel launches and
 // one reduction).
 struct Batch {

@@ -1,5 +1,6 @@
 // Host logic of csrc/hr_runtime.{h,cu} against fake_cudart.cpp; one case per run.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -162,6 +163,26 @@ void workspace_given_back() {
   CHECK(throws([&] { dev_alloc(11 * mb); }));
 }
 
+// The items' order is that of a stable comparison sort.
+void order_of_items() {
+  unsigned r = 1;
+  auto next = [&] { return r = r * 1664525u + 1013904223u, r >> 8; };
+  for (int n : {0, 1, 2, 17, 5000})
+    for (double most : {0.5, 3.0, 2047.5, 2048.0, 1e6, 1e9}) {
+      std::vector<double> cost(n);
+      std::vector<uint8_t> lean(n);
+      for (int i = 0; i < n; i++) {
+        cost[i] = i % 5 ? 0.5 * std::floor(2.0 * most * ((next() % 1000) / 999.0)) : 0.0;
+        lean[i] = next() % 3 == 0;
+      }
+      std::vector<int> want(n);
+      for (int i = 0; i < n; i++) want[i] = i;
+      std::stable_sort(want.begin(), want.end(),
+                       [&](int x, int y) { return lean[x] != lean[y] ? lean[x] > lean[y] : cost[x] > cost[y]; });
+      CHECK(item_order(cost, lean) == want);
+    }
+}
+
 int main(int, char** argv) {
   const std::string c = argv[1];
   if (c == "failed_growth") failed_growth();
@@ -169,6 +190,7 @@ int main(int, char** argv) {
   else if (c == "no_page_locked_memory") no_page_locked_memory();
   else if (c == "workspace_growth") workspace_growth();
   else if (c == "workspace_given_back") workspace_given_back();
+  else if (c == "order_of_items") order_of_items();
   else return 2;
   return 0;
 }

@@ -26,6 +26,6 @@ def _run(cases, name):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("name", ["failed_growth", "page_locked_copies", "no_page_locked_memory", "workspace_growth", "workspace_given_back"])
+@pytest.mark.parametrize("name", ["failed_growth", "page_locked_copies", "no_page_locked_memory", "workspace_growth", "workspace_given_back", "order_of_items"])
 def test_case(cases, name):
     _run(cases, name)
