@@ -31,6 +31,7 @@ def _sources():
     cpp = sorted(f for f in glob.glob(os.path.join(HERE, "host", "*.cpp"))
                  if not f.endswith(("hr_ref_api.cpp", "hr_fftw_shim.cpp")))
     hdr = sorted(glob.glob(os.path.join(HERE, "csrc", "*.h")) + glob.glob(os.path.join(HERE, "csrc", "*.cuh"))
+                 + glob.glob(os.path.join(HERE, "csrc", "*.inc"))
                  + glob.glob(os.path.join(HERE, "host", "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
                  + glob.glob(os.path.join(ROOT, "include", "fftw_shim", "*.h")))
     return cu, cpp, hdr
