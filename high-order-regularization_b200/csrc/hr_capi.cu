@@ -169,10 +169,13 @@ void single_eval(Ctx& C, int kind, const hr_eval_opts* opt, double delta, const 
   if (kind == K_DL_OFF) tg.g0.upload(dens0, 3 * (size_t)nt, st);
   // Target blocks. A treecode's lists, and the FP32 sums (coordinates relative
   // to a block's first target), take the full Morton order. In an FP64 direct
-  // sum the order changes no target's result; it only decides which targets
-  // share a warp's branches, for which 128 cells per axis do (two of the sort's
-  // six passes: 1.9 -> 0.6 ms of host time for 55,298 targets), and the plain
-  // box-face sums have no branches at all.
+  // sum the order decides which targets share a warp's branches, for which 128
+  // cells per axis do (two of the sort's six passes: 1.9 -> 0.6 ms of host time
+  // for 55,298 targets), and the plain box-face sums have no branches at all.
+  // A target's result depends on the order and on the other targets at rounding
+  // level only: its sources are cut into the items of its block, and an
+  // off-surface stresslet's warp takes a pair beyond 8 delta in the plain or in
+  // the subtraction form for all its targets at once (pairs_dl_off).
   std::vector<int> order;
   if (direct && !reduced) {
     if (kind == K_E2G_SL_AWAY || kind == K_E2G_P_AWAY) {

@@ -349,7 +349,8 @@ Lists build_lists(const Tree& T, int nt, const double* txyz, const uint8_t* near
       // Targets with the same (or a similar) interaction list take neighbouring
       // positions, so that a warp's 32 targets tend to share their entries and
       // warps skip more entries whole. A target's sums do not depend on its
-      // position in the block.
+      // position in the block (an off-surface FP64 stresslet's do in the last
+      // bits: pairs_dl_off chooses between two forms of a pair by the warp).
       for (int tt = 0; tt < cnt_t; tt++) order[tt] = tt;
       std::stable_sort(order.begin(), order.begin() + cnt_t,
                        [&](int x, int y) { return keys[x] < keys[y]; });
