@@ -488,7 +488,7 @@ void launch_moments(int C, int P1, const MomTree& t0, const MomTree& t1, cudaStr
   if (nitems <= 0) return;
   const MomShape m = mom_shape(C, P1);
   auto* fn = C == 9 ? moments_kernel<9> : moments_kernel<6>;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, m.smem);
+  allow_shared(fn);
   fn<<<dim3(nitems, m.ctas), m.warps * 32, m.smem, st>>>(t0, t1, m);
 }
 

@@ -164,6 +164,17 @@ void launch_matvec_combine(const CombineSet& s0, const CombineSet& s1, double fa
                            cudaStream_t st);
 void launch_rhs_combine(const CombineSet& s0, const CombineSet& s1, double factor, double* b, cudaStream_t st);
 
+// Lets a kernel (without static shared memory) be launched with any dynamic shared
+// memory that a CTA can have. The limit belongs to the kernel on its device, not
+// to a launch: one set to what a launch needs would refuse a larger launch by
+// another thread, or by a plan made earlier. Set on every launch, as it belongs
+// to the current device.
+constexpr int kCtaShared = 227 * 1024;
+template <class F>
+inline cudaError_t allow_shared(F* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtaShared);
+}
+
 // Vector kernels for GMRES (deterministic reductions).
 constexpr int kRedBlocks = 296;
 struct DotWork {

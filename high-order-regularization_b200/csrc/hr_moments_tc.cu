@@ -345,11 +345,11 @@ void launch_moments_tc(int dl, const MomItem* d_items, int nitems, int P1, const
   sh.M2 = P1 * P1;
   const size_t smem = moments_tc_smem(dl, P1, &sh.Npad, &sh.cols);
   if (dl) {
-    cudaFuncSetAttribute(moments_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_shared(moments_tc_kernel<true>);
     moments_tc_kernel<true><<<nitems, kTcThreads, smem, st>>>(d_items, sh, tcheb, x, y, z, nx, ny, nz, a, qx, qy,
                                                               qz, partial, err);
   } else {
-    cudaFuncSetAttribute(moments_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_shared(moments_tc_kernel<false>);
     moments_tc_kernel<false><<<nitems, kTcThreads, smem, st>>>(d_items, sh, tcheb, x, y, z, nx, ny, nz, a, qx, qy,
                                                                qz, partial, err);
   }
