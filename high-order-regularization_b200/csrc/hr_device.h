@@ -167,8 +167,7 @@ void launch_rhs_combine(const CombineSet& s0, const CombineSet& s1, double facto
 // Lets a kernel (without static shared memory) be launched with any dynamic shared
 // memory that a CTA can have. The limit belongs to the kernel on its device, not
 // to a launch: one set to what a launch needs would refuse a larger launch by
-// another thread, or by a plan made earlier. Set on every launch, as it belongs
-// to the current device.
+// another thread, or by a plan made earlier.
 constexpr int kCtaShared = 227 * 1024;
 template <class F>
 inline cudaError_t allow_shared(F* kernel) {

@@ -748,8 +748,8 @@ struct DstPlan {
       fn = P == 48 ? dst_pass_kernel<48> : P == 24 ? dst_pass_kernel<24> : dst_pass_kernel<0>;
       smem = 2 * (size_t)dst_bufd(P) * sizeof(double);
     }
-    HR_REQUIRE(smem <= 227 * 1024, "DST-I line longer than one CTA's shared memory holds");
-    HR_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HR_REQUIRE(smem <= kCtaShared, "DST-I line longer than one CTA's shared memory holds");
+    HR_CHECK_CUDA(allow_shared(fn));  // also for the plans of other sizes that share the kernel
     tmp.alloc((size_t)n * n * n);
     // twiddles e^{-2 pi i k/N} and sin(j pi/N), evaluated in extended precision
     std::vector<double2> t(N);

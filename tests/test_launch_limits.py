@@ -10,7 +10,7 @@ PKG = os.path.join(os.path.dirname(HERE), "high-order-regularization_b200")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
-def _program(d, cpp, cu):
+def _program(d, cpp, cu, more=()):
     """The program of host_runtime/*.cpp sources and the package's .cu files."""
     objs = []
     for f in cu:
@@ -19,7 +19,7 @@ def _program(d, cpp, cu):
                         "-std=c++17", "--expt-relaxed-constexpr", "-c", os.path.join(PKG, "csrc", f), "-o", objs[-1]], check=True)
     exe = str(d / "program")
     subprocess.run(["g++", "-O1", "-g", "-std=c++17", "-fopenmp", "-I", os.path.join(CUDA, "include"),
-                    *(os.path.join(HERE, "host_runtime", f) for f in cpp), *objs, "-o", exe], check=True)
+                    *(os.path.join(HERE, "host_runtime", f) for f in cpp), *more, *objs, "-o", exe], check=True)
     return exe
 
 
@@ -30,3 +30,8 @@ def _run(exe, *args):
 
 def test_upward_passes_of_two_degrees(tmp_path):
     _run(_program(tmp_path, ["upward_cases.cpp", "fake_launch.cpp"], ["hr_aux.cu", "hr_moments_tc.cu"]))
+
+
+def test_sine_transform_plans_of_two_sizes(tmp_path):
+    _run(_program(tmp_path, ["dst_cases.cpp", "fake_cudart.cpp", "fake_launch.cpp"], ["hr_poisson.cu", "hr_runtime.cu"],
+                  [os.path.join(PKG, "host", "hr_tree.cpp")]))
