@@ -480,7 +480,7 @@ def run_ours(args, rank, world, local_rank):
     plan.matvec_dev(x, b)
     ms_dl = plan.time_batch(0, 20)
     ms_dl_mixed = plan.time_batch(2, 20)
-    moment_flops = 2.0 * 12 * w_mv["moment_terms"]
+    moment_flops = 2.0 * 12 * w_mv["moment_terms"]  # as hr_plan2s_work counts them (the reference's 12 channels)
     fl_launch = w_mv["flops"] - moment_flops
     peak = ctx.fp64_peak()
     peak32 = ctx.fp32_peak()

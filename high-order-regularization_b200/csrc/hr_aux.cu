@@ -9,7 +9,6 @@ namespace hr {
 
 namespace {
 
-
 // Upward pass: the barycentric Lagrange proxy moments of Panel_Moments_SL /
 // Panel_Moments_DL (2S/KITC.cpp:351-668) of one (node, source range) item,
 //   M[c][ijk] = sum_s L_i(x_s) L_j(y_s) L_k(z_s) A_s q_c(s),
@@ -191,20 +190,19 @@ __global__ void __launch_bounds__(kMomWarps * 32) moments_kernel(MomTree t0, Mom
   if (!has_job) return;
   // accumulator of a lane: row l / 4, columns 2 (l mod 4) and the next
 #pragma unroll
-  for (int r = 0; r < kMomRT; r++)
+  for (int r = 0; r < kMomRT; r++) {
+    const int row = (rt0 + r) * 8 + (lane >> 2);
 #pragma unroll
     for (int c = 0; c < kMomCT; c++)
-    {
-        const int row = (rt0 + r) * 8 + (lane >> 2);
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int col = (ct0 + c) * 8 + 2 * (lane & 3) + h;
-          if (row < M2 && col < C * P1) {
-            const int ch = col / P1, i = col - ch * P1;
-            t.partial[((size_t)it.out * C + ch) * Pf + (size_t)i * M2 + row] = acc[r][c][h];
-          }
+      for (int h = 0; h < 2; h++) {
+        const int col = (ct0 + c) * 8 + 2 * (lane & 3) + h;
+        if (row < M2 && col < C * P1) {
+          const int ch = col / P1, i = col - ch * P1;
+          t.partial[((size_t)it.out * C + ch) * Pf + (size_t)i * M2 + row] = acc[r][c][h];
         }
-    }
+      }
+  }
 }
 
 // Sums the partial moments of each node in item order (deterministic) and

@@ -1215,7 +1215,7 @@ extern "C" int hr_plan2s_work(hr_plan2s* plan, int which, hr_work* w) {
       fl += q[0] * F.reg + q[1] * F.near_plain + q[2] * F.far_target + q[3] * F.proxy;
     }
     if (plan->opt.mode == HR_TREE) {
-      const int C = which == 0 ? 12 : 6;
+      const int C = which == 0 ? 12 : 6;  // the reference's channels (2S/KITC.cpp:507-668); the FP64 pass forms 9 of the 12
       for (int s = 0; s < 2; s++) {
         w->moment_terms += plan->tree[s].moment_terms;
         fl += 2.0 * C * (double)plan->tree[s].moment_terms;

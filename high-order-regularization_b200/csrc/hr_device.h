@@ -8,11 +8,11 @@
 
 namespace hr {
 
-// One boundary sum: a source surface (tree order SoA) evaluated at a target
-// set (reference order). All pointers are device pointers.
 // doubles per target in a work item's partial sums (3 velocity + 1 pressure)
 constexpr int kPartComps = 4;
 
+// One boundary sum: a source surface (tree order SoA) evaluated at a target
+// set (reference order). All pointers are device pointers.
 struct EvalTask {
   int kind;       // Kind
   int jump_mode;  // DL kinds: 0 = treecode convention, 1 = direct-sum convention
@@ -43,7 +43,7 @@ struct EvalTask {
   const Entry* entries;                               // interaction entries
   unsigned long long* counters;  // [0] regularized pairs [1] near-target plain [2] far-target [3] proxy
   const int* item_start;  // per target block: its work items' partial slots [start, end)
-  double* partial;        // 3 x 128 doubles per work item
+  double* partial;        // kTB x kPartComps doubles per work item
 };
 
 // A piece of one entry: a near entry's source sub-range [s0, s1), or a whole

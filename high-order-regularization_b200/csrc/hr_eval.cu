@@ -791,9 +791,6 @@ __device__ __noinline__ double3 tile_near(const EvalTask& T, int t, bool act, in
   RegF gf;
   gf.inv_d = (float)g.inv_d;
   gf.d64 = (float)g.d64;
-  gf.inv_d2 = (float)g.inv_d2;
-  gf.inv_d3 = (float)g.inv_d3;
-  gf.inv_d5 = (float)g.inv_d5;
   const float cut2f = T.mixed == 2 ? 1e-28f : (float)(9.0 * T.DEL * T.DEL);
   double a0 = a.x, a1 = a.y, a2 = a.z;
   for (int j0 = 0; j0 < cnt; j0 += 16) {
@@ -1061,9 +1058,6 @@ __device__ __forceinline__ void run_item(const EvalTask& T, const BlockRef& it, 
   RegF gf;
   gf.inv_d = (float)g.inv_d;
   gf.d64 = (float)g.d64;
-  gf.inv_d2 = (float)g.inv_d2;
-  gf.inv_d3 = (float)g.inv_d3;
-  gf.inv_d5 = (float)g.inv_d5;
   // FP64 below, FP32 above: (3 delta)^2 in the mixed mode; in the all-FP32 mode
   // only the r < 1e-14 limits of the reference stay in FP64
   const float cut2f = T.mixed == 2 ? 1e-28f : (float)(9.0 * T.DEL * T.DEL);

@@ -19,11 +19,11 @@ namespace hr {
 // sqrt(pi) as the reference computes it: sqrt of the double nearest pi (0x1.c5bf891b4ef6ap+0)
 __device__ __forceinline__ double d_rootpi() { return 1.7724538509055159; }
 
+// Per-target constants of the regularized kernels.
 struct Coef {
   double c1, c2, c3;
 };
 
-// Per-target constants of the regularized kernels.
 // Beyond r = sqrt(51) delta (r/delta = 7.14) the on-surface smoothing factors
 // G1, G2, G3 equal the singular kernel's to a relative 2^-54 (their erfc and
 // polynomial-times-Gaussian terms are smaller; 7.11 is the largest of the three
@@ -32,9 +32,10 @@ struct Coef {
 constexpr double kPlainOnSurf64 = 51.0;
 constexpr float kPlainOnSurf32 = 28.5f;
 
+// Constants of a regularization length.
 struct Reg {
-  double d, inv_d, d64, r0sq;  // delta, 1/delta, 64 delta^2, (1e-14)^2
-  double inv_d2, inv_d3, inv_d5;
+  double d, inv_d, d64, r0sq;     // delta, 1/delta, 64 delta^2, (1e-14)^2
+  double inv_d2, inv_d3, inv_d5;  // 1/delta^k for the tabulated on-surface factors
 };
 
 __device__ __forceinline__ Reg make_reg(double d) {
@@ -180,8 +181,7 @@ __device__ __forceinline__ bool sl_lapl_7ord(double r2, double rinv, const Reg& 
 namespace hr {
 
 struct RegF {
-  float inv_d, d64;             // 1/delta, 64 delta^2
-  float inv_d2, inv_d3, inv_d5;  // 1/delta^k for the tabulated on-surface factors
+  float inv_d, d64;  // 1/delta, 64 delta^2
 };
 
 struct CoefF {
