@@ -497,7 +497,7 @@ def run_ours(args, rank, world, local_rank):
         # dram__bytes_read.sum + dram__bytes_write.sum of this launch from one ncu capture
         # of both kernels of the batch at this workload: sources are staged once per tile,
         # so DRAM traffic is tiny next to the compute; the bound is the FP64 pipe
-        roofline["traffic"] = 10916864 + 2613504 + 10324480 + 3138048
+        roofline["traffic"] = 10917888 + 2622720 + 10322688 + 2979328
         roofline["traffic_source"] = "ncu capture of this kernel at this workload"
 
     # end to end through the C ABI with host buffers: scene upload + plan

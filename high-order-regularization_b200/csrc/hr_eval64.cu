@@ -26,7 +26,7 @@
 // 6, N0 = 2000), against one-thread-per-target CTAs with a table each and
 // CUDA's rsqrt, erf and exp: stresslet 4.91 -> 3.60 ms (on-surface 2.98 -> 2.31,
 // FP64 pipe 57 -> 67 %, data pipe 70 -> 54 %), Stokeslet 4.91 -> 3.58 ms;
-// extend-to-grid sums at N = 96 / 192 2.36 / 29.0 -> 1.79 / 22.8 ms (box faces
+// extend-to-grid sums at N = 96 / 192 2.36 / 29.0 -> 1.80 / 22.9 ms (box faces
 // 81 % of the FP64 pipe). What they do for that:
 //   * Smoothing factors come from piecewise polynomials in s = r^2/delta^2
 //     (pieces of width 1/4, hr_eval64_tables.inc), not from erf. Each lane
@@ -41,8 +41,9 @@
 //     constant-coefficient polynomial in the piece's offset.
 //   * A piece's polynomial is in the offset from its centre in pieces, which
 //     one multiply-add forms from r^2. Offsets in r^2 with the powers of delta
-//     in the coefficients cost the same and lose the high-order coefficients
-//     to underflow from delta = 1e12 on (delta^-23).
+//     in the coefficients cost the same (two-surface sums; extend-to-grid sums
+//     at N = 192 / 384 22.8 / 335 ms against 22.9 / 340) and lose the high-order
+//     coefficients to underflow from delta = 1e12 on (delta^-23).
 //   * 1/r^3 and 1/r^5 come from the hardware's approximate reciprocal square
 //     root y (rsqrt.approx.ftz.f64: a 20-bit result, so y^2 is exact) and the
 //     binomial series (1 - e)^{-k/2} in e = 1 - r^2 y^2 (|e| < 2^-18) to second
